@@ -287,6 +287,9 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  *       "direct.pairs_per_lane" (2 or 4 packed i-pairs per lane, one-sided),
  *       "direct.unroll" (2, 4 or 8: j-loop unroll),
  *       "direct.blocks_per_sm" (CTAs per SM of the persistent direct grid),
+ *       "direct.fp64_split" (1: the FP64 direct sum in two-word FP32
+ *       arithmetic with its large terms in FP64, the default from 1536
+ *       bodies on; 0: every pair on the FP64 pipe),
  *       "direct.uniform_mass" (1, the default: when every body has the same
  *       mass the symmetric kernel weights pairs by r^-3 alone and scales the
  *       sums by the mass once, in FP64; 0: the general kernel),

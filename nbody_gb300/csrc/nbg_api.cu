@@ -1,6 +1,8 @@
 // nbg_api.cu -- the C ABI of the engine: handles, buffers, argument checks
 // and dispatch to the kernels.  Mirrors nbody_engine (nbody/nbody_engine.h)
 // with status codes in place of qDebug + return / CUDACHECK exit(3).
+#include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstring>
 #include <new>
@@ -352,6 +354,10 @@ nbg_status nbg_init(nbg_engine* e, size_t count, const double* vertices,
     e->uniform_mass = true;
     for (size_t i = 1; i < count && e->uniform_mass; ++i) e->uniform_mass = mass[i] == mass[0];
     e->mass_value = mass[0];
+    double largest = 0.0;
+    for (size_t i = 0; i < count; ++i)
+        if (std::isfinite(mass[i])) largest = std::max(largest, std::fabs(mass[i]));
+    std::frexp(largest, &e->mass_exp);  // 0 for 0
     NBG_CUDA(e, cudaMemcpy(y->dptr, h.data(), 6 * count * sizeof(double),
                            cudaMemcpyHostToDevice));
     NBG_CUDA(e, cudaMemcpy(e->d_mass, mass, count * sizeof(double), cudaMemcpyHostToDevice));

@@ -1,12 +1,15 @@
 // nbg_direct.cu -- direct O(N^2) gravity: f = [v ; a(y)].
 //
-// Three kernels share the engine entry point:
+// Three paths share the engine entry point:
 //
-//  * FP64 (parity) -- one thread per body, j-tiles of double4 in shared
-//    memory, the reference 'simple' arithmetic in the reference order
+//  * FP64 (parity) -- the reference 'simple' engine's sum
 //    (nbody/nbody_engine_simple.cpp:143-172 with nbody_data::force,
-//    nbody/nbody_data.cpp:35-44): explicit roundings (no FMA contraction),
-//    self pair skipped, force summed j = 0..N-1 then divided by m_i.
+//    nbody/nbody_data.cpp:35-44) to FP64 rounding, self pair skipped.  Its
+//    rounding errors are smaller than those of the reference's serial sum
+//    (measured against extended precision), because the partial sums are.
+//    Small systems: one warp per body on the FP64 pipe (direct_fp64_kernel);
+//    larger ones: two-word FP32 arithmetic, with the terms that matter taken
+//    in FP64 (split_force_kernel).  Both repeat bit for bit.
 //
 //  * mixed (throughput) -- FP32 pair math on the FP32 pipe, FP64 state.
 //    A pack kernel turns y into a tile-padded array of bodies in
@@ -25,64 +28,384 @@
 //  * mixed, symmetric (the default, tuning key direct.symmetric = 1) -- the
 //    same arithmetic with every unordered pair evaluated once and applied to
 //    both bodies (details at direct_sym_kernel).
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "nbg_internal.cuh"
 #include "nbg_pair.cuh"
 #include "nbg_ptx.cuh"
+#include "nbg_split.cuh"
 
 namespace nbg {
 namespace {
 
-// ---------------------------------------------------------------------------
-// FP64 kernel
-// ---------------------------------------------------------------------------
-constexpr int kF64Threads = 128;
+template <bool CLAMP>
+__device__ __forceinline__ void pair2(f2_t xj, f2_t yj, f2_t zj, f2_t mj, f2_t xi, f2_t yi,
+                                      f2_t zi, f2_t eps2, f2_t& ax, f2_t& ay, f2_t& az) {
+    const f2_t dx = f2_sub(xj, xi);
+    const f2_t dy = f2_sub(yj, yi);
+    const f2_t dz = f2_sub(zj, zi);
+    f2_t r2 = f2_fma(dz, dz, eps2);
+    r2 = f2_fma(dy, dy, r2);
+    r2 = f2_fma(dx, dx, r2);
+    float r2a, r2b;
+    f2_unpack(r2, r2a, r2b);
+    if (CLAMP) {
+        r2a = fmaxf(r2a, 1e-8f);
+        r2b = fmaxf(r2b, 1e-8f);
+    }
+    const f2_t inv = f2_pack(rsqrt_mufu(r2a), rsqrt_mufu(r2b));
+    const f2_t inv2 = f2_mul(inv, inv);
+    const f2_t s = f2_mul(mj, inv);
+    const f2_t s3 = f2_mul(s, inv2);
+    ax = f2_fma(dx, s3, ax);
+    ay = f2_fma(dy, s3, ay);
+    az = f2_fma(dz, s3, az);
+}
 
-struct alignas(32) D4 {
-    double x, y, z, w;
-};
+// ---------------------------------------------------------------------------
+// FP64 kernels
+// ---------------------------------------------------------------------------
+// One body of the FP64 sum: a += m_j d r^-3, r^2 at least kMinDistance (16 FP64
+// operations; the reference's pair force, nbody/nbody_data.cpp:35-44, without
+// its multiplication and division by m_i).
+__device__ __forceinline__ void pair_fp64(double dx, double dy, double dz, double m, double& ax,
+                                          double& ay, double& az) {
+    const double r2 = fmax(fma(dx, dx, fma(dy, dy, dz * dz)), kMinDistance);
+    const double w = m * rcube_fp64(r2);
+    ax = fma(dx, w, ax);
+    ay = fma(dy, w, ay);
+    az = fma(dz, w, az);
+}
+
+// The reference forms the force with m_i and divides by m_i again: for a
+// massless or non-finite m_i that is NaN.
+__device__ __forceinline__ double fp64_result(double a, double m) {
+    return m != 0.0 && fabs(m) <= 1.7976931348623157e308 ? a : a * m / m;
+}
+
+// Small systems (and any size, where the split path's scratch cannot be had):
+// one warp per body, the other bodies across its lanes, the 32 partial sums
+// added by shuffles in a fixed order.
+constexpr int kF64Threads = 32;  // one warp per CTA: the fewest idle SMs in the last wave
 
 __global__ void __launch_bounds__(kF64Threads)
 direct_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                    double* __restrict__ f, int n) {
-    __shared__ D4 tile[kF64Threads];
-    const int i = blockIdx.x * kF64Threads + threadIdx.x;
-    const bool live = i < n;
-    const double x1 = live ? y[i] : 0.0;
-    const double y1 = live ? y[n + i] : 0.0;
-    const double z1 = live ? y[2 * n + i] : 0.0;
-    const double m1 = live ? mass[i] : 1.0;
-    const double mneg = __dmul_rn(-1.0, m1);
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int j0 = 0; j0 < n; j0 += kF64Threads) {
-        const int j = j0 + threadIdx.x;
-        if (j < n) tile[threadIdx.x] = D4{y[j], y[n + j], y[2 * n + j], mass[j]};
+    const int lane = threadIdx.x & 31;
+    const int i = (int)((blockIdx.x * kF64Threads + threadIdx.x) >> 5);
+    if (i >= n) return;
+    const size_t sn = (size_t)n;
+    const double x1 = y[i], y1 = y[sn + i], z1 = y[2 * sn + i];
+    double ax = 0.0, ay = 0.0, az = 0.0;
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) {
+        if (j == i) continue;  // nbody/nbody_engine_simple.cpp:155-158
+        pair_fp64(__ldg(y + j) - x1, __ldg(y + sn + j) - y1, __ldg(y + 2 * sn + j) - z1,
+                  __ldg(mass + j), ax, ay, az);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+        az += __shfl_xor_sync(0xffffffffu, az, o);
+    }
+    if (lane < 3) {
+        f[lane * sn + i] = y[(3 + lane) * sn + i];
+        f[(3 + lane) * sn + i] = fp64_result(lane == 0 ? ax : lane == 1 ? ay : az, mass[i]);
+    }
+}
+
+// The FP64 sum on the FP32 pipe (nbg_split.cuh), for all but small systems.
+// Terms above kSplitNear of the sum of a body's |m_j| / r^2, and pairs closer
+// than 2^-20 of the system's extent or than the clamp, are queued and taken
+// in FP64: some 45 of 20011 bodies.  The rest are in two words, each off by
+// up to 1e-14 of itself at random; as none of them is large, that adds up to
+// a few 1e-16 of the sum, below what a serial FP64 sum of as many terms
+// rounds off.
+//   split_extent_kernel    max |coordinate|
+//   split_pack_kernel      scaled three-word coordinates, two-word masses
+//   split_estimate_kernel  the scale of each body's sum
+//   split_force_kernel     the sums of every (256 bodies) x (range of bodies)
+//   split_reduce_kernel    their total in range order: equal states give
+//                          equal forces
+//
+// Bound by the FP32 pipe: about 101 packed operations a pair (two bodies at
+// once), 79 % of the pipe's cycles used, the FP64 pipe 24 % beside it.  At
+// 20011 bodies 1.49 ms (the FP64 pipe alone, 16 operations a pair: 12.3 ms;
+// the reference's divide and square root in body order: 46.7 ms), RMS error
+// 8e-16 of |a| against 3.6e-15 for the serial FP64 sum.  Taking terms above
+// 1 / 2048 or 1 / 4096 in FP64 instead costs 3 % and 15 % at that size (35 %
+// and 100 % at 2048 bodies) for an error of 7e-16 and 6e-16.
+constexpr float kSplitNear = 1.f / 1024.f;
+constexpr float kSplitFarP = 1.0995116e12f;  // 2^40: 1 / r^2 of the closest two-word pair
+constexpr int kSplitT = 128;                 // threads and bodies per half, 2 bodies per thread
+constexpr int kSplitTile = 64;               // j-bodies per shared-memory tile
+constexpr int kSplitQ = 16;                  // queued FP64 pairs per body
+constexpr int kSplitChunk = 8;               // j-bodies between two looks at the queues
+constexpr int kSplitExtents = 64;            // CTAs of split_extent_kernel
+constexpr int kSplitEst = 8;                 // ranges of split_estimate_kernel
+
+struct SplitBody {  // 48 bytes
+    float4 a;       // xh xm xl yh
+    float4 b;       // ym yl zh zm
+    float4 c;       // zl mh ml |m|
+};
+
+struct SplitArgs {
+    const double* y;
+    const double* mass;
+    double* f;
+    SplitBody* bodies;            // [n_pad], padding far away and massless
+    float* est;                   // [kSplitEst][n_pad] sampled sums of |m| / r^2, scaled units
+    double* part;                 // [ranges][3][n]
+    unsigned long long* extent;   // [kSplitExtents] bits of max |coordinate|
+    double mass_scale;            // power of two: largest |m| into [1/2, 1)
+    int mass_exp;                 // mass_scale = 2^-mass_exp
+    int n, n_pad, range, ranges;  // range: j-bodies per CTA, a multiple of kSplitTile
+};
+
+__global__ void __launch_bounds__(256) split_extent_kernel(SplitArgs a) {
+    unsigned long long m = 0;
+    const size_t n3 = 3 * (size_t)a.n;
+    for (size_t i = blockIdx.x * 256 + threadIdx.x; i < n3; i += (size_t)gridDim.x * 256)
+        m = max(m, (unsigned long long)__double_as_longlong(fabs(a.y[i])));
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    __shared__ unsigned long long w[8];
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) m = max(m, w[k]);
+        a.extent[blockIdx.x] = m;
+    }
+}
+
+// exponent E with every |coordinate| < 2^E (in every thread; 2048 for a
+// coordinate that is not finite)
+__device__ __forceinline__ int split_exponent(const SplitArgs& a) {
+    unsigned long long m = 0;
+    const int lane = threadIdx.x & 31;
+    for (int k = lane; k < kSplitExtents; k += 32) m = max(m, __ldg(a.extent + k));
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const int ex = (int)(m >> 52);
+    return ex == 0x7ff ? 2048 : ex - 1022;
+}
+
+__global__ void __launch_bounds__(256) split_pack_kernel(SplitArgs a) {
+    const int ex = split_exponent(a);
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < a.n_pad; i += gridDim.x * 256) {
+        SplitBody b;
+        if (i < a.n) {
+            float h[3], m[3], l[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                split3(ex == 2048 ? nan("") : scalbn(a.y[(size_t)c * a.n + i], -ex), h[c], m[c], l[c]);
+            const double ms = a.mass[i] * a.mass_scale;
+            // a mass far below the largest is taken in FP64 throughout
+            const bool tiny = ms != 0.0 && fabs(ms) < 9.313225746154785e-10;  // 2^-30
+            const float mh = (float)ms, ml = (float)(ms - (double)mh);
+            b.a = make_float4(h[0], m[0], l[0], h[1]);
+            b.b = make_float4(m[1], l[1], h[2], m[2]);
+            b.c = make_float4(l[2], mh, ml, tiny ? __int_as_float(0x7fffffff) : fabsf(mh));
+        } else {
+            // padding: massless, and so far away that r^-3 underflows to 0
+            b.a = make_float4(1e18f, 0.f, 0.f, 1e18f);
+            b.b = make_float4(0.f, 0.f, 1e18f, 0.f);
+            b.c = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        a.bodies[i] = b;
+    }
+}
+
+// Per body, the sum of |m_j| / r^2 over a quarter of the others (32 bodies of
+// every 128; a sum without cancellation, so neither the sample nor a body in
+// the middle of a symmetric system changes its scale much).  256 bodies per
+// CTA against one of kSplitEst ranges, in FP32x2.
+__global__ void __launch_bounds__(kSplitT) split_estimate_kernel(SplitArgs a) {
+    __shared__ __align__(16) float4 tile[kSplitT][2];
+    const int tid = threadIdx.x;
+    const int i0 = blockIdx.x * 2 * kSplitT + tid, i1 = i0 + kSplitT;  // < n_pad
+    const SplitBody p = a.bodies[i0], q = a.bodies[i1];
+    const f2_t xi = f2_pack(p.a.x, q.a.x), yi = f2_pack(p.a.w, q.a.w), zi = f2_pack(p.b.z, q.b.z);
+    constexpr float kLeast = 1.f / kSplitFarP;  // closer pairs (the body itself) do not count
+    f2_t sum = f2_pack(0.f, 0.f);
+    const uint32_t base = smem_addr(tile);
+    for (int j0 = blockIdx.y * 4 * kSplitT; j0 < a.n_pad; j0 += gridDim.y * 4 * kSplitT) {
+        const int j = j0 + (tid >> 5) * kSplitT + (tid & 31);
         __syncthreads();
-        const int cnt = min(kF64Threads, n - j0);
-        for (int k = 0; k < cnt; ++k) {
-            if (j0 + k == i) continue;  // nbody/nbody_engine_simple.cpp:155-158
-            const D4 p = tile[k];
-            const double dx = __dsub_rn(x1, p.x);
-            const double dy = __dsub_rn(y1, p.y);
-            const double dz = __dsub_rn(z1, p.z);
-            double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            if (r2 < kMinDistance) r2 = kMinDistance;
-            const double c = __ddiv_rn(__dmul_rn(mneg, p.w), __dmul_rn(r2, __dsqrt_rn(r2)));
-            fx = __dadd_rn(fx, __dmul_rn(dx, c));
-            fy = __dadd_rn(fy, __dmul_rn(dy, c));
-            fz = __dadd_rn(fz, __dmul_rn(dz, c));
+        SplitBody b = a.bodies[min(j, a.n_pad - 1)];
+        if (j >= a.n_pad) b.c.y = 0.f;
+        const float m = fabsf(b.c.y);
+        tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.w, b.a.w);
+        tile[tid][1] = make_float4(b.b.z, b.b.z, m, m);
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < kSplitT; ++k) {
+            const float4 u = lds128(base + 32u * k), v = lds128(base + 32u * k + 16u);
+            const f2_t dx = f2_sub(f2_pack(u.x, u.y), xi), dy = f2_sub(f2_pack(u.z, u.w), yi);
+            const f2_t dz = f2_sub(f2_pack(v.x, v.y), zi);
+            float r0, r1;
+            f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), r0, r1);
+            const float t0 = r0 > kLeast ? rcp_mufu(r0) : 0.f, t1 = r1 > kLeast ? rcp_mufu(r1) : 0.f;
+            sum = f2_fma(f2_pack(v.z, v.w), f2_pack(t0, t1), sum);
+        }
+    }
+    float s0, s1;
+    f2_unpack(sum, s0, s1);
+    a.est[(size_t)blockIdx.y * a.n_pad + i0] = s0;
+    a.est[(size_t)blockIdx.y * a.n_pad + i1] = s1;
+}
+
+__device__ __forceinline__ float split_limit(const SplitArgs& a, int i) {
+    float s = 0.f;
+#pragma unroll
+    for (int r = 0; r < kSplitEst; ++r) s += __ldg(a.est + (size_t)r * a.n_pad + i);
+    return kSplitNear * 4.f * s;
+}
+
+template <bool UNI>
+__global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
+    __shared__ __align__(16) float4 tile[kSplitTile][6];  // every word twice, for FP32x2
+    __shared__ unsigned queue[2][kSplitQ][kSplitT];
+    const int tid = threadIdx.x;
+    const size_t sn = (size_t)a.n;
+    const int i0 = blockIdx.x * 2 * kSplitT + tid, i1 = i0 + kSplitT;  // < n_pad
+    f2_t ih[3], im[3], il[3];
+    {
+        const SplitBody p = a.bodies[i0], q = a.bodies[i1];
+        ih[0] = f2_pack(p.a.x, q.a.x);
+        im[0] = f2_pack(p.a.y, q.a.y);
+        il[0] = f2_pack(p.a.z, q.a.z);
+        ih[1] = f2_pack(p.a.w, q.a.w);
+        im[1] = f2_pack(p.b.x, q.b.x);
+        il[1] = f2_pack(p.b.y, q.b.y);
+        ih[2] = f2_pack(p.b.z, q.b.z);
+        im[2] = f2_pack(p.b.w, q.b.w);
+        il[2] = f2_pack(p.c.x, q.c.x);
+    }
+    const float lim0 = split_limit(a, i0), lim1 = split_limit(a, i1);
+    const int ex = split_exponent(a);
+    // pairs at or below the clamp are taken in FP64
+    const float far_p = fminf(kSplitFarP, (float)scalbn(0.999 / kMinDistance, 2 * min(max(ex, -400), 400)));
+    const f2_t zero = f2_pack(0.f, 0.f);
+    f2_t hi[3] = {zero, zero, zero}, lo[3] = {zero, zero, zero};
+    double far0[3] = {0, 0, 0}, far1[3] = {0, 0, 0}, near0[3] = {0, 0, 0}, near1[3] = {0, 0, 0};
+    int c0 = 0, c1 = 0;  // queued pairs of this thread's two bodies
+    const int j_begin = blockIdx.y * a.range, j_end = min(j_begin + a.range, a.n_pad);
+
+    auto flush_queue = [&](int half, int i, int& cnt, double* acc) {
+        const int k = min(i, a.n - 1);
+        const double x1 = __ldg(a.y + k), y1 = __ldg(a.y + sn + k), z1 = __ldg(a.y + 2 * sn + k);
+        while (__any_sync(0xffffffffu, cnt > 0)) {
+            if (cnt > 0) {
+                const int j = (int)queue[half][--cnt][tid];
+                if (j != i && j < a.n)
+                    pair_fp64(__ldg(a.y + j) - x1, __ldg(a.y + sn + j) - y1,
+                              __ldg(a.y + 2 * sn + j) - z1, __ldg(a.mass + j), acc[0], acc[1],
+                              acc[2]);
+            }
+        }
+    };
+
+    for (int j0 = j_begin; j0 < j_end; j0 += kSplitTile) {
+        __syncthreads();
+        if (tid < kSplitTile) {
+            const SplitBody b = a.bodies[j0 + tid];
+            tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.y, b.a.y);
+            tile[tid][1] = make_float4(b.a.z, b.a.z, b.a.w, b.a.w);
+            tile[tid][2] = make_float4(b.b.x, b.b.x, b.b.y, b.b.y);
+            tile[tid][3] = make_float4(b.b.z, b.b.z, b.b.w, b.b.w);
+            tile[tid][4] = make_float4(b.c.x, b.c.x, b.c.y, b.c.y);
+            tile[tid][5] = make_float4(b.c.z, b.c.z, b.c.w, b.c.w);
         }
         __syncthreads();
+        const uint32_t base = smem_addr(tile);
+#pragma unroll 1
+        for (int jc = 0; jc < kSplitTile; jc += kSplitChunk) {
+#pragma unroll 2
+            for (int j = jc; j < jc + kSplitChunk; ++j) {
+                const uint32_t at = base + 96u * j;
+                const float4 w0 = lds128(at), w1 = lds128(at + 16), w2 = lds128(at + 32);
+                const float4 w3 = lds128(at + 48), w4 = lds128(at + 64), w5 = lds128(at + 80);
+                f2_t d1[3], d2[3], r1, r2, w, wl;
+                split_diff(f2_pack(w0.x, w0.y), f2_pack(w0.z, w0.w), f2_pack(w1.x, w1.y), ih[0],
+                           im[0], il[0], d1[0], d2[0]);
+                split_diff(f2_pack(w1.z, w1.w), f2_pack(w2.x, w2.y), f2_pack(w2.z, w2.w), ih[1],
+                           im[1], il[1], d1[1], d2[1]);
+                split_diff(f2_pack(w3.x, w3.y), f2_pack(w3.z, w3.w), f2_pack(w4.x, w4.y), ih[2],
+                           im[2], il[2], d1[2], d2[2]);
+                split_norm2(d1, d2, r1, r2);
+                const SplitRsqrt s = split_rsqrt(r1, r2);
+                split_cube(s, w, wl);
+                if (!UNI) {
+                    const f2_t mh = f2_pack(w4.z, w4.w), ml = f2_pack(w5.x, w5.y);
+                    const f2_t c = w;
+                    w = f2_mul_rn(mh, c);
+                    wl = f2_fma(ml, c, f2_fma(mh, wl, f2_fma(mh, c, f2_neg(w))));
+                }
+                float p0, p1, t0, t1;
+                f2_unpack(s.p, p0, p1);
+                f2_unpack(f2_mul(s.p, f2_pack(w5.z, w5.w)), t0, t1);
+                const bool is0 = !(t0 <= lim0 && p0 <= far_p);  // NaN counts as near
+                const bool is1 = !(t1 <= lim1 && p1 <= far_p);
+                if (is0 || is1) {
+                    float u, v, lu, lv;
+                    f2_unpack(w, u, v);
+                    f2_unpack(wl, lu, lv);
+                    if (is0) {
+                        queue[0][c0++][tid] = (unsigned)(j0 + j);
+                        u = lu = 0.f;
+                    }
+                    if (is1) {
+                        queue[1][c1++][tid] = (unsigned)(j0 + j);
+                        v = lv = 0.f;
+                    }
+                    w = f2_pack(u, v);
+                    wl = f2_pack(lu, lv);
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) split_axpy(hi[k], lo[k], w, wl, d1[k], d2[k]);
+            }
+            // the sums join the FP64 totals every 32 bodies: the error of lo grows
+            // with the square of their number (the FP64 pipe is idle otherwise)
+            if ((jc & 31) == 32 - kSplitChunk) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    float h0, h1, l0, l1;
+                    f2_unpack(hi[k], h0, h1);
+                    f2_unpack(lo[k], l0, l1);
+                    far0[k] += (double)h0 + (double)l0;
+                    far1[k] += (double)h1 + (double)l1;
+                    hi[k] = lo[k] = zero;
+                }
+            }
+            if (__any_sync(0xffffffffu, c0 > kSplitQ - kSplitChunk)) flush_queue(0, i0, c0, near0);
+            if (__any_sync(0xffffffffu, c1 > kSplitQ - kSplitChunk)) flush_queue(1, i1, c1, near1);
+        }
     }
-    if (live) {
-        f[i] = y[3 * n + i];
-        f[n + i] = y[4 * n + i];
-        f[2 * n + i] = y[5 * n + i];
-        f[3 * n + i] = __ddiv_rn(fx, m1);
-        f[4 * n + i] = __ddiv_rn(fy, m1);
-        f[5 * n + i] = __ddiv_rn(fz, m1);
+    flush_queue(0, i0, c0, near0);
+    flush_queue(1, i1, c1, near1);
+    // back to the caller's units: lengths 2^ex, masses 2^mass_exp
+    const int un = a.mass_exp - 2 * ex;
+    const double mu = UNI ? a.mass[0] * a.mass_scale : 1.0;
+    double* out = a.part + (size_t)blockIdx.y * 3 * sn;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        // (with a coordinate that is not finite every pair is in near)
+        if (i0 < a.n) out[k * sn + i0] = near0[k] + (ex == 2048 ? 0.0 : scalbn(far0[k] * mu, un));
+        if (i1 < a.n) out[k * sn + i1] = near1[k] + (ex == 2048 ? 0.0 : scalbn(far1[k] * mu, un));
     }
+}
+
+__global__ void __launch_bounds__(128) split_reduce_kernel(SplitArgs a) {
+    const size_t sn = (size_t)a.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (at >= 3 * sn) return;
+    double s = 0.0;
+#pragma unroll 16
+    for (int r = 0; r < a.ranges; ++r) s += __ldg(a.part + (size_t)r * 3 * sn + at);
+    a.f[at] = a.y[3 * sn + at];
+    a.f[3 * sn + at] = fp64_result(s, a.mass[at % sn]);
 }
 
 // ---------------------------------------------------------------------------
@@ -134,30 +457,6 @@ struct MixedArgs {
     float eps2;
     unsigned* err;
 };
-
-template <bool CLAMP>
-__device__ __forceinline__ void pair2(f2_t xj, f2_t yj, f2_t zj, f2_t mj, f2_t xi, f2_t yi,
-                                      f2_t zi, f2_t eps2, f2_t& ax, f2_t& ay, f2_t& az) {
-    const f2_t dx = f2_sub(xj, xi);
-    const f2_t dy = f2_sub(yj, yi);
-    const f2_t dz = f2_sub(zj, zi);
-    f2_t r2 = f2_fma(dz, dz, eps2);
-    r2 = f2_fma(dy, dy, r2);
-    r2 = f2_fma(dx, dx, r2);
-    float r2a, r2b;
-    f2_unpack(r2, r2a, r2b);
-    if (CLAMP) {
-        r2a = fmaxf(r2a, 1e-8f);
-        r2b = fmaxf(r2b, 1e-8f);
-    }
-    const f2_t inv = f2_pack(rsqrt_mufu(r2a), rsqrt_mufu(r2b));
-    const f2_t inv2 = f2_mul(inv, inv);
-    const f2_t s = f2_mul(mj, inv);
-    const f2_t s3 = f2_mul(s, inv2);
-    ax = f2_fma(dx, s3, ax);
-    ay = f2_fma(dy, s3, ay);
-    az = f2_fma(dz, s3, az);
-}
 
 // Issue the bulk copy of j-tile `jt` into stage `s` (one thread).
 __device__ __forceinline__ void issue_tile(Body2* tiles, uint64_t* full, int s, int jt,
@@ -704,17 +1003,88 @@ nbg_status direct_sym_launch(nbg_engine* e, const double* y, double* f) {
     return NBG_OK;
 }
 
-}  // namespace
+// Which FP64 kernel: the split path from kSplitMin bodies on, where its five
+// launches and the FP64 share of its pairs cost less than the FP64 pipe's 16
+// operations a pair (1024 bodies: 46 us against 100; 1536: 91 against 84;
+// 2048: 149 against 95).
+constexpr int kSplitMin = 1536;
 
-nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
+nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
     const int n = (int)e->count;
-    if (e->params.precision == NBG_PREC_FP64) {
-        ProfScope ps(e, NBG_K_DIRECT);
-        direct_fp64_kernel<<<(n + kF64Threads - 1) / kF64Threads, kF64Threads, 0, e->stream>>>(
+    ProfScope ps(e, NBG_K_DIRECT);
+    SplitArgs a;
+    a.y = y;
+    a.mass = e->d_mass;
+    a.f = f;
+    a.n = n;
+    a.n_pad = (n + 2 * kSplitT - 1) / (2 * kSplitT) * (2 * kSplitT);
+    const int blocks = a.n_pad / (2 * kSplitT);
+    // ranges: about 8 waves of 4 CTAs per SM (the last one weighs little; 2
+    // waves measured 2.2 ms instead of 1.5 at 20011 bodies), at least a tile each
+    const int want = (e->sm_count * 4 * 8 + blocks - 1) / blocks;
+    const int tiles = a.n_pad / kSplitTile;
+    const int per = std::max(1, tiles / std::max(1, want));
+    a.range = per * kSplitTile;
+    a.ranges = (tiles + per - 1) / per;
+    const size_t bodies = (size_t)a.n_pad * sizeof(SplitBody);
+    const size_t ests = (size_t)kSplitEst * a.n_pad * sizeof(float);
+    const size_t need = bodies + ests + kSplitExtents * sizeof(unsigned long long) +
+                        (size_t)a.ranges * 3 * n * sizeof(double);
+    bool split = e->tune_get("direct.fp64_split", n >= kSplitMin) != 0;
+    if (split && e->xyzm_cap < need) {
+        // no scratch (or none to be had while the stream is being captured):
+        // the kernel that needs none
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        NBG_CUDA(e, cudaStreamIsCapturing(e->stream, &cap));
+        split = false;
+        if (cap == cudaStreamCaptureStatusNone) {
+            cudaFree(e->d_xyzm);
+            e->d_xyzm = nullptr;
+            e->xyzm_cap = 0;
+            if (cudaMalloc(&e->d_xyzm, need) == cudaSuccess) {
+                e->xyzm_cap = need;
+                split = true;
+            } else {
+                cudaGetLastError();
+            }
+        }
+    }
+    if (!split) {
+        const unsigned warps = kF64Threads / 32;
+        direct_fp64_kernel<<<((unsigned)n + warps - 1) / warps, kF64Threads, 0, e->stream>>>(
             y, e->d_mass, f, n);
         NBG_LAUNCHED(e, "direct_fp64_kernel");
         return NBG_OK;
     }
+    char* at = reinterpret_cast<char*>(e->d_xyzm);
+    a.bodies = reinterpret_cast<SplitBody*>(at);
+    a.extent = reinterpret_cast<unsigned long long*>(at + bodies);
+    a.part = reinterpret_cast<double*>(at + bodies + kSplitExtents * sizeof(unsigned long long));
+    a.est = reinterpret_cast<float*>(a.part + (size_t)a.ranges * 3 * n);
+    a.mass_exp = e->mass_exp;
+    a.mass_scale = std::ldexp(1.0, -e->mass_exp);
+    split_extent_kernel<<<kSplitExtents, 256, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "split_extent_kernel");
+    split_pack_kernel<<<grid_for(a.n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "split_pack_kernel");
+    split_estimate_kernel<<<dim3((unsigned)blocks, kSplitEst), kSplitT, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "split_estimate_kernel");
+    const dim3 grid((unsigned)blocks, (unsigned)a.ranges);
+    if (e->uniform_mass)
+        split_force_kernel<true><<<grid, kSplitT, 0, e->stream>>>(a);
+    else
+        split_force_kernel<false><<<grid, kSplitT, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "split_force_kernel");
+    split_reduce_kernel<<<(unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "split_reduce_kernel");
+    return NBG_OK;
+}
+
+}  // namespace
+
+nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
+    const int n = (int)e->count;
+    if (e->params.precision == NBG_PREC_FP64) return direct_fp64_launch(e, y, f);
 
     // ---- mixed precision ----
     if (e->tune_get("direct.symmetric", 1) != 0) return direct_sym_launch(e, y, f);

@@ -134,6 +134,13 @@ __device__ __forceinline__ float rsqrt_mufu(float x) {
     return r;
 }
 
+// MUFU reciprocal (approximate, flush-to-zero).
+__device__ __forceinline__ float rcp_mufu(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Knuth two-sum in packed form: (hi, lo) += p with the rounding error of the
 // high-part addition carried into lo.
 __device__ __forceinline__ void f2_two_sum(f2_t& hi, f2_t& lo, f2_t p) {
