@@ -290,6 +290,8 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  *       "direct.fp64_split" (1: the FP64 direct sum in two-word FP32
  *       arithmetic with its large terms in FP64, the default from 1536
  *       bodies on; 0: every pair on the FP64 pipe),
+ *       "statistics.split_min" (bodies from which nbg_statistics sums the
+ *       potential in two-word FP32 arithmetic, default 3072),
  *       "direct.uniform_mass" (1, the default: when every body has the same
  *       mass the symmetric kernel weights pairs by r^-3 alone and scales the
  *       sums by the mass once, in FP64; 0: the general kernel),

@@ -35,7 +35,7 @@
 #include "nbg_internal.cuh"
 #include "nbg_pair.cuh"
 #include "nbg_ptx.cuh"
-#include "nbg_split.cuh"
+#include "nbg_split_sys.cuh"
 
 namespace nbg {
 namespace {
@@ -138,171 +138,42 @@ direct_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass
 // 8e-16 of |a| against 3.6e-15 for the serial FP64 sum.  Taking terms above
 // 1 / 2048 or 1 / 4096 in FP64 instead costs 3 % and 15 % at that size (35 %
 // and 100 % at 2048 bodies) for an error of 7e-16 and 6e-16.
-constexpr float kSplitNear = 1.f / 1024.f;
-constexpr float kSplitFarP = 1.0995116e12f;  // 2^40: 1 / r^2 of the closest two-word pair
-constexpr int kSplitT = 128;                 // threads and bodies per half, 2 bodies per thread
-constexpr int kSplitTile = 64;               // j-bodies per shared-memory tile
-constexpr int kSplitQ = 16;                  // queued FP64 pairs per body
-constexpr int kSplitChunk = 8;               // j-bodies between two looks at the queues
-constexpr int kSplitExtents = 64;            // CTAs of split_extent_kernel
-constexpr int kSplitEst = 8;                 // ranges of split_estimate_kernel
-
-struct SplitBody {  // 48 bytes
-    float4 a;       // xh xm xl yh
-    float4 b;       // ym yl zh zm
-    float4 c;       // zl mh ml |m|
-};
-
 struct SplitArgs {
-    const double* y;
-    const double* mass;
+    SplitSystem s;
     double* f;
-    SplitBody* bodies;            // [n_pad], padding far away and massless
-    float* est;                   // [kSplitEst][n_pad] sampled sums of |m| / r^2, scaled units
-    double* part;                 // [ranges][3][n]
-    unsigned long long* extent;   // [kSplitExtents] bits of max |coordinate|
-    double mass_scale;            // power of two: largest |m| into [1/2, 1)
-    int mass_exp;                 // mass_scale = 2^-mass_exp
-    int n, n_pad, range, ranges;  // range: j-bodies per CTA, a multiple of kSplitTile
+    double* part;       // [ranges][3][n]
+    int range, ranges;  // range: j-bodies per CTA, a multiple of kSplitTile
 };
-
-__global__ void __launch_bounds__(256) split_extent_kernel(SplitArgs a) {
-    unsigned long long m = 0;
-    const size_t n3 = 3 * (size_t)a.n;
-    for (size_t i = blockIdx.x * 256 + threadIdx.x; i < n3; i += (size_t)gridDim.x * 256)
-        m = max(m, (unsigned long long)__double_as_longlong(fabs(a.y[i])));
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __shared__ unsigned long long w[8];
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < 8; ++k) m = max(m, w[k]);
-        a.extent[blockIdx.x] = m;
-    }
-}
-
-// exponent E with every |coordinate| < 2^E (in every thread; 2048 for a
-// coordinate that is not finite)
-__device__ __forceinline__ int split_exponent(const SplitArgs& a) {
-    unsigned long long m = 0;
-    const int lane = threadIdx.x & 31;
-    for (int k = lane; k < kSplitExtents; k += 32) m = max(m, __ldg(a.extent + k));
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const int ex = (int)(m >> 52);
-    return ex == 0x7ff ? 2048 : ex - 1022;
-}
-
-__global__ void __launch_bounds__(256) split_pack_kernel(SplitArgs a) {
-    const int ex = split_exponent(a);
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < a.n_pad; i += gridDim.x * 256) {
-        SplitBody b;
-        if (i < a.n) {
-            float h[3], m[3], l[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                split3(ex == 2048 ? nan("") : scalbn(a.y[(size_t)c * a.n + i], -ex), h[c], m[c], l[c]);
-            const double ms = a.mass[i] * a.mass_scale;
-            // a mass far below the largest is taken in FP64 throughout
-            const bool tiny = ms != 0.0 && fabs(ms) < 9.313225746154785e-10;  // 2^-30
-            const float mh = (float)ms, ml = (float)(ms - (double)mh);
-            b.a = make_float4(h[0], m[0], l[0], h[1]);
-            b.b = make_float4(m[1], l[1], h[2], m[2]);
-            b.c = make_float4(l[2], mh, ml, tiny ? __int_as_float(0x7fffffff) : fabsf(mh));
-        } else {
-            // padding: massless, and so far away that r^-3 underflows to 0
-            b.a = make_float4(1e18f, 0.f, 0.f, 1e18f);
-            b.b = make_float4(0.f, 0.f, 1e18f, 0.f);
-            b.c = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        a.bodies[i] = b;
-    }
-}
-
-// Per body, the sum of |m_j| / r^2 over a quarter of the others (32 bodies of
-// every 128; a sum without cancellation, so neither the sample nor a body in
-// the middle of a symmetric system changes its scale much).  256 bodies per
-// CTA against one of kSplitEst ranges, in FP32x2.
-__global__ void __launch_bounds__(kSplitT) split_estimate_kernel(SplitArgs a) {
-    __shared__ __align__(16) float4 tile[kSplitT][2];
-    const int tid = threadIdx.x;
-    const int i0 = blockIdx.x * 2 * kSplitT + tid, i1 = i0 + kSplitT;  // < n_pad
-    const SplitBody p = a.bodies[i0], q = a.bodies[i1];
-    const f2_t xi = f2_pack(p.a.x, q.a.x), yi = f2_pack(p.a.w, q.a.w), zi = f2_pack(p.b.z, q.b.z);
-    constexpr float kLeast = 1.f / kSplitFarP;  // closer pairs (the body itself) do not count
-    f2_t sum = f2_pack(0.f, 0.f);
-    const uint32_t base = smem_addr(tile);
-    for (int j0 = blockIdx.y * 4 * kSplitT; j0 < a.n_pad; j0 += gridDim.y * 4 * kSplitT) {
-        const int j = j0 + (tid >> 5) * kSplitT + (tid & 31);
-        __syncthreads();
-        SplitBody b = a.bodies[min(j, a.n_pad - 1)];
-        if (j >= a.n_pad) b.c.y = 0.f;
-        const float m = fabsf(b.c.y);
-        tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.w, b.a.w);
-        tile[tid][1] = make_float4(b.b.z, b.b.z, m, m);
-        __syncthreads();
-#pragma unroll 8
-        for (int k = 0; k < kSplitT; ++k) {
-            const float4 u = lds128(base + 32u * k), v = lds128(base + 32u * k + 16u);
-            const f2_t dx = f2_sub(f2_pack(u.x, u.y), xi), dy = f2_sub(f2_pack(u.z, u.w), yi);
-            const f2_t dz = f2_sub(f2_pack(v.x, v.y), zi);
-            float r0, r1;
-            f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), r0, r1);
-            const float t0 = r0 > kLeast ? rcp_mufu(r0) : 0.f, t1 = r1 > kLeast ? rcp_mufu(r1) : 0.f;
-            sum = f2_fma(f2_pack(v.z, v.w), f2_pack(t0, t1), sum);
-        }
-    }
-    float s0, s1;
-    f2_unpack(sum, s0, s1);
-    a.est[(size_t)blockIdx.y * a.n_pad + i0] = s0;
-    a.est[(size_t)blockIdx.y * a.n_pad + i1] = s1;
-}
-
-__device__ __forceinline__ float split_limit(const SplitArgs& a, int i) {
-    float s = 0.f;
-#pragma unroll
-    for (int r = 0; r < kSplitEst; ++r) s += __ldg(a.est + (size_t)r * a.n_pad + i);
-    return kSplitNear * 4.f * s;
-}
 
 template <bool UNI>
 __global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
     __shared__ __align__(16) float4 tile[kSplitTile][6];  // every word twice, for FP32x2
     __shared__ unsigned queue[2][kSplitQ][kSplitT];
     const int tid = threadIdx.x;
-    const size_t sn = (size_t)a.n;
+    const SplitSystem& s = a.s;
+    const size_t sn = (size_t)s.n;
     const int i0 = blockIdx.x * 2 * kSplitT + tid, i1 = i0 + kSplitT;  // < n_pad
     f2_t ih[3], im[3], il[3];
-    {
-        const SplitBody p = a.bodies[i0], q = a.bodies[i1];
-        ih[0] = f2_pack(p.a.x, q.a.x);
-        im[0] = f2_pack(p.a.y, q.a.y);
-        il[0] = f2_pack(p.a.z, q.a.z);
-        ih[1] = f2_pack(p.a.w, q.a.w);
-        im[1] = f2_pack(p.b.x, q.b.x);
-        il[1] = f2_pack(p.b.y, q.b.y);
-        ih[2] = f2_pack(p.b.z, q.b.z);
-        im[2] = f2_pack(p.b.w, q.b.w);
-        il[2] = f2_pack(p.c.x, q.c.x);
-    }
-    const float lim0 = split_limit(a, i0), lim1 = split_limit(a, i1);
-    const int ex = split_exponent(a);
+    split_load(s, i0, i1, ih, im, il);
+    const float lim0 = split_limit(s, i0), lim1 = split_limit(s, i1);
+    const int ex = split_exponent(s);
     // pairs at or below the clamp are taken in FP64
     const float far_p = fminf(kSplitFarP, (float)scalbn(0.999 / kMinDistance, 2 * min(max(ex, -400), 400)));
     const f2_t zero = f2_pack(0.f, 0.f);
     f2_t hi[3] = {zero, zero, zero}, lo[3] = {zero, zero, zero};
     double far0[3] = {0, 0, 0}, far1[3] = {0, 0, 0}, near0[3] = {0, 0, 0}, near1[3] = {0, 0, 0};
     int c0 = 0, c1 = 0;  // queued pairs of this thread's two bodies
-    const int j_begin = blockIdx.y * a.range, j_end = min(j_begin + a.range, a.n_pad);
+    const int j_begin = blockIdx.y * a.range, j_end = min(j_begin + a.range, s.n_pad);
 
     auto flush_queue = [&](int half, int i, int& cnt, double* acc) {
-        const int k = min(i, a.n - 1);
-        const double x1 = __ldg(a.y + k), y1 = __ldg(a.y + sn + k), z1 = __ldg(a.y + 2 * sn + k);
+        const int k = min(i, s.n - 1);
+        const double x1 = __ldg(s.y + k), y1 = __ldg(s.y + sn + k), z1 = __ldg(s.y + 2 * sn + k);
         while (__any_sync(0xffffffffu, cnt > 0)) {
             if (cnt > 0) {
                 const int j = (int)queue[half][--cnt][tid];
-                if (j != i && j < a.n)
-                    pair_fp64(__ldg(a.y + j) - x1, __ldg(a.y + sn + j) - y1,
-                              __ldg(a.y + 2 * sn + j) - z1, __ldg(a.mass + j), acc[0], acc[1],
+                if (j != i && j < s.n)
+                    pair_fp64(__ldg(s.y + j) - x1, __ldg(s.y + sn + j) - y1,
+                              __ldg(s.y + 2 * sn + j) - z1, __ldg(s.mass + j), acc[0], acc[1],
                               acc[2]);
             }
         }
@@ -310,62 +181,45 @@ __global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
 
     for (int j0 = j_begin; j0 < j_end; j0 += kSplitTile) {
         __syncthreads();
-        if (tid < kSplitTile) {
-            const SplitBody b = a.bodies[j0 + tid];
-            tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.y, b.a.y);
-            tile[tid][1] = make_float4(b.a.z, b.a.z, b.a.w, b.a.w);
-            tile[tid][2] = make_float4(b.b.x, b.b.x, b.b.y, b.b.y);
-            tile[tid][3] = make_float4(b.b.z, b.b.z, b.b.w, b.b.w);
-            tile[tid][4] = make_float4(b.c.x, b.c.x, b.c.y, b.c.y);
-            tile[tid][5] = make_float4(b.c.z, b.c.z, b.c.w, b.c.w);
-        }
+        if (tid < kSplitTile) split_store_tile(tile, s.bodies[j0 + tid]);
         __syncthreads();
         const uint32_t base = smem_addr(tile);
 #pragma unroll 1
         for (int jc = 0; jc < kSplitTile; jc += kSplitChunk) {
 #pragma unroll 2
             for (int j = jc; j < jc + kSplitChunk; ++j) {
-                const uint32_t at = base + 96u * j;
-                const float4 w0 = lds128(at), w1 = lds128(at + 16), w2 = lds128(at + 32);
-                const float4 w3 = lds128(at + 48), w4 = lds128(at + 64), w5 = lds128(at + 80);
-                f2_t d1[3], d2[3], r1, r2, w, wl;
-                split_diff(f2_pack(w0.x, w0.y), f2_pack(w0.z, w0.w), f2_pack(w1.x, w1.y), ih[0],
-                           im[0], il[0], d1[0], d2[0]);
-                split_diff(f2_pack(w1.z, w1.w), f2_pack(w2.x, w2.y), f2_pack(w2.z, w2.w), ih[1],
-                           im[1], il[1], d1[1], d2[1]);
-                split_diff(f2_pack(w3.x, w3.y), f2_pack(w3.z, w3.w), f2_pack(w4.x, w4.y), ih[2],
-                           im[2], il[2], d1[2], d2[2]);
-                split_norm2(d1, d2, r1, r2);
-                const SplitRsqrt s = split_rsqrt(r1, r2);
-                split_cube(s, w, wl);
+                const SplitPair p = split_pair(base + 96u * j, ih, im, il);
+                f2_t r1, r2, w, wl;
+                split_norm2(p.d1, p.d2, r1, r2);
+                const SplitRsqrt v = split_rsqrt(r1, r2);
+                split_cube(v, w, wl);
                 if (!UNI) {
-                    const f2_t mh = f2_pack(w4.z, w4.w), ml = f2_pack(w5.x, w5.y);
                     const f2_t c = w;
-                    w = f2_mul_rn(mh, c);
-                    wl = f2_fma(ml, c, f2_fma(mh, wl, f2_fma(mh, c, f2_neg(w))));
+                    w = f2_mul_rn(p.mh, c);
+                    wl = f2_fma(p.ml, c, f2_fma(p.mh, wl, f2_fma(p.mh, c, f2_neg(w))));
                 }
                 float p0, p1, t0, t1;
-                f2_unpack(s.p, p0, p1);
-                f2_unpack(f2_mul(s.p, f2_pack(w5.z, w5.w)), t0, t1);
+                f2_unpack(v.p, p0, p1);
+                f2_unpack(f2_mul(v.p, p.mabs), t0, t1);
                 const bool is0 = !(t0 <= lim0 && p0 <= far_p);  // NaN counts as near
                 const bool is1 = !(t1 <= lim1 && p1 <= far_p);
                 if (is0 || is1) {
-                    float u, v, lu, lv;
-                    f2_unpack(w, u, v);
-                    f2_unpack(wl, lu, lv);
+                    float u0, u1, l0, l1;
+                    f2_unpack(w, u0, u1);
+                    f2_unpack(wl, l0, l1);
                     if (is0) {
                         queue[0][c0++][tid] = (unsigned)(j0 + j);
-                        u = lu = 0.f;
+                        u0 = l0 = 0.f;
                     }
                     if (is1) {
                         queue[1][c1++][tid] = (unsigned)(j0 + j);
-                        v = lv = 0.f;
+                        u1 = l1 = 0.f;
                     }
-                    w = f2_pack(u, v);
-                    wl = f2_pack(lu, lv);
+                    w = f2_pack(u0, u1);
+                    wl = f2_pack(l0, l1);
                 }
 #pragma unroll
-                for (int k = 0; k < 3; ++k) split_axpy(hi[k], lo[k], w, wl, d1[k], d2[k]);
+                for (int k = 0; k < 3; ++k) split_axpy(hi[k], lo[k], w, wl, p.d1[k], p.d2[k]);
             }
             // the sums join the FP64 totals every 32 bodies: the error of lo grows
             // with the square of their number (the FP64 pipe is idle otherwise)
@@ -387,25 +241,25 @@ __global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
     flush_queue(0, i0, c0, near0);
     flush_queue(1, i1, c1, near1);
     // back to the caller's units: lengths 2^ex, masses 2^mass_exp
-    const int un = a.mass_exp - 2 * ex;
-    const double mu = UNI ? a.mass[0] * a.mass_scale : 1.0;
+    const int un = s.mass_exp - 2 * ex;
+    const double mu = UNI ? s.mass[0] * s.mass_scale : 1.0;
     double* out = a.part + (size_t)blockIdx.y * 3 * sn;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         // (with a coordinate that is not finite every pair is in near)
-        if (i0 < a.n) out[k * sn + i0] = near0[k] + (ex == 2048 ? 0.0 : scalbn(far0[k] * mu, un));
-        if (i1 < a.n) out[k * sn + i1] = near1[k] + (ex == 2048 ? 0.0 : scalbn(far1[k] * mu, un));
+        if (i0 < s.n) out[k * sn + i0] = near0[k] + (ex == 2048 ? 0.0 : scalbn(far0[k] * mu, un));
+        if (i1 < s.n) out[k * sn + i1] = near1[k] + (ex == 2048 ? 0.0 : scalbn(far1[k] * mu, un));
     }
 }
 
 __global__ void __launch_bounds__(128) split_reduce_kernel(SplitArgs a) {
-    const size_t sn = (size_t)a.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
+    const size_t sn = (size_t)a.s.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
     if (at >= 3 * sn) return;
     double s = 0.0;
 #pragma unroll 16
     for (int r = 0; r < a.ranges; ++r) s += __ldg(a.part + (size_t)r * 3 * sn + at);
-    a.f[at] = a.y[3 * sn + at];
-    a.f[3 * sn + at] = fp64_result(s, a.mass[at % sn]);
+    a.f[at] = a.s.y[3 * sn + at];
+    a.f[3 * sn + at] = fp64_result(s, a.s.mass[at % sn]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1013,42 +867,19 @@ nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
     const int n = (int)e->count;
     ProfScope ps(e, NBG_K_DIRECT);
     SplitArgs a;
-    a.y = y;
-    a.mass = e->d_mass;
-    a.f = f;
-    a.n = n;
-    a.n_pad = (n + 2 * kSplitT - 1) / (2 * kSplitT) * (2 * kSplitT);
-    const int blocks = a.n_pad / (2 * kSplitT);
+    const size_t system = split_bytes(&a.s, n);
+    const int blocks = a.s.n_pad / (2 * kSplitT);
     // ranges: about 8 waves of 4 CTAs per SM (the last one weighs little; 2
     // waves measured 2.2 ms instead of 1.5 at 20011 bodies), at least a tile each
     const int want = (e->sm_count * 4 * 8 + blocks - 1) / blocks;
-    const int tiles = a.n_pad / kSplitTile;
+    const int tiles = a.s.n_pad / kSplitTile;
     const int per = std::max(1, tiles / std::max(1, want));
     a.range = per * kSplitTile;
     a.ranges = (tiles + per - 1) / per;
-    const size_t bodies = (size_t)a.n_pad * sizeof(SplitBody);
-    const size_t ests = (size_t)kSplitEst * a.n_pad * sizeof(float);
-    const size_t need = bodies + ests + kSplitExtents * sizeof(unsigned long long) +
-                        (size_t)a.ranges * 3 * n * sizeof(double);
     bool split = e->tune_get("direct.fp64_split", n >= kSplitMin) != 0;
-    if (split && e->xyzm_cap < need) {
-        // no scratch (or none to be had while the stream is being captured):
-        // the kernel that needs none
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        NBG_CUDA(e, cudaStreamIsCapturing(e->stream, &cap));
-        split = false;
-        if (cap == cudaStreamCaptureStatusNone) {
-            cudaFree(e->d_xyzm);
-            e->d_xyzm = nullptr;
-            e->xyzm_cap = 0;
-            if (cudaMalloc(&e->d_xyzm, need) == cudaSuccess) {
-                e->xyzm_cap = need;
-                split = true;
-            } else {
-                cudaGetLastError();
-            }
-        }
-    }
+    // without scratch (or with none to be had while the stream is being
+    // captured): the kernel that needs none
+    split = split && reserve_scratch(e, system + (size_t)a.ranges * 3 * n * sizeof(double));
     if (!split) {
         const unsigned warps = kF64Threads / 32;
         direct_fp64_kernel<<<((unsigned)n + warps - 1) / warps, kF64Threads, 0, e->stream>>>(
@@ -1056,19 +887,10 @@ nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
         NBG_LAUNCHED(e, "direct_fp64_kernel");
         return NBG_OK;
     }
-    char* at = reinterpret_cast<char*>(e->d_xyzm);
-    a.bodies = reinterpret_cast<SplitBody*>(at);
-    a.extent = reinterpret_cast<unsigned long long*>(at + bodies);
-    a.part = reinterpret_cast<double*>(at + bodies + kSplitExtents * sizeof(unsigned long long));
-    a.est = reinterpret_cast<float*>(a.part + (size_t)a.ranges * 3 * n);
-    a.mass_exp = e->mass_exp;
-    a.mass_scale = std::ldexp(1.0, -e->mass_exp);
-    split_extent_kernel<<<kSplitExtents, 256, 0, e->stream>>>(a);
-    NBG_LAUNCHED(e, "split_extent_kernel");
-    split_pack_kernel<<<grid_for(a.n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(a);
-    NBG_LAUNCHED(e, "split_pack_kernel");
-    split_estimate_kernel<<<dim3((unsigned)blocks, kSplitEst), kSplitT, 0, e->stream>>>(a);
-    NBG_LAUNCHED(e, "split_estimate_kernel");
+    a.f = f;
+    a.part = reinterpret_cast<double*>(reinterpret_cast<char*>(e->d_xyzm) + system);
+    nbg_status s = split_prepare<false>(e, &a.s, y, e->d_mass, 0.0, e->d_xyzm);
+    if (s != NBG_OK) return s;
     const dim3 grid((unsigned)blocks, (unsigned)a.ranges);
     if (e->uniform_mass)
         split_force_kernel<true><<<grid, kSplitT, 0, e->stream>>>(a);

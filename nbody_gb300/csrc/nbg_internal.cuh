@@ -54,7 +54,7 @@ struct nbg_engine {
     double mass_value = 0.0;
     int mass_exp = 0;            // largest finite |mass| < 2^mass_exp
 
-    // direct-sum scratch: packed FP32 bodies (x, y, z, m), padded to tiles
+    // scratch of one call (packed bodies, partial sums), kept and grown
     float4* d_xyzm = nullptr;
     size_t xyzm_cap = 0;
 
@@ -103,6 +103,24 @@ nbg_status cuda_error(nbg_engine* e, cudaError_t err, const char* what);
         cudaError_t _err = cudaGetLastError();                     \
         if (_err != cudaSuccess) return nbg::cuda_error(e, _err, what); \
     } while (0)
+
+// At least `bytes` of e->d_xyzm: false (and the old block kept, or none) when
+// they cannot be had, which includes a growth while the stream is captured.
+inline bool reserve_scratch(nbg_engine* e, size_t bytes) {
+    if (e->xyzm_cap >= bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        return false;
+    cudaFree(e->d_xyzm);
+    e->d_xyzm = nullptr;
+    e->xyzm_cap = 0;
+    if (cudaMalloc(&e->d_xyzm, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    e->xyzm_cap = bytes;
+    return true;
+}
 
 // ---- profiling: bracket a kernel class with events on the engine stream ----
 void prof_begin(nbg_engine* e, int kid, cudaEvent_t* ev);
