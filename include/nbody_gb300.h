@@ -290,6 +290,9 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  *       "direct.fp64_split" (1: the FP64 direct sum in two-word FP32
  *       arithmetic with its large terms in FP64, the default from 1536
  *       bodies on; 0: every pair on the FP64 pipe),
+ *       "bh.fp64_split" (1, the default: the FP64 walk's sums in two-word FP32
+ *       arithmetic with the large terms in FP64; 0: one thread per body on
+ *       the FP64 pipe),
  *       "statistics.split_min" (bodies from which nbg_statistics sums the
  *       potential in two-word FP32 arithmetic, default 3072),
  *       "direct.uniform_mass" (1, the default: when every body has the same

@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "nbg_ptx.cuh"
+#include "nbg_split_sys.cuh"
 #include "nbg_tree.cuh"
 
 namespace nbg {
@@ -108,6 +109,334 @@ __global__ void bh_walk_fp64_kernel(const double* __restrict__ y, const double* 
     f[3 * n + b] = __ddiv_rn(fx, m1);
     f[4 * n + b] = __ddiv_rn(fy, m1);
     f[5 * n + b] = __ddiv_rn(fz, m1);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 walk on the FP32 pipe
+// ---------------------------------------------------------------------------
+// A group of 64 consecutive leaves, two per lane, is walked by `parts` warps
+// that share the tree.  A warp walks nodes with the set of bodies that opened
+// the parent (two 32-bit masks per stack entry, which stands for both
+// children), so every body meets exactly the nodes of its own walk, and a
+// node's record is read once for all 64.  A step tests 32 nodes, one per
+// lane, against the bounding box of the 64 bodies: most are accepted or
+// opened by every body whatever its place in the box; the others (a quarter
+// in a Plummer sphere) are tested body by body, in FP32 outside a margin of
+// 2^-20 around the critical radius and by the reference's FP64 expression
+// inside it.  Accepted nodes are listed and summed as in the direct sum
+// (split_force_kernel): two-word terms; large ones (t > kSplitNear of the
+// body's scale) and close ones are queued per body and taken in FP64.
+// Nodes above level `top` are tested by every part and summed by one, the
+// subtrees under that level are dealt out to the parts; split_walk_sum_kernel
+// adds the parts in order, so equal states give equal forces.
+//
+// Bound by instruction issue and latency (16 warps of 128 registers per SM):
+// 2^15 bodies of a Plummer sphere at ratio 2 (2448 interactions a body) in
+// 1.4 ms, 2^18 in 26 ms and 2^20 in 0.21 s with the kd build; one thread per
+// body on the FP64 pipe 18.4 ms, 0.49 s and 4.66 s, testing every node body
+// by body 2.0 ms, 43 ms and - (59 % of the time).  Fewer, larger parts leave
+// SMs idle at the end (2^18 bodies: 32 ms with 1 part, 27 with 4), more repeat
+// the top of the tree (2^15 bodies of a uniform cube: 1.70 ms with 16, 1.79
+// with 32).
+constexpr int kSWStack = 320;   // see the pop rule
+constexpr int kSWList = 64;     // accepted nodes: fewer than 32 before a step adds at most 32
+constexpr int kSWQ = 16;        // queued nodes per body
+constexpr int kSWWarps = 16384;  // warps wanted: parts = kSWWarps / groups, 2 to 16
+
+struct SplitWalkArgs {
+    SplitSystem s;
+    TreeState t;
+    double* part;  // [parts][3][n], leaf order
+    int parts, top;
+};
+
+// 64 bytes per node: SplitBody, then crit2 (1 + 2^-20), crit2 (1 - 2^-20) in
+// scaled units
+struct SplitNode {
+    SplitBody b;
+    float4 crit;
+};
+
+__global__ void __launch_bounds__(256) split_nodes_kernel(SplitSystem s, TreeState t) {
+    const int ex = split_exponent(s);
+    for (size_t i = 1 + blockIdx.x * (size_t)256 + threadIdx.x; i < t.size; i += (size_t)gridDim.x * 256) {
+        // with masses of both signs a centre may lie outside the bodies'
+        // extent, where the words do not reach: such a node is tested and
+        // summed in FP64 (crit and |m| that no FP32 comparison passes)
+        bool inside = true;
+        float h[3], m[3], l[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double x = scalbn(t.com[c * t.size + i], -min(ex, 1100));
+            inside = inside && fabs(x) < 1.0;
+            split3(ex == 2048 ? nan("") : fabs(x) < 1.0 ? x : 0.0, h[c], m[c], l[c]);
+        }
+        const double ms = t.mass[i] * s.mass_scale;
+        const bool tiny = ms != 0.0 && fabs(ms) < 9.313225746154785e-10;  // as in split_pack_kernel
+        const float mh = (float)ms, ml = (float)(ms - (double)mh);
+        const double cr = scalbn(t.crit2[i], -2 * min(ex, 1000));
+        SplitNode& o = reinterpret_cast<SplitNode*>(t.split)[i];
+        o.b.a = make_float4(h[0], m[0], l[0], h[1]);
+        o.b.b = make_float4(m[1], l[1], h[2], m[2]);
+        const float none = __int_as_float(0x7fffffff);
+        o.b.c = make_float4(l[2], mh, ml, tiny || !inside ? none : fabsf(mh));
+        o.crit = make_float4(inside ? (float)(cr * (1.0 + 9.5367431640625e-07)) : none,
+                             inside ? (float)(cr * (1.0 - 9.5367431640625e-07)) : none, 0.f, 0.f);
+    }
+}
+
+// the reference's acceptance test (nbody/nbody_space_heap_stackless.cpp:3-28)
+__device__ __noinline__ bool accept_fp64(const TreeState& t, size_t node, size_t leaf) {
+    const size_t sz = t.size;
+    const double dx = __dsub_rn(t.com[leaf], t.com[node]);
+    const double dy = __dsub_rn(t.com[sz + leaf], t.com[sz + node]);
+    const double dz = __dsub_rn(t.com[2 * sz + leaf], t.com[2 * sz + node]);
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)) > t.crit2[node];
+}
+
+__global__ void __launch_bounds__(32, 16) bh_walk_split_kernel(SplitWalkArgs a) {
+    __shared__ uint3 stack[kSWStack];
+    __shared__ uint3 list[kSWList + 1];  // node, bodies that accepted it (two masks)
+    __shared__ unsigned queue[2][kSWQ][32];
+    const SplitSystem& s = a.s;
+    const TreeState& t = a.t;
+    const int lane = threadIdx.x;
+    const int n = s.n;
+    const size_t sz = t.size;
+    const int k0 = min(blockIdx.x * 64 + lane, n - 1), k1 = min(blockIdx.x * 64 + 32 + lane, n - 1);
+    const SplitNode* nodes = reinterpret_cast<const SplitNode*>(t.split);
+    f2_t ih[3], im[3], il[3];
+    split_words(nodes[n + k0].b, nodes[n + k1].b, ih, im, il);
+    const float lim0 = split_limit(s, t.body_n[n + k0]), lim1 = split_limit(s, t.body_n[n + k1]);
+    const int ex = split_exponent(s);
+    const float far_p = fminf(kSplitFarP, (float)scalbn(0.999 / kMinDistance, 2 * min(max(ex, -400), 400)));
+    const f2_t zero = f2_pack(0.f, 0.f);
+    f2_t hi[3] = {zero, zero, zero}, lo[3] = {zero, zero, zero};
+    double far0[3] = {0, 0, 0}, far1[3] = {0, 0, 0}, near0[3] = {0, 0, 0}, near1[3] = {0, 0, 0};
+    int c0 = 0, c1 = 0;  // queued nodes of this lane's two bodies
+    unsigned long long visits = 0, inter = 0;
+    auto fold = [&]() {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            float h0, h1, l0, l1;
+            f2_unpack(hi[k], h0, h1);
+            f2_unpack(lo[k], l0, l1);
+            far0[k] += (double)h0 + (double)l0;
+            far1[k] += (double)h1 + (double)l1;
+            hi[k] = lo[k] = zero;
+        }
+    };
+    auto flush_queue = [&](int half, int k, int& cnt, double* acc) {
+        const double x = t.com[n + k], y = t.com[sz + n + k], z = t.com[2 * sz + n + k];
+        while (__any_sync(0xffffffffu, cnt > 0)) {
+            if (cnt > 0) {
+                const size_t c = queue[half][--cnt][lane];
+                pair_fp64(__ldg(t.com + c) - x, __ldg(t.com + sz + c) - y,
+                          __ldg(t.com + 2 * sz + c) - z, __ldg(t.mass + c), acc[0], acc[1], acc[2]);
+            }
+        }
+    };
+
+    // sums the listed nodes, two independent terms in flight
+    auto evaluate = [&](int count) {
+        if (count & 1) {
+            if (lane == 0) list[count] = make_uint3(1u, 0u, 0u);
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int e = 0; e < ((count + 1) & ~1); ++e) {
+            const uint3 en = list[e];
+            const SplitNode& r = nodes[en.x];
+            const float4 ra = __ldg(&r.b.a), rb = __ldg(&r.b.b), rc = __ldg(&r.b.c);
+            f2_t d1[3], d2[3], r1, r2, w, wl;
+            split_diff(f2_pack(ra.x, ra.x), f2_pack(ra.y, ra.y), f2_pack(ra.z, ra.z), ih[0], im[0],
+                       il[0], d1[0], d2[0]);
+            split_diff(f2_pack(ra.w, ra.w), f2_pack(rb.x, rb.x), f2_pack(rb.y, rb.y), ih[1], im[1],
+                       il[1], d1[1], d2[1]);
+            split_diff(f2_pack(rb.z, rb.z), f2_pack(rb.w, rb.w), f2_pack(rc.x, rc.x), ih[2], im[2],
+                       il[2], d1[2], d2[2]);
+            split_norm2(d1, d2, r1, r2);
+            const SplitRsqrt v = split_rsqrt(r1, r2);
+            split_cube(v, w, wl);
+            const f2_t mh = f2_pack(rc.y, rc.y), ml = f2_pack(rc.z, rc.z), cw = w;
+            w = f2_mul_rn(mh, cw);
+            wl = f2_fma(ml, cw, f2_fma(mh, wl, f2_fma(mh, cw, f2_neg(w))));
+            float p0, p1, u0, u1, l0, l1;
+            f2_unpack(v.p, p0, p1);
+            f2_unpack(w, u0, u1);
+            f2_unpack(wl, l0, l1);
+            const bool in0 = (en.y >> lane) & 1u, in1 = (en.z >> lane) & 1u;
+            const bool far_0 = in0 && p0 * rc.w <= lim0 && p0 <= far_p;
+            const bool far_1 = in1 && p1 * rc.w <= lim1 && p1 <= far_p;
+            if (in0 && !far_0) queue[0][c0++][lane] = en.x;
+            if (in1 && !far_1) queue[1][c1++][lane] = en.x;
+            w = f2_pack(far_0 ? u0 : 0.f, far_1 ? u1 : 0.f);
+            wl = f2_pack(far_0 ? l0 : 0.f, far_1 ? l1 : 0.f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) split_axpy(hi[k], lo[k], w, wl, d1[k], d2[k]);
+            if ((e & 1) != 0) {
+                if (__any_sync(0xffffffffu, c0 >= kSWQ - 1)) flush_queue(0, k0, c0, near0);
+                if (__any_sync(0xffffffffu, c1 >= kSWQ - 1)) flush_queue(1, k1, c1, near1);
+            }
+            if ((e & 3) == 3) {
+                // lo back below the last place of hi, so that its own rounding
+                // stays small until the fold (4096 terms: RMS error 1.1e-15;
+                // 2.6e-15 once per evaluation; the serial FP64 sum 1.7e-15)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const f2_t h = f2_add(hi[k], lo[k]);
+                    lo[k] = f2_sub(lo[k], f2_sub(h, hi[k]));
+                    hi[k] = h;
+                }
+            }
+        }
+        fold();
+        __syncwarp();
+    };
+
+    // the group's box (FP32, unscaled), with a margin that covers the rounding
+    // of the bodies' and the nodes' coordinates
+    float cb[3], hb[3];
+    {
+        const float4 p = __ldg(&t.node4[n + k0]), q = __ldg(&t.node4[n + k1]);
+        float lo3[3] = {fminf(p.x, q.x), fminf(p.y, q.y), fminf(p.z, q.z)};
+        float hi3[3] = {fmaxf(p.x, q.x), fmaxf(p.y, q.y), fmaxf(p.z, q.z)};
+        const float margin = scalbnf(1.f, min(ex, 200) - 21);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            for (int o = 16; o > 0; o >>= 1) {
+                lo3[c] = fminf(lo3[c], __shfl_xor_sync(0xffffffffu, lo3[c], o));
+                hi3[c] = fmaxf(hi3[c], __shfl_xor_sync(0xffffffffu, hi3[c], o));
+            }
+            cb[c] = 0.5f * (lo3[c] + hi3[c]);
+            hb[c] = 0.5f * (hi3[c] - lo3[c]) + margin;
+        }
+    }
+    const unsigned lt = (1u << lane) - 1u;
+    // entry 0 stands for the unused slot 0 and the root
+    {
+        const unsigned v0 = __ballot_sync(0xffffffffu, blockIdx.x * 64 + lane < n);
+        const unsigned v1 = __ballot_sync(0xffffffffu, blockIdx.x * 64 + 32 + lane < n);
+        if (lane == 0) stack[0] = make_uint3(0u, v0, v1);
+    }
+    __syncwarp();
+    int sp = 1, lc = 0;
+    while (sp > 0) {
+        // 16 entries a step; one at a time (which grows the stack by at most
+        // one entry per level) once the stack is nearly full
+        const int k = sp > kSWStack - 64 ? 1 : min(sp, 16);
+        uint3 en = make_uint3(0u, 0u, 0u);
+        unsigned node = 0u;
+        if (lane < 2 * k) {
+            en = stack[sp - 1 - (lane >> 1)];
+            node = 2u * en.x + (lane & 1);
+        }
+        __syncwarp();
+        sp -= k;
+        const int lv = 31 - __clz(node);
+        const bool mine = (node & (a.parts - 1u)) == blockIdx.y;
+        if (lv == a.top && !mine) node = 0u;
+        bool all_in = false, all_out = false;
+        if (node != 0u) {
+            const float4 nd = __ldg(&t.node4[node]);
+            float in2 = 0.f, out2 = 0.f;
+            const float dc[3] = {fabsf(nd.x - cb[0]), fabsf(nd.y - cb[1]), fabsf(nd.z - cb[2])};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float u = fmaxf(dc[c] - hb[c], 0.f), v = dc[c] + hb[c];
+                in2 = fmaf(u, u, in2);
+                out2 = fmaf(v, v, out2);
+            }
+            all_in = in2 > nd.w * 1.00001f && in2 > 1e-30f;
+            all_out = out2 < nd.w * 0.99999f && nd.w > 1e-30f && node < (unsigned)n;
+        }
+        const bool sum = lv > a.top || mine;
+        if (node != 0u && (all_in || all_out) && sum) {
+            const int bodies = __popc(en.y) + __popc(en.z);
+            visits += bodies;
+            inter += all_in ? bodies : 0;
+        }
+        const unsigned li = __ballot_sync(0xffffffffu, all_in && sum);
+        if (all_in && sum) list[lc + __popc(li & lt)] = make_uint3(node, en.y, en.z);
+        lc += __popc(li);
+        const unsigned oi = __ballot_sync(0xffffffffu, all_out);
+        if (all_out) stack[sp + __popc(oi & lt)] = make_uint3(node, en.y, en.z);
+        sp += __popc(oi);
+        // the rest body by body
+        unsigned rest = __ballot_sync(0xffffffffu, node != 0u && !all_in && !all_out);
+        while (rest != 0u) {
+            const int src = __ffs(rest) - 1;
+            rest &= rest - 1;
+            const unsigned nr = __shfl_sync(0xffffffffu, node, src);
+            const unsigned m0 = __shfl_sync(0xffffffffu, en.y, src);
+            const unsigned m1 = __shfl_sync(0xffffffffu, en.z, src);
+            const bool sr = __shfl_sync(0xffffffffu, (int)sum, src) != 0;
+            const SplitNode& r = nodes[nr];
+            const float4 ra = __ldg(&r.b.a), rb = __ldg(&r.b.b), cr = __ldg(&r.crit);
+            const f2_t dx = f2_add(f2_sub(f2_pack(ra.x, ra.x), ih[0]), f2_sub(f2_pack(ra.y, ra.y), im[0]));
+            const f2_t dy = f2_add(f2_sub(f2_pack(ra.w, ra.w), ih[1]), f2_sub(f2_pack(rb.x, rb.x), im[1]));
+            const f2_t dz = f2_add(f2_sub(f2_pack(rb.z, rb.z), ih[2]), f2_sub(f2_pack(rb.w, rb.w), im[2]));
+            float r0, r1;
+            f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), r0, r1);
+            bool a0 = r0 > cr.x, a1 = r1 > cr.x;
+            const bool sure0 = a0 ? r0 > 1e-24f : r0 < cr.y && cr.y > 1e-24f;
+            const bool sure1 = a1 ? r1 > 1e-24f : r1 < cr.y && cr.y > 1e-24f;
+            if (!sure0) a0 = accept_fp64(t, nr, n + k0);
+            if (!sure1) a1 = accept_fp64(t, nr, n + k1);
+            const unsigned A0 = __ballot_sync(0xffffffffu, a0) & m0;
+            const unsigned A1 = __ballot_sync(0xffffffffu, a1) & m1;
+            const unsigned o0 = m0 & ~A0, o1 = m1 & ~A1;
+            if (lane == 0) {
+                if (sr) {
+                    visits += __popc(m0) + __popc(m1);
+                    inter += __popc(A0) + __popc(A1);
+                    if ((A0 | A1) != 0u) list[lc] = make_uint3(nr, A0, A1);
+                }
+                if ((o0 | o1) != 0u && nr < (unsigned)n) stack[sp] = make_uint3(nr, o0, o1);
+            }
+            lc += sr && (A0 | A1) != 0u ? 1 : 0;
+            sp += (o0 | o1) != 0u && nr < (unsigned)n ? 1 : 0;
+        }
+        __syncwarp();
+        if (lc >= 32) {
+            evaluate(lc);
+            lc = 0;
+        }
+    }
+    evaluate(lc);
+    fold();
+    flush_queue(0, k0, c0, near0);
+    flush_queue(1, k1, c1, near1);
+    const int un = s.mass_exp - 2 * ex;
+    double* out = a.part + (size_t)blockIdx.y * 3 * n;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (blockIdx.x * 64 + lane < n)
+            out[(size_t)k * n + k0] = near0[k] + (ex == 2048 ? 0.0 : scalbn(far0[k], un));
+        if (blockIdx.x * 64 + 32 + lane < n)
+            out[(size_t)k * n + k1] = near1[k] + (ex == 2048 ? 0.0 : scalbn(far1[k], un));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        visits += __shfl_xor_sync(0xffffffffu, visits, o);
+        inter += __shfl_xor_sync(0xffffffffu, inter, o);
+    }
+    if (lane == 0) {
+        atomicAdd(&t.counters[0], visits);
+        atomicAdd(&t.counters[1], inter);
+    }
+}
+
+__global__ void __launch_bounds__(128)
+split_walk_sum_kernel(SplitWalkArgs a, const double* __restrict__ y, double* __restrict__ f) {
+    const size_t n = (size_t)a.s.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (at >= 3 * n) return;
+    const int b = a.t.body_n[n + at % n];
+    double s = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < a.parts; ++p) s += __ldg(a.part + (size_t)p * 3 * n + at);
+    const size_t row = at / n * n + b;
+    f[row] = y[3 * n + row];
+    f[3 * n + row] = fp64_result(s, a.s.mass[b]);
 }
 
 // Warp-coherent FP32 walk; acceleration a_i = sum m (c - x_i) (d^2 + eps^2)^-3/2.
@@ -1070,6 +1399,29 @@ nbg_status bh_fcompute(nbg_engine* e, uint64_t step, const double* y, double* f)
         nbg_status s = bh_tree(e, step, y, true, lambda);
         if (s != NBG_OK) return s;
         ProfScope ps(e, NBG_K_BH_WALK);
+        SplitWalkArgs a;
+        const size_t system = split_bytes(&a.s, n);
+        const int groups = (n + 63) / 64;
+        a.parts = 2;
+        while (a.parts < 16 && a.parts * groups < kSWWarps) a.parts *= 2;
+        a.top = 0;
+        while ((1 << a.top) < 4 * a.parts) ++a.top;
+        // (without scratch for it, one thread per body on the FP64 pipe)
+        if (e->tree->split != nullptr && e->tune_get("bh.fp64_split", 1) != 0 &&
+            reserve_scratch(e, system + (size_t)a.parts * 3 * n * sizeof(double))) {
+            s = split_prepare<false>(e, &a.s, y, e->d_mass, 0.0, e->d_xyzm);
+            if (s != NBG_OK) return s;
+            a.t = *e->tree;
+            a.part = reinterpret_cast<double*>(reinterpret_cast<char*>(e->d_xyzm) + system);
+            split_nodes_kernel<<<grid_for(2 * (size_t)n, 256, (unsigned)e->sm_count * 8u), 256, 0,
+                                 e->stream>>>(a.s, a.t);
+            NBG_LAUNCHED(e, "split_nodes_kernel");
+            bh_walk_split_kernel<<<dim3((unsigned)groups, (unsigned)a.parts), 32, 0, e->stream>>>(a);
+            NBG_LAUNCHED(e, "bh_walk_split_kernel");
+            split_walk_sum_kernel<<<(unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream>>>(a, y, f);
+            NBG_LAUNCHED(e, "split_walk_sum_kernel");
+            return NBG_OK;
+        }
         bh_walk_fp64_kernel<<<(n + 127) / 128, 128, 0, e->stream>>>(
             y, e->d_mass, f, n, e->params.traverse_type == NBG_TRAVERSE_NESTED_TREE ? 1 : 0,
             *e->tree, e->d_err);

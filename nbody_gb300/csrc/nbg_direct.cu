@@ -67,24 +67,6 @@ __device__ __forceinline__ void pair2(f2_t xj, f2_t yj, f2_t zj, f2_t mj, f2_t x
 // ---------------------------------------------------------------------------
 // FP64 kernels
 // ---------------------------------------------------------------------------
-// One body of the FP64 sum: a += m_j d r^-3, r^2 at least kMinDistance (16 FP64
-// operations; the reference's pair force, nbody/nbody_data.cpp:35-44, without
-// its multiplication and division by m_i).
-__device__ __forceinline__ void pair_fp64(double dx, double dy, double dz, double m, double& ax,
-                                          double& ay, double& az) {
-    const double r2 = fmax(fma(dx, dx, fma(dy, dy, dz * dz)), kMinDistance);
-    const double w = m * rcube_fp64(r2);
-    ax = fma(dx, w, ax);
-    ay = fma(dy, w, ay);
-    az = fma(dz, w, az);
-}
-
-// The reference forms the force with m_i and divides by m_i again: for a
-// massless or non-finite m_i that is NaN.
-__device__ __forceinline__ double fp64_result(double a, double m) {
-    return m != 0.0 && fabs(m) <= 1.7976931348623157e308 ? a : a * m / m;
-}
-
 // Small systems (and any size, where the split path's scratch cannot be had):
 // one warp per body, the other bodies across its lanes, the 32 partial sums
 // added by shuffles in a fixed order.

@@ -20,6 +20,24 @@ constexpr int kSplitChunk = 8;               // j-bodies between two looks at th
 constexpr int kSplitExtents = 64;            // CTAs of split_extent_kernel
 constexpr int kSplitEst = 8;                 // ranges of split_estimate_kernel
 
+// One body of the FP64 sum: a += m_j d r^-3, r^2 at least kMinDistance (16 FP64
+// operations; the reference's pair force, nbody/nbody_data.cpp:35-44, without
+// its multiplication and division by m_i).
+__device__ __forceinline__ void pair_fp64(double dx, double dy, double dz, double m, double& ax,
+                                          double& ay, double& az) {
+    const double r2 = fmax(fma(dx, dx, fma(dy, dy, dz * dz)), kMinDistance);
+    const double w = m * rcube_fp64(r2);
+    ax = fma(dx, w, ax);
+    ay = fma(dy, w, ay);
+    az = fma(dz, w, az);
+}
+
+// The reference forms the force with m_i and divides by m_i again: for a
+// massless or non-finite m_i that is NaN.
+__device__ __forceinline__ double fp64_result(double a, double m) {
+    return m != 0.0 && fabs(m) <= 1.7976931348623157e308 ? a : a * m / m;
+}
+
 struct SplitBody {  // 48 bytes
     float4 a;       // xh xm xl yh
     float4 b;       // ym yl zh zm
@@ -36,6 +54,7 @@ struct SplitSystem {
     double mass_scale;           // power of two: largest |m| into [1/2, 1)
     int mass_exp;                // mass_scale = 2^-mass_exp
     int n, n_pad;                // n_pad: a multiple of 2 kSplitT
+    int sample;                  // the estimate takes 32 of every 32 sample bodies
 };
 
 __global__ void __launch_bounds__(256) split_extent_kernel(SplitSystem a) {
@@ -105,11 +124,13 @@ __global__ void __launch_bounds__(kSplitT) split_estimate_kernel(SplitSystem a) 
     const float eps2 = POT ? (float)scalbn(a.eps2, -2 * min(split_exponent(a), 1000)) : 0.f;
     f2_t sum = f2_pack(0.f, 0.f);
     const uint32_t base = smem_addr(tile);
-    for (int j0 = blockIdx.y * 4 * kSplitT; j0 < a.n_pad; j0 += gridDim.y * 4 * kSplitT) {
-        const int j = j0 + (tid >> 5) * kSplitT + (tid & 31);
+    // 4 runs of 32 bodies per tile
+    const int runs = a.n_pad / 32, tiles = (runs / a.sample + 3) / 4;
+    for (int q = blockIdx.y; q < max(tiles, 1); q += gridDim.y) {
+        const int run = (q * 4 + (tid >> 5)) * a.sample;
         __syncthreads();
-        SplitBody b = a.bodies[min(j, a.n_pad - 1)];
-        if (j >= a.n_pad) b.c.y = 0.f;
+        SplitBody b = a.bodies[min(run, runs - 1) * 32 + (tid & 31)];
+        if (run >= runs) b.c.y = 0.f;
         const float m = fabsf(b.c.y);
         tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.w, b.a.w);
         tile[tid][1] = make_float4(b.b.z, b.b.z, m, m);
@@ -136,13 +157,12 @@ __device__ __forceinline__ float split_limit(const SplitSystem& a, int i) {
     float s = 0.f;
 #pragma unroll
     for (int r = 0; r < kSplitEst; ++r) s += __ldg(a.est + (size_t)r * a.n_pad + i);
-    return kSplitNear * 4.f * s;
+    return kSplitNear * (float)a.sample * s;
 }
 
-// The three words of bodies i0 and i1, packed.
-__device__ __forceinline__ void split_load(const SplitSystem& a, int i0, int i1, f2_t* h, f2_t* m,
-                                           f2_t* l) {
-    const SplitBody p = a.bodies[i0], q = a.bodies[i1];
+// The three words of two bodies, packed.
+__device__ __forceinline__ void split_words(const SplitBody& p, const SplitBody& q, f2_t* h, f2_t* m,
+                                            f2_t* l) {
     h[0] = f2_pack(p.a.x, q.a.x);
     m[0] = f2_pack(p.a.y, q.a.y);
     l[0] = f2_pack(p.a.z, q.a.z);
@@ -152,6 +172,10 @@ __device__ __forceinline__ void split_load(const SplitSystem& a, int i0, int i1,
     h[2] = f2_pack(p.b.z, q.b.z);
     m[2] = f2_pack(p.b.w, q.b.w);
     l[2] = f2_pack(p.c.x, q.c.x);
+}
+__device__ __forceinline__ void split_load(const SplitSystem& a, int i0, int i1, f2_t* h, f2_t* m,
+                                           f2_t* l) {
+    split_words(a.bodies[i0], a.bodies[i1], h, m, l);
 }
 
 // A shared-memory tile holds every word twice, for FP32x2: the first
@@ -191,6 +215,8 @@ __device__ __forceinline__ SplitPair split_pair(uint32_t at, const f2_t* h, cons
 size_t split_bytes(SplitSystem* a, int n) {
     a->n = n;
     a->n_pad = (n + 2 * kSplitT - 1) / (2 * kSplitT) * (2 * kSplitT);
+    a->sample = 4;
+    while (a->n_pad / a->sample > 16384) a->sample *= 2;
     return (size_t)a->n_pad * (sizeof(SplitBody) + kSplitEst * sizeof(float)) +
            kSplitExtents * sizeof(unsigned long long);
 }

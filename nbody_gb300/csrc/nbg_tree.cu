@@ -567,6 +567,11 @@ nbg_status tree_alloc(nbg_engine* e) {
     NBG_TRY(alloc(e, &t->box4, 2 * sz));
     NBG_TRY(alloc(e, &t->counters, 5));
 #undef NBG_TRY
+    if (e->params.precision == NBG_PREC_FP64 &&
+        cudaMalloc(&t->split, 4 * sz * sizeof(float4)) != cudaSuccess) {
+        cudaGetLastError();  // the walk that needs no records runs
+        t->split = nullptr;
+    }
     // index 0 is unused; zero everything once so stray reads are defined
     NBG_CUDA(e, cudaMemsetAsync(t->node4, 0, sz * sizeof(float4), e->stream));
     NBG_CUDA(e, cudaMemsetAsync(t->nodem, 0, sz * sizeof(float), e->stream));
@@ -639,7 +644,7 @@ void tree_destroy(nbg_engine* e) {
                     t->lists[2], t->spare[0], t->spare[1], t->flag, t->tile_count, t->hist, t->totals, t->box,
                     t->fb_list, t->fb_count, t->cap_state,
                     t->com, t->mass, t->bmin, t->bmax, t->crit2, t->body_n, t->node4,
-                    t->nodem, t->box4, t->feat, t->quad, t->counters, t->node4_acc,
+                    t->nodem, t->split, t->box4, t->feat, t->quad, t->counters, t->node4_acc,
                     t->leaf_lo};
     for (void* p : ptrs) cudaFree(p);
     delete t;

@@ -38,6 +38,10 @@ struct TreeState {
     double* crit2 = nullptr;  // [size] (lambda * r)^2, 0 for leaves
     int* body_n = nullptr;    // [size] body of a leaf
 
+    // node records of the FP64 walk on the FP32 pipe (nbg_bh.cu, 64 bytes
+    // each), or null: FP64 engines that have the memory
+    float4* split = nullptr;  // [4 size]
+
     // FP32 node records for the mixed-precision walk: (com.xyz, crit2), mass
     float4* node4 = nullptr;  // [size]
     float* nodem = nullptr;   // [size]
