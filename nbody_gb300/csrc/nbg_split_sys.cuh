@@ -216,7 +216,7 @@ size_t split_bytes(SplitSystem* a, int n) {
     a->n = n;
     a->n_pad = (n + 2 * kSplitT - 1) / (2 * kSplitT) * (2 * kSplitT);
     a->sample = 4;
-    while (a->n_pad / a->sample > 16384) a->sample *= 2;
+    while (a->n_pad / a->sample > 4096) a->sample *= 2;
     return (size_t)a->n_pad * (sizeof(SplitBody) + kSplitEst * sizeof(float)) +
            kSplitExtents * sizeof(unsigned long long);
 }

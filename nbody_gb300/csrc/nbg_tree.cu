@@ -28,6 +28,8 @@
 // bits from 16 up, leaf p = the p-th body along the curve, every node the
 // union of its two halves; mixed precision updates the nodes in FP32 from
 // FP32 boxes when no FP64 node arrays are needed.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 
@@ -44,6 +46,20 @@ constexpr int kDigits = 256;
 __device__ __forceinline__ uint64_t order_key(double v) {
     const uint64_t b = (uint64_t)__double_as_longlong(v);
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+
+// Lanes with this lane's digit (8 bits), by one ballot per bit: the ballots of
+// several digits are independent and overlap, where __match_any_sync takes a
+// step per distinct value.
+__device__ __forceinline__ unsigned digit_peers(unsigned dig) {
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool set = (dig >> b) & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, set);
+        peers &= set ? m : ~m;
+    }
+    return peers;
 }
 
 __global__ void init_keys_kernel(const double* __restrict__ coord, int n,
@@ -256,7 +272,9 @@ radix_scatter_kernel(const uint64_t* __restrict__ kin, const int* __restrict__ v
         key[r] = live ? kin[i] : 0ull;
         val[r] = live ? vin[i] : 0;
         dig[r] = live ? ((unsigned)(key[r] >> shift) & 0xFFu) : kDigits;  // kDigits = dead
-        const unsigned peers = __match_any_sync(0xffffffffu, dig[r]);
+        // (dead lanes, past the last key, have the digit 0 of live ones here:
+        // they come after them and are not counted)
+        const unsigned peers = digit_peers(dig[r] & 0xFFu) & __ballot_sync(0xffffffffu, live);
         const unsigned before = __popc(peers & lt);
         const int leader = __ffs(peers) - 1;
         unsigned b = 0;
@@ -299,6 +317,158 @@ radix_scatter_kernel(const uint64_t* __restrict__ kin, const int* __restrict__ v
         const unsigned dst = gbase[d] + (unsigned)j - lbase[d];
         kout[dst] = k;
         vout[dst] = sval[j];
+    }
+}
+
+// ---- sorts of up to 32768 keys: one cluster in one launch ----
+// The keys stay in the shared memory of a cluster of up to 8 CTAs (4096 keys
+// each) for all passes; a pass ranks its keys as radix_scatter_kernel does,
+// exchanges the CTAs' digit counts through distributed shared memory and
+// stores every key to its place in the cluster's other buffer.  The
+// multi-launch sort spends 3 launches (18 us) on a pass of so few keys, a
+// handful of CTAs each: 105 us for the 6 passes of 16384 curve keys and 432 us
+// for the 24 of 32768 bodies' coordinates, against 31 us and 65 us here (5 and
+// 8 us a pass of 2048 and 4096 keys per CTA).
+constexpr int kCSThreads = 512;
+constexpr int kCSWarps = kCSThreads / 32;
+constexpr int kCSCtas = 8;                        // portable cluster size
+constexpr int kCSItems = 8;                       // keys per thread at most
+constexpr int kCSMax = kCSCtas * kCSThreads * kCSItems;
+
+template <int ITEMS>
+struct ClusterSortSmem {
+    uint64_t key[2][kCSThreads * ITEMS];
+    int val[2][kCSThreads * ITEMS];
+    unsigned cnt[kCSWarps][kDigits];
+    unsigned total[kDigits];  // this CTA's count per digit, read by the cluster
+    unsigned start[kDigits];  // place of this CTA's first key of each digit ...
+    unsigned local[kDigits];  // ... in the cluster, and in the CTA's own order
+    unsigned wsum[2][kDigits / 32];
+};
+
+struct ClusterSortArgs {
+    const uint64_t* keys;  // the keys, or null: order keys of coord + blockIdx.y n
+    const double* coord;
+    int* out[3];           // sorted indices, of axis blockIdx.y
+    int n, first_pass;     // passes first_pass .. 7 (an even number)
+};
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kCSThreads, 1) cluster_sort_kernel(ClusterSortArgs a) {
+    constexpr int kCSTile = kCSThreads * ITEMS;  // keys per CTA
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ClusterSortSmem<ITEMS>& S = *reinterpret_cast<ClusterSortSmem<ITEMS>*>(smem_raw);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int ctas = (int)cl.num_blocks(), me = (int)cl.block_rank();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int k = tid; k < kCSTile; k += kCSThreads) {
+        const int i = me * kCSTile + k;
+        // places past the end hold the largest key; they come last and stay there
+        S.key[0][k] = i >= a.n ? ~0ull : a.keys != nullptr ? a.keys[i] : order_key(a.coord[(size_t)blockIdx.y * a.n + i]);
+        S.val[0][k] = i;
+    }
+    cl.sync();
+    int cur = 0;
+    for (int pass = a.first_pass; pass < 8; ++pass, cur ^= 1) {
+        const int shift = 8 * pass;
+        for (int d = lane; d < kDigits; d += 32) S.cnt[warp][d] = 0;
+        __syncwarp();
+        uint64_t key[ITEMS];
+        int val[ITEMS];
+        unsigned rank[ITEMS], peers[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int k = warp * (32 * ITEMS) + r * 32 + lane;
+            key[r] = S.key[cur][k];
+            val[r] = S.val[cur][k];
+            peers[r] = digit_peers((unsigned)(key[r] >> shift) & 0xFFu);
+        }
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const unsigned dig = (unsigned)(key[r] >> shift) & 0xFFu;
+            const unsigned b = S.cnt[warp][dig];
+            rank[r] = b + __popc(peers[r] & lt);
+            __syncwarp();
+            if (lane == __ffs(peers[r]) - 1) S.cnt[warp][dig] = b + __popc(peers[r]);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (tid < kDigits) {
+            unsigned tot = 0;
+#pragma unroll
+            for (int w = 0; w < kCSWarps; ++w) {
+                const unsigned c = S.cnt[w][tid];
+                S.cnt[w][tid] = tot;
+                tot += c;
+            }
+            S.total[tid] = tot;
+        }
+        cl.sync();
+        if (tid < kDigits) {
+            unsigned below = 0, all = 0;
+            for (int c = 0; c < ctas; ++c) {
+                const unsigned v = cl.map_shared_rank(S.total, c)[tid];
+                below += c < me ? v : 0u;
+                all += v;
+            }
+            // exclusive prefixes over the digits (8 warps), of the cluster's
+            // and of the CTA's counts
+            const unsigned own = S.total[tid];
+            unsigned incl = all, lincl = own;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+                const unsigned u = __shfl_up_sync(0xffffffffu, lincl, o);
+                if (lane >= o) {
+                    incl += v;
+                    lincl += u;
+                }
+            }
+            if (lane == 31) {
+                S.wsum[0][warp] = incl;
+                S.wsum[1][warp] = lincl;
+            }
+            S.start[tid] = incl - all + below;
+            S.local[tid] = lincl - own;
+        }
+        __syncthreads();
+        if (tid < kDigits) {
+            unsigned base = 0, lbase = 0;
+            for (int w = 0; w < warp; ++w) {
+                base += S.wsum[0][w];
+                lbase += S.wsum[1][w];
+            }
+            S.start[tid] += base;
+            S.local[tid] += lbase;
+        }
+        __syncthreads();
+        // the CTA's keys in order first (over the buffer just read), so that
+        // the stores to the cluster are runs
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const unsigned dig = (unsigned)(key[r] >> shift) & 0xFFu;
+            const unsigned k = S.local[dig] + S.cnt[warp][dig] + rank[r];
+            S.key[cur][k] = key[r];
+            S.val[cur][k] = val[r];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const unsigned j = r * kCSThreads + tid;
+            const uint64_t kk = S.key[cur][j];
+            const unsigned dig = (unsigned)(kk >> shift) & 0xFFu;
+            const unsigned at = S.start[dig] + j - S.local[dig];
+            const int c = (int)(at / kCSTile), k = (int)(at % kCSTile);
+            cl.map_shared_rank(&S.key[cur ^ 1][0], c)[k] = kk;
+            cl.map_shared_rank(&S.val[cur ^ 1][0], c)[k] = S.val[cur][j];
+        }
+        cl.sync();
+    }
+    int* out = a.out[blockIdx.y];
+    for (int k = tid; k < kCSTile; k += kCSThreads) {
+        const int i = me * kCSTile + k;
+        if (i < a.n) out[i] = S.val[cur][k];
     }
 }
 
@@ -403,6 +573,100 @@ __global__ void __launch_bounds__(256) part_scatter_kernel(PartArgs a) {
         const int dst = fl[k] ? seg + left_before : seg + half + ((p - seg) - left_before);
         out[dst] = body[k];
     }
+}
+
+// The remaining levels of the median splits, from segments of at most
+// kLocalTile bodies down to one, in one launch: a CTA holds the three lists of
+// its segment in shared memory as 16-bit local ids (places in the first
+// list), flags the left half of every segment of the split axis's list and
+// stably partitions the other two, level by level: 48 us for the last 12
+// levels of 32768 bodies, where two launches a level took 8 us each.
+constexpr int kLocalThreads = 512;
+constexpr int kLocalItems = 8;
+constexpr int kLocalTile = kLocalThreads * kLocalItems;
+
+constexpr int kLocalRows = kLocalTile / 32;
+
+struct LocalSmem {
+    unsigned short id[3][2][kLocalTile];
+    int body[kLocalTile];
+    unsigned char flag[kLocalTile];
+    unsigned bits[2][kLocalRows];  // flags of 32 places
+    unsigned pre[2][kLocalRows];   // flags set before them
+};
+
+__global__ void __launch_bounds__(kLocalThreads)
+kd_local_kernel(const int* __restrict__ l0, const int* __restrict__ l1, const int* __restrict__ l2,
+                int* __restrict__ loc, int* __restrict__ order, int n, int lv) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    LocalSmem& S = *reinterpret_cast<LocalSmem*>(smem_raw);
+    const int seg = min(n, kLocalTile), base = blockIdx.x * seg;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int p = tid; p < seg; p += kLocalThreads) {
+        const int b = l0[base + p];
+        S.body[p] = b;
+        S.id[0][0][p] = (unsigned short)p;
+        loc[b] = p;  // (the segment's bodies only, in all three lists)
+    }
+    __syncthreads();
+    for (int p = tid; p < seg; p += kLocalThreads) {
+        S.id[1][0][p] = (unsigned short)loc[l1[base + p]];
+        S.id[2][0][p] = (unsigned short)loc[l2[base + p]];
+    }
+    __syncthreads();
+    int cur[3] = {0, 0, 0};
+    for (int size = seg; size > 1; size >>= 1, ++lv) {
+        const int d = lv % 3, half = size >> 1;
+        for (int p = tid; p < seg; p += kLocalThreads)
+            S.flag[S.id[d][cur[d]][p]] = (unsigned char)((p & (size - 1)) < half);
+        __syncthreads();
+        const int ax[2] = {(d + 1) % 3, (d + 2) % 3};
+        unsigned short id[2][kLocalItems];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int k = 0; k < kLocalItems; ++k) {
+                const int p = k * kLocalThreads + tid;
+                id[e][k] = p < seg ? S.id[ax[e]][cur[ax[e]]][p] : 0;
+                const unsigned m = __ballot_sync(0xffffffffu, p < seg && S.flag[id[e][k]]);
+                if (lane == 0) S.bits[e][p >> 5] = m;
+            }
+        __syncthreads();
+        if (warp < 2) {  // prefix over the rows, 4 per lane
+            unsigned c[kLocalRows / 32], sum = 0;
+#pragma unroll
+            for (int q = 0; q < kLocalRows / 32; ++q) {
+                c[q] = sum;
+                sum += __popc(S.bits[warp][lane * (kLocalRows / 32) + q]);
+            }
+            unsigned incl = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+#pragma unroll
+            for (int q = 0; q < kLocalRows / 32; ++q)
+                S.pre[warp][lane * (kLocalRows / 32) + q] = incl - sum + c[q];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int k = 0; k < kLocalItems; ++k) {
+                const int p = k * kLocalThreads + tid, s0 = p & ~(size - 1);
+                if (p >= seg) continue;
+                const unsigned m = S.bits[e][p >> 5];
+                const int before = (int)S.pre[e][p >> 5] + __popc(m & ((1u << lane) - 1u));
+                const int first = (int)S.pre[e][s0 >> 5] +
+                                  __popc(S.bits[e][s0 >> 5] & ((1u << (s0 & 31)) - 1u));
+                const int l = before - first;
+                S.id[ax[e]][cur[ax[e]] ^ 1][(m >> lane) & 1u ? s0 + l : s0 + half + (p - s0 - l)] = id[e][k];
+            }
+        cur[ax[0]] ^= 1;
+        cur[ax[1]] ^= 1;
+        __syncthreads();
+    }
+    for (int p = tid; p < seg; p += kLocalThreads) order[base + p] = S.body[S.id[0][cur[0]][p]];
 }
 
 // Leaves: leaf n + p holds body list[p] (nbody/nbody_space_heap.cpp:141-148).
@@ -599,6 +863,37 @@ nbg_status radix_sort(nbg_engine* e, TreeState* t, int n, int first_pass = 0) {
     return NBG_OK;
 }
 
+// cluster_sort_kernel for n <= kCSMax keys; axes: 3 for the coordinate lists
+template <int ITEMS>
+nbg_status cluster_sort_launch(nbg_engine* e, const ClusterSortArgs& a, int axes) {
+    const size_t smem = sizeof(ClusterSortSmem<ITEMS>);
+    NBG_CUDA(e, cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kCSCtas;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kCSCtas, (unsigned)axes);
+    cfg.blockDim = dim3(kCSThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = e->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    NBG_CUDA(e, cudaLaunchKernelEx(&cfg, cluster_sort_kernel<ITEMS>, a));
+    NBG_LAUNCHED(e, "cluster_sort_kernel");
+    return NBG_OK;
+}
+
+nbg_status cluster_sort(nbg_engine* e, const ClusterSortArgs& a, int axes) {
+    const int per = (a.n + kCSCtas * kCSThreads - 1) / (kCSCtas * kCSThreads);
+    if (per <= 1) return cluster_sort_launch<1>(e, a, axes);
+    if (per <= 2) return cluster_sort_launch<2>(e, a, axes);
+    if (per <= 4) return cluster_sort_launch<4>(e, a, axes);
+    return cluster_sort_launch<kCSItems>(e, a, axes);
+}
+
 // Levels [lv_lo, lv_hi) of the heap, bottom-up, in one launch: block b owns
 // the subtree under node 2^lv_lo + b down to level lv_hi - 1 (at most
 // kFusedLevels levels, 256 nodes at its bottom), with a block barrier
@@ -693,7 +988,11 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         NBG_LAUNCHED(e, "morton_keys_kernel");
         // the key bits from 16 up (47 of 63: the curve down to cells of
         // about 2^-16 of the box per axis), bodies sharing one in index order
-        nbg_status s = radix_sort(e, t, n, 2);
+        nbg_status s;
+        if (n <= kCSMax)
+            s = cluster_sort(e, ClusterSortArgs{t->keys[0], nullptr, {t->vals[0], nullptr, nullptr}, n, 2}, 1);
+        else
+            s = radix_sort(e, t, n, 2);
         if (s != NBG_OK) return s;
         if (t->f32)
             leaf_init_kernel<true><<<g, 256, 0, e->stream>>>(t->vals[0], y, e->d_mass, n, *t);
@@ -708,7 +1007,12 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
     }
     t->curve = 0;
     // 1. three sorted lists
-    for (int d = 0; d < 3; ++d) {
+    if (n <= kCSMax) {
+        nbg_status s = cluster_sort(
+            e, ClusterSortArgs{nullptr, y, {t->lists[0], t->lists[1], t->lists[2]}, n, 0}, 3);
+        if (s != NBG_OK) return s;
+    }
+    for (int d = 0; d < 3 && n > kCSMax; ++d) {
         init_keys_kernel<<<g, 256, 0, e->stream>>>(y + (size_t)d * n, n, t->keys[0], t->vals[0]);
         NBG_LAUNCHED(e, "init_keys_kernel");
         nbg_status s = radix_sort(e, t, n);
@@ -718,7 +1022,8 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
     }
     // 2. median splits, level by level
     const int ntiles = (n + kPartTile - 1) / kPartTile;
-    for (int lv = 0; lv < t->levels; ++lv) {
+    int lv = 0;
+    for (; (n >> lv) > kLocalTile; ++lv) {
         const int S = n >> lv;
         const int d = lv % 3;
         split_flag_kernel<<<g, 256, 0, e->stream>>>(t->lists[d], n, S, t->flag);
@@ -734,10 +1039,8 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         a.ntiles = ntiles;
         a.n = n;
         a.S = S;
-        if (S > kPartTile) {
-            part_count_kernel<<<dim3(ntiles, 2), 256, 0, e->stream>>>(a);
-            NBG_LAUNCHED(e, "part_count_kernel");
-        }
+        part_count_kernel<<<dim3(ntiles, 2), 256, 0, e->stream>>>(a);
+        NBG_LAUNCHED(e, "part_count_kernel");
         part_scatter_kernel<<<dim3(ntiles, 2), 256, 0, e->stream>>>(a);
         NBG_LAUNCHED(e, "part_scatter_kernel");
         int* tmp0 = t->lists[e0];
@@ -747,11 +1050,16 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         t->spare[0] = tmp0;
         t->spare[1] = tmp1;
     }
+    NBG_CUDA(e, cudaFuncSetAttribute(kd_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(LocalSmem)));
+    kd_local_kernel<<<std::max(1, n / kLocalTile), kLocalThreads, sizeof(LocalSmem), e->stream>>>(
+        t->lists[0], t->lists[1], t->lists[2], t->spare[0], t->spare[1], n, lv);
+    NBG_LAUNCHED(e, "kd_local_kernel");
     // 3. leaves, then the bottom-up update
     if (t->f32)
-        leaf_init_kernel<true><<<g, 256, 0, e->stream>>>(t->lists[0], y, e->d_mass, n, *t);
+        leaf_init_kernel<true><<<g, 256, 0, e->stream>>>(t->spare[1], y, e->d_mass, n, *t);
     else
-        leaf_init_kernel<false><<<g, 256, 0, e->stream>>>(t->lists[0], y, e->d_mass, n, *t);
+        leaf_init_kernel<false><<<g, 256, 0, e->stream>>>(t->spare[1], y, e->d_mass, n, *t);
     NBG_LAUNCHED(e, "leaf_init_kernel");
     nbg_status s = update_levels(e, t);
     if (s != NBG_OK) return s;
