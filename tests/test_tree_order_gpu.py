@@ -38,10 +38,12 @@ def test_curve(make_engine, n, ties):
 @pytest.mark.parametrize("ties", [False, True])
 @pytest.mark.parametrize("n", SIZES)
 def test_median(make_engine, n, ties):
-    """Every segment's left half: its smallest bodies along the level's axis,
-    ties by body index."""
+    """Every segment's left half: its smallest bodies along the level's axis in
+    the order of the FP64 keys (-0 before +0), ties by body index."""
     v = _positions(n, ties)
-    rank = [np.argsort(np.argsort(v[:, c], kind="stable")) for c in range(3)]
+    bits = np.ascontiguousarray(v.T).view(np.uint64)
+    keys = np.where(bits >> np.uint64(63), ~bits, bits | np.uint64(1 << 63))
+    rank = [np.argsort(np.argsort(keys[c], kind="stable")) for c in range(3)]
     order, level = np.arange(n), 0
     while (n >> level) > 1:
         seg = order.reshape(1 << level, -1)
