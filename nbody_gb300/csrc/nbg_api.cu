@@ -238,6 +238,7 @@ void nbg_engine_destroy(nbg_engine* e) {
     cudaFree(e->d_mass);
     cudaFree(e->d_massf);
     cudaFree(e->d_xyzm);
+    for (void* p : e->xyzm_retired) cudaFree(p);
     cudaFree(e->d_scalar);
     cudaFree(e->d_err);
     if (e->h_scalar) cudaFreeHost(e->h_scalar);

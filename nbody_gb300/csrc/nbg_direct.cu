@@ -775,13 +775,8 @@ nbg_status direct_sym_launch(nbg_engine* e, const double* y, double* f) {
     const int n_ranges = (n + range - 1) / range;
     const int n_pad = n_ranges * range;
     const size_t need = 2 * (size_t)n_pad * sizeof(float4);
-    if (e->xyzm_cap < need) {
-        cudaFree(e->d_xyzm);
-        e->d_xyzm = nullptr;
-        e->xyzm_cap = 0;
-        NBG_CUDA(e, cudaMalloc(&e->d_xyzm, need));
-        e->xyzm_cap = need;
-    }
+    if (!reserve_scratch(e, need))
+        return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
     float4* bodies = reinterpret_cast<float4*>(e->d_xyzm);
     pack_sym_kernel<<<grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
         y, e->d_mass, bodies, f, n, n_pad);
@@ -895,13 +890,8 @@ nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
     const int n_jt = (n + kT - 1) / kT;
     const int n_pad = n_jt * kT;
     const size_t need = (size_t)n_pad * sizeof(Body2);
-    if (e->xyzm_cap < need) {
-        cudaFree(e->d_xyzm);
-        e->d_xyzm = nullptr;
-        e->xyzm_cap = 0;
-        NBG_CUDA(e, cudaMalloc(&e->d_xyzm, need));
-        e->xyzm_cap = need;
-    }
+    if (!reserve_scratch(e, need))
+        return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
     Body2* bodies = reinterpret_cast<Body2*>(e->d_xyzm);
     pack_mixed_kernel<<<grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
         y, e->d_mass, bodies, f, n, n_pad);

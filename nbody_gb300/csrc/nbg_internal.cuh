@@ -57,6 +57,8 @@ struct nbg_engine {
     // scratch of one call (packed bodies, partial sums), kept and grown
     float4* d_xyzm = nullptr;
     size_t xyzm_cap = 0;
+    bool xyzm_captured = false;       // a captured launch reads d_xyzm
+    std::vector<void*> xyzm_retired;  // outgrown blocks that captured launches read
 
     // reductions
     unsigned long long* d_scalar = nullptr;  // fmaxabs bits
@@ -105,15 +107,23 @@ nbg_status cuda_error(nbg_engine* e, cudaError_t err, const char* what);
     } while (0)
 
 // At least `bytes` of e->d_xyzm: false (and the old block kept, or none) when
-// they cannot be had, which includes a growth while the stream is captured.
+// they cannot be had, which includes a growth while the stream is captured.  A
+// block that a captured launch reads lives as long as the engine, since the
+// caller may replay the graph after another call has outgrown the block.
 inline bool reserve_scratch(nbg_engine* e, size_t bytes) {
-    if (e->xyzm_cap >= bytes) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-        return false;
-    cudaFree(e->d_xyzm);
+    const bool capturing = cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess ||
+                           cap != cudaStreamCaptureStatusNone;
+    if (e->xyzm_cap >= bytes) {
+        e->xyzm_captured = e->xyzm_captured || capturing;
+        return true;
+    }
+    if (capturing) return false;
+    if (e->xyzm_captured) e->xyzm_retired.push_back(e->d_xyzm);
+    else cudaFree(e->d_xyzm);
     e->d_xyzm = nullptr;
     e->xyzm_cap = 0;
+    e->xyzm_captured = false;
     if (cudaMalloc(&e->d_xyzm, bytes) != cudaSuccess) {
         cudaGetLastError();
         return false;
