@@ -302,6 +302,9 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  *       stackless walk) for the mixed-precision Barnes-Hut path,
  *       "bh.group" (64 (default), 32 or 128 bodies per warp in the group
  *       walk; 128 with monopole cells only),
+ *       "bh.parts" (warps that share a group of the default group walk: 0,
+ *       the default, chooses by the number of groups; 1, 2, 4, 8, 16 or 32,
+ *       other values are rounded down to one of these),
  *       "bh.walk_npl" (node tests per lane and traversal step of the
  *       group walk: 2, the default with monopole cells, or 1, the default
  *       with quadrupole cells),

@@ -533,8 +533,6 @@ struct GroupSmem {  // followed by the stacks, kGWWarps x stack_cap ints
     float lm[kGWWarps][kGWList];
 };
 
-// groups whose node tests set the group walk's test cap (one warp each, one block)
-constexpr int kCapSamples = 32;
 
 // Second list of the quadrupole walk (bh.order = 2): accepted cells with their
 // second moments; leaves stay in the monopole list.  Arrays in the order
@@ -633,6 +631,35 @@ __device__ __forceinline__ void group_pair_lo(f2_t xj, f2_t yj, f2_t zj, f2_t mj
     az = f2_fma(dz, s3, az);
 }
 
+// The cap of a walk whose sampled groups have (so far) the node tests in
+// ctl.finished: ratio x their median, the value of rank samples / 2 over all
+// samples; with some of them unknown an upper bound of it, ~0 while half are.
+// All lanes of a warp call it and get it.
+__device__ __forceinline__ unsigned long long walk_cap(const TreeState& t) {
+    const WalkCtl* ctl = reinterpret_cast<const WalkCtl*>(t.fb_count);
+    const int lane = threadIdx.x & 31;
+    const unsigned f = lane < t.cap_samples ? *(volatile const unsigned*)&ctl->finished[lane] : 0u;
+    const unsigned v = f - 1u;  // unknown: the largest value
+    int rank = 0;
+    for (int j = 0; j < 32; ++j) {
+        const unsigned o = __shfl_sync(0xffffffffu, v, j);
+        rank += o < v || (o == v && j < lane) ? 1 : 0;
+    }
+    const unsigned at = __ballot_sync(0xffffffffu, rank == t.cap_samples / 2);
+    const unsigned m = __shfl_sync(0xffffffffu, v, __ffs(at) - 1);
+    return m == ~0u ? ~0ull : max((unsigned long long)t.cap_ratio * m, 4096ull);
+}
+
+// a group's counts: 64 bits, 32 where a group's fit (nodes of one tree)
+template <bool SMALL>
+struct CountOf {
+    using T = unsigned long long;
+};
+template <>
+struct CountOf<true> {
+    using T = unsigned;
+};
+
 // BPL bodies per lane: a group of 32 BPL consecutive leaves per warp (lane l
 // holds leaves l, l + 32, ...); every list entry is evaluated for all of them.
 // SMACC: the per-body two-sum accumulators (6 BPL packed values per lane)
@@ -641,12 +668,14 @@ __device__ __forceinline__ void group_pair_lo(f2_t xj, f2_t yj, f2_t zj, f2_t mj
 // EMIT: cells accepted with the group box's nearest point inside the tight
 // ratio (the learned correction's band) are recorded in t.cand; a group
 // with more than t.cand_cap of them is handed to the per-body walk.
+// SPLIT: this warp is one of t.parts of its group (bh_split_walk_kernel).
 template <bool CLAMP, int BPL, int ORDER, int EUNR, bool SMACC, bool FROZEN = false,
-          bool EMIT = false, int NPL = 1>
+          bool EMIT = false, int NPL = 1, bool SPLIT = false>
 __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, double* __restrict__ f,
                                                int n, float eps2v, const TreeState& t,
                                                int stack_cap, unsigned* err,
-                                               unsigned char* smem_raw, const int gw) {
+                                               unsigned char* smem_raw, const int gw,
+                                               const int part = 0) {
     GroupSmem& S = *reinterpret_cast<GroupSmem*>(smem_raw);
     QuadLists& Q = *reinterpret_cast<QuadLists*>(smem_raw + sizeof(GroupSmem));
     int* stacks = reinterpret_cast<int*>(smem_raw + sizeof(GroupSmem) +
@@ -726,12 +755,15 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         for (int q = 0; q < 6; ++q) slot(6 * b + q) = zero;
     }
     const unsigned lt = (1u << lane) - 1u;
-    unsigned long long tests = 0, inter = 0;
+    using Count = typename CountOf<SPLIT>::T;
+    Count tests = 0, inter = 0;
     if (lane == 0) stack[0] = 0;
     __syncwarp();
     int sp = 1, lc = 0, peak = 1, ec = 0;
     bool overflow = false, abandoned = false;
     const unsigned long long test_cap = t.test_cap != 0 ? t.test_cap : t.cap_state[0];
+    WalkCtl* ctl = reinterpret_cast<WalkCtl*>(t.fb_count);
+    unsigned sent = 0;  // SPLIT: tests already added to the group's
 
     auto evaluate = [&]() {
         // pad to a whole quad with massless entries
@@ -800,7 +832,7 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
             f2_two_sum(slot(6 * b + 2), slot(6 * b + 3), f2_add(ay[b], by[b]));
             f2_two_sum(slot(6 * b + 4), slot(6 * b + 5), f2_add(az[b], bz[b]));
         }
-        inter += (unsigned long long)lc;
+        inter += (Count)lc;
         lc = 0;
         __syncwarp();
     };
@@ -840,7 +872,7 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
             f2_two_sum(slot(6 * b + 2), slot(6 * b + 3), ay[b]);
             f2_two_sum(slot(6 * b + 4), slot(6 * b + 5), az[b]);
         }
-        inter += (unsigned long long)qc;
+        inter += (Count)qc;
         qc = 0;
         __syncwarp();
     };
@@ -857,6 +889,17 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         }
         __syncwarp();
         sp -= k;
+        bool mine[NPL];  // summed by this warp
+#pragma unroll
+        for (int w = 0; w < NPL; ++w) {
+            mine[w] = true;
+            if constexpr (SPLIT) {
+                const int lv = 31 - __clz(c[w]);
+                const bool own = (c[w] & (t.parts - 1)) == part;
+                if (lv == t.top && !own) c[w] = 0;
+                mine[w] = lv > t.top || own;
+            }
+        }
         // issued before a full list is evaluated, which covers their latency;
         // lanes past the popped entries read record 0 (unused, zeroed), and
         // leaves' second moments are zero
@@ -872,8 +915,24 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
                 nq1[w] = __ldg(&t.quad[2 * c[w] + 1]);
             }
         }
-        if (lc > kGWList - 32 * NPL) evaluate();  // room for this step's entries
-        if (ORDER == 2 && qc > kGWQList - 32 * NPL) evaluate_quad();
+        const bool full = lc > kGWList - 32 * NPL, qfull = ORDER == 2 && qc > kGWQList - 32 * NPL;
+        // SPLIT: at each evaluation (which hides the atomic) the group's node
+        // tests so far, over all its parts, are compared with the cap
+        unsigned seen = 0;
+        if (SPLIT && (full || qfull)) {
+            if (lane == 0) seen = atomicAdd(&ctl->group[gw], (unsigned)tests - sent);
+            __syncwarp();  // else lane 0 evaluates the list by itself: 505 -> 832 us at 2^18 bodies
+        }
+        if (full) evaluate();  // room for this step's entries
+        if (qfull) evaluate_quad();
+        if (SPLIT && (full || qfull)) {
+            seen = __shfl_sync(0xffffffffu, seen, 0) + (unsigned)tests - sent;
+            sent = (unsigned)tests;
+            if ((unsigned long long)seen + 1 > test_cap) {
+                abandoned = true;
+                break;
+            }
+        }
         bool accept[NPL], open[NPL], band[NPL];
 #pragma unroll
         for (int w = 0; w < NPL; ++w) {
@@ -894,10 +953,19 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         }
         // every popped entry stands for two tested children, except the root's
         // stand-in entry 0 at the first step (its child 0 is not a node)
-        tests += (unsigned long long)(2 * k);
-        if (tests > test_cap) {  // a group spread over much of the system:
-            abandoned = true;      // its bodies are walked one by one instead
-            break;
+        if constexpr (SPLIT) {
+#pragma unroll
+            for (int w = 0; w < NPL; ++w) {
+                tests += (Count)__popc(__ballot_sync(0xffffffffu, c[w] != 0 && mine[w]));
+                accept[w] = accept[w] && mine[w];
+                band[w] = band[w] && mine[w];
+            }
+        } else {
+            tests += (unsigned long long)(2 * k);
+            if (tests > test_cap) {  // a group spread over much of the system:
+                abandoned = true;      // its bodies are walked one by one instead
+                break;
+            }
         }
         if constexpr (EMIT) {
             unsigned bm[NPL];
@@ -909,11 +977,14 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
             }
             if (ec + nb > t.cand_cap) {  // walked body by body instead
                 abandoned = true;
+                if (SPLIT && lane == 0) t.cand_part_n[gw * t.parts + part] = (unsigned)t.cand_cap + 1u;
                 break;
             }
+            int* cells = SPLIT ? t.cand_part + ((size_t)gw * t.parts + part) * t.cand_cap
+                               : t.cand + (size_t)gw * t.cand_cap;
 #pragma unroll
             for (int w = 0; w < NPL; ++w) {
-                if (band[w]) t.cand[(size_t)gw * t.cand_cap + ec + __popc(bm[w] & lt)] = c[w];
+                if (band[w]) cells[ec + __popc(bm[w] & lt)] = c[w];
                 ec += __popc(bm[w]);
             }
         }
@@ -984,16 +1055,15 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
     if (overflow) {
         if (lane == 0) atomicOr(err, kDevErrWalkOverflow);
     }
-    tests -= 1;  // child 0 of the first step
+    if (!SPLIT) tests -= 1;  // child 0 of the first step
     if (lane == 0) {
-        atomicAdd(&t.counters[0], tests);
+        if (SPLIT) atomicAdd(&ctl->group[gw], (unsigned)tests - sent);
+        else atomicAdd(&t.counters[0], (unsigned long long)tests);
         atomicMax(&t.counters[2], (unsigned long long)peak);
-    }
-    if constexpr (EMIT) {
-        if (lane == 0) t.cand_n[gw] = abandoned ? 0u : (unsigned)ec;
+        if (EMIT && !SPLIT) t.cand_n[gw] = abandoned ? 0u : (unsigned)ec;
     }
     if (abandoned) {
-        if (lane == 0) {
+        if (!SPLIT && lane == 0) {
             t.fb_list[atomicAdd(t.fb_count, 1u)] = gw;
             atomicAdd(&t.counters[3], 1ull);
         }
@@ -1001,6 +1071,23 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
     }
     if (lc > 0) evaluate();
     if (ORDER == 2 && qc > 0) evaluate_quad();
+    if constexpr (SPLIT) {
+        if (lane == 0) {
+            atomicAdd(&ctl->group[n / (32 * BPL) + gw], (unsigned)inter);
+            if (EMIT) t.cand_part_n[gw * t.parts + part] = (unsigned)ec;
+        }
+        double* out = t.part + (size_t)part * 3 * n + gw * 32 * BPL + lane;
+#pragma unroll
+        for (int bb = 0; bb < BPL; ++bb)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                float h0, h1, l0, l1;
+                f2_unpack(slot(6 * bb + 2 * k), h0, h1);
+                f2_unpack(slot(6 * bb + 2 * k + 1), l0, l1);
+                out[(size_t)k * n + bb * 32] = ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
+            }
+        return;
+    }
 #pragma unroll
     for (int bb = 0; bb < BPL; ++bb) {
         float h0, h1, l0, l1;
@@ -1018,7 +1105,7 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         f2_unpack(slot(6 * bb + 5), l0, l1);
         f[5 * n + b] = ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
     }
-    if (lane == 0) atomicAdd(&t.counters[1], inter * 32ull * BPL);
+    if (!SPLIT && lane == 0) atomicAdd(&t.counters[1], inter * 32ull * BPL);
 }
 
 // Persistent over the groups (n is a power of two >= 32 BPL, so groups are
@@ -1045,34 +1132,105 @@ bh_group_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n
     }
 }
 
+// The default group walk with t.parts warps per group, which share the tree:
+// nodes above level t.top are tested by every part and summed by one, the
+// subtrees under that level are dealt out (node mod parts).  A system of few
+// groups then fills the GPU: 16384 bodies are 256 groups, and one warp each
+// took 152 us (59 us with 16, and 5 us in bh_walk_finish_kernel).  A part stops once its group's tests exceed the cap;
+// whether the group goes to the per-body walk is decided by
+// bh_walk_finish_kernel from the totals alone, and the parts are added in
+// order, so equal trees give equal forces.
+template <bool CLAMP, int MINB, int ORDER, bool SMACC, int NPL, bool EMIT = false>
+__global__ void __launch_bounds__(kGWThreads, MINB)
+bh_split_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2v,
+                     TreeState t, int stack_cap, unsigned* err) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    const int tasks = n / 64 * t.parts;
+    int task = blockIdx.x * kGWWarps + (threadIdx.x >> 5);
+    while (task < tasks) {
+        group_walk_one<CLAMP, 2, ORDER, 2, SMACC, false, EMIT, NPL, true>(
+            y, f, n, eps2v, t, stack_cap, err, smem_raw, task / t.parts, task % t.parts);
+        int next = 0;
+        if (lane == 0) next = (int)atomicAdd(&t.fb_count[1], 1u);
+        task = gridDim.x * kGWWarps + __shfl_sync(0xffffffffu, next, 0);
+    }
+}
+
+// A CTA per group of the shared walk: whether the group goes to the per-body
+// walk, else the sum of its parts in order, and with EMIT its parts' lists of
+// band cells one after the other.
+template <bool EMIT>
+__global__ void __launch_bounds__(192)
+bh_walk_finish_kernel(const double* __restrict__ y, double* __restrict__ f, int n, TreeState t) {
+    const WalkCtl* ctl = reinterpret_cast<const WalkCtl*>(t.fb_count);
+    const int gw = blockIdx.x, tid = threadIdx.x;
+    const unsigned long long cap = t.test_cap != 0 ? t.test_cap : t.cap_state[0];
+    const unsigned long long tests = ctl->group[gw];
+    unsigned cells = 0;
+    if (EMIT)
+        for (int q = 0; q < t.parts; ++q)
+            cells = min(cells + t.cand_part_n[gw * t.parts + q], (unsigned)t.cand_cap + 1u);
+    const bool hand = tests + 1 > cap || (EMIT && cells > (unsigned)t.cand_cap);
+    if (tid == 0) {
+        if (hand) t.fb_list[atomicAdd(t.fb_count, 1u)] = gw;
+        if (EMIT) t.cand_n[gw] = hand ? 0u : cells;
+        atomicAdd(&t.counters[0], min(tests, cap));
+        atomicAdd(&t.counters[hand ? 3 : 1], hand ? 1ull : 64ull * ctl->group[gridDim.x + gw]);
+    }
+    if (hand) return;
+    const int k = tid / 64;
+    const size_t p = (size_t)gw * 64 + (tid & 63);
+    double s = 0.0;
+#pragma unroll 16
+    for (int q = 0; q < t.parts; ++q) s += __ldg(t.part + ((size_t)q * 3 + k) * n + p);
+    const int b = t.body_n[n + p];
+    f[(size_t)k * n + b] = y[(size_t)(3 + k) * n + b];
+    f[(size_t)(3 + k) * n + b] = s;
+    unsigned at = 0;
+    for (int q = 0; EMIT && q < t.parts; ++q) {
+        const unsigned c = t.cand_part_n[gw * t.parts + q];
+        const int* from = t.cand_part + ((size_t)gw * t.parts + q) * t.cand_cap;
+        for (unsigned j = tid; j < c; j += 192) t.cand[(size_t)gw * t.cand_cap + at + j] = from[j];
+        at += c;
+    }
+}
+
 // The group walk's test cap: ratio x the median node tests of kCapSamples
 // groups spread over the leaves (every stride-th), a function of the tree
-// alone, so that equal trees give equal forces.  One block, one warp per
-// sample, each running the group walk's traversal without its force
-// evaluation.  The samples walk in rounds of doubling test limits (4096,
-// 8192, ...) and stop once more than half have finished: the median is then
-// known without walking the samples above it, which are the slow ones.
+// alone, so that equal trees give equal forces.  A CTA per sample runs the
+// group walk's traversal without its force evaluation, its warps sharing the
+// tree as in bh_split_walk_kernel.  Samples that exceed the upper bound of
+// the cap which the finished ones give (known once more than half are) are
+// above the median and stop.  It is bound by the longest chain of dependent
+// node loads; all samples as the warps of one CTA took 43 us at 16384 bodies
+// and 95 us at 2^20 (18 and 65 us).
+constexpr int kCapWarps = 16;
+constexpr int kCapTop = 6;
+
 template <int BPL>
-__global__ void __launch_bounds__(kCapSamples * 32, 1)
-bh_test_cap_kernel(int n, int stride, int samples, TreeState t, int stack_cap, unsigned ratio) {
+__global__ void __launch_bounds__(kCapWarps * 32, 1)
+bh_test_cap_kernel(int n, TreeState t, int stack_cap) {
     extern __shared__ int cap_stacks[];
-    __shared__ unsigned long long counts[kCapSamples];
-    __shared__ int finished[kCapSamples];
+    __shared__ unsigned total;
+    __shared__ int stopped;
+    WalkCtl* ctl = reinterpret_cast<WalkCtl*>(t.fb_count);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool active = warp < samples;
-    const int gw = warp * stride;
+    const int gw = blockIdx.x * t.cap_stride;
+    if (threadIdx.x == 0) {
+        total = 0;
+        stopped = 0;
+    }
     float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    if (active) {
 #pragma unroll
-        for (int b = 0; b < BPL; ++b) {
-            const float4 me = __ldg(&t.node4[n + gw * 32 * BPL + b * 32 + lane]);
-            lo[0] = fminf(lo[0], me.x);
-            lo[1] = fminf(lo[1], me.y);
-            lo[2] = fminf(lo[2], me.z);
-            hi[0] = fmaxf(hi[0], me.x);
-            hi[1] = fmaxf(hi[1], me.y);
-            hi[2] = fmaxf(hi[2], me.z);
-        }
+    for (int b = 0; b < BPL; ++b) {
+        const float4 me = __ldg(&t.node4[n + gw * 32 * BPL + b * 32 + lane]);
+        lo[0] = fminf(lo[0], me.x);
+        lo[1] = fminf(lo[1], me.y);
+        lo[2] = fminf(lo[2], me.z);
+        hi[0] = fmaxf(hi[0], me.x);
+        hi[1] = fmaxf(hi[1], me.y);
+        hi[2] = fmaxf(hi[2], me.z);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -1090,68 +1248,67 @@ bh_test_cap_kernel(int n, int stride, int samples, TreeState t, int stack_cap, u
     int* stack = cap_stacks + warp * stack_cap;
     const unsigned lt = (1u << lane) - 1u;
     if (lane == 0) stack[0] = 0;
+    __syncthreads();
+    int sp = 1;
+    while (sp > 0) {
+        const unsigned long long bound = ~*(volatile unsigned long long*)&ctl->bound;
+        // two node tests per lane and step (32 entries popped)
+        const int k = min(sp, 32);
+        int c[2];
+        bool open[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const int slot = lane + 32 * w;
+            c[w] = slot < 2 * k ? 2 * stack[sp - 1 - (slot >> 1)] + (slot & 1) : 0;
+        }
+        __syncwarp();
+        sp -= k;
+        unsigned counted = 0;
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const int lv = 31 - __clz(c[w]);
+            const bool own = (c[w] & (kCapWarps - 1)) == warp;
+            if (lv == kCapTop && !own) c[w] = 0;
+            open[w] = false;
+            if (c[w] != 0 && c[w] < n) {
+                const float4 nd = __ldg(&t.node4[c[w]]);
+                const float ex = fmaxf(fabsf(nd.x - cb[0]) - hb[0], 0.f);
+                const float ey = fmaxf(fabsf(nd.y - cb[1]) - hb[1], 0.f);
+                const float ez = fmaxf(fabsf(nd.z - cb[2]) - hb[2], 0.f);
+                open[w] = !(fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > nd.w);
+            }
+            counted += __popc(__ballot_sync(0xffffffffu, c[w] != 0 && (lv > kCapTop || own)));
+        }
+        unsigned sum = 0;
+        if (lane == 0) sum = atomicAdd(&total, counted) + counted;
+        sum = __shfl_sync(0xffffffffu, sum, 0);
+        if ((unsigned long long)sum > bound) {
+            stopped = 1;
+            break;
+        }
+        const unsigned om0 = __ballot_sync(0xffffffffu, open[0]);
+        const unsigned om1 = __ballot_sync(0xffffffffu, open[1]);
+        const int npush = __popc(om0) + __popc(om1);
+        if (sp + npush > stack_cap) break;  // the walk itself reports the overflow
+        if (open[0]) stack[sp + __popc(om0 & lt)] = c[0];
+        if (open[1]) stack[sp + __popc(om0) + __popc(om1 & lt)] = c[1];
+        sp += npush;
+        __syncwarp();
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    if (lane == 0 && !stopped) atomicExch(&ctl->finished[blockIdx.x], total + 1u);
+    __threadfence();
     __syncwarp();
-    int sp = active ? 1 : 0;
-    unsigned long long tests = 0, limit = 4096;
-    for (int round = 0; round < 40; ++round, limit *= 2) {
-        // two node tests per lane and step (32 entries popped): the same
-        // tests as the walk in another order, with two loads in flight
-        while (sp > 0 && tests <= limit) {
-            const int k = min(sp, 32);
-            int c[2];
-            bool open[2];
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const int slot = lane + 32 * w;
-                c[w] = slot < 2 * k ? 2 * stack[sp - 1 - (slot >> 1)] + (slot & 1) : 0;
-            }
-            __syncwarp();
-            sp -= k;
-            int nvalid = 0;
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                open[w] = false;
-                if (c[w] != 0 && c[w] < n) {
-                    const float4 nd = __ldg(&t.node4[c[w]]);
-                    const float ex = fmaxf(fabsf(nd.x - cb[0]) - hb[0], 0.f);
-                    const float ey = fmaxf(fabsf(nd.y - cb[1]) - hb[1], 0.f);
-                    const float ez = fmaxf(fabsf(nd.z - cb[2]) - hb[2], 0.f);
-                    open[w] = !(fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > nd.w);
-                }
-                nvalid += __popc(__ballot_sync(0xffffffffu, c[w] != 0));
-            }
-            tests += (unsigned long long)nvalid;
-            const unsigned om0 = __ballot_sync(0xffffffffu, open[0]);
-            const unsigned om1 = __ballot_sync(0xffffffffu, open[1]);
-            const int npush = __popc(om0) + __popc(om1);
-            if (sp + npush > stack_cap) {  // the walk itself reports the overflow
-                sp = 0;
-                break;
-            }
-            if (open[0]) stack[sp + __popc(om0 & lt)] = c[0];
-            if (open[1]) stack[sp + __popc(om0) + __popc(om1 & lt)] = c[1];
-            sp += npush;
-            __syncwarp();
-        }
-        if (lane == 0 && active) {
-            counts[warp] = tests;
-            finished[warp] = sp == 0;
-        }
-        __syncthreads();
-        int fin = 0;
-        for (int j = 0; j < samples; ++j) fin += finished[j];
-        if (2 * fin > samples) break;  // the same decision in every thread
-        __syncthreads();
-    }
-    // finished samples hold their counts, the others a count above the last
-    // limit: the value of rank samples / 2 is the median
-    if (threadIdx.x < samples) {
-        const unsigned long long v = counts[threadIdx.x];
-        int rank = 0;
-        for (int j = 0; j < samples; ++j)
-            rank += (counts[j] < v || (counts[j] == v && j < (int)threadIdx.x)) ? 1 : 0;
-        if (rank == samples / 2) t.cap_state[0] = max((unsigned long long)ratio * v, 4096ull);
-    }
+    unsigned long long u = walk_cap(t);
+    if (lane == 0 && u != ~0ull) atomicMax(&ctl->bound, ~u);
+    unsigned d = 0;
+    __threadfence();
+    if (lane == 0) d = atomicAdd(&ctl->done, 1u);
+    if (__shfl_sync(0xffffffffu, d, 0) != gridDim.x - 1) return;
+    __threadfence();
+    u = walk_cap(t);  // every sample is in: the cap
+    if (lane == 0) t.cap_state[0] = u;
 }
 
 // The bodies of the groups the group walk gave up on, one warp per body: the
@@ -1446,6 +1603,43 @@ nbg_status mixed_walk(nbg_engine* e, const double* y, double* f, bool emit) {
 }
 
 namespace {
+using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, unsigned*);
+
+// Warps per group of the default walk, and the state of such a walk with its
+// scratch (the parts' sums and, with emit, their band cells): a.parts is 1
+// where the groups fill half of the resident warps (20 per SM) or there is no
+// scratch.  A whole Euler step, one part against the number chosen here: 1024
+// bodies 128 / 98 us (16 parts), 16384 bodies 266 / 180 us (16), 2^16 bodies
+// 436 / 373 us (4; 385 with 8), and where one is kept, 2^17 bodies 528 / 532 us
+// (2), 2^17 with quadrupoles at ratio 1.3 468 / 524 us, 2^18 722 / 752 us: what
+// the parts save there their finish kernel and the doubled top of the tree cost.
+TreeState split_state(nbg_engine* e, bool emit) {
+    TreeState a = *e->tree;
+    const size_t n = e->count, groups = n / 64;
+    const size_t slots = 20 * (size_t)e->sm_count;
+    const int64_t asked = std::min<int64_t>(e->tune_get("bh.parts", 0), 32);
+    a.parts = 1;
+    if (asked > 0)
+        while (2 * a.parts <= asked) a.parts *= 2;
+    else if (2 * groups <= slots)
+        while (a.parts < 16 && a.parts * groups < slots) a.parts *= 2;
+    if (a.parts == 1) return a;
+    const size_t sums = (size_t)a.parts * 3 * n * sizeof(double);
+    const size_t counts = groups * a.parts * sizeof(unsigned);
+    const size_t cells = emit ? counts * a.cand_cap : 0;
+    if (!reserve_scratch(e, sums + cells + counts)) {
+        a.parts = 1;
+        return a;
+    }
+    char* at = reinterpret_cast<char*>(e->d_xyzm);
+    a.part = reinterpret_cast<double*>(at);
+    a.cand_part = reinterpret_cast<int*>(at + sums);
+    a.cand_part_n = reinterpret_cast<unsigned*>(at + sums + cells);
+    a.top = 0;
+    while ((1 << a.top) < 8 * a.parts) ++a.top;
+    return a;
+}
+
 nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit) {
     const int n = (int)e->count;
     TreeState* t = e->tree;
@@ -1477,7 +1671,6 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
         // (164 registers, no spill; at 4 CTAs it spills and is 5 % slower)
         const int64_t wb = e->tune_get("bh.walk_blocks",
                                        bpl == 2 ? (order == 2 ? 3 : acc_smem ? 5 : 4) : 6);
-        using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, unsigned*);
         WalkKernel kern;
         // frozen acceptance runs its own build of the default walk (64-body
         // groups, monopole cells, shared-memory accumulators, residual
@@ -1554,9 +1747,33 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
         else
             kern = clamp ? NBG_GW(true, 1) : NBG_GW(false, 1);
 #undef NBG_GW
+        const int warps = n / (32 * bpl);
+        // the default builds of the walk also run with several warps per group
+        // ("bh.parts": 0, the default, chooses; 1, 2, 4 ... 32)
+        const int64_t npl = e->tune_get("bh.walk_npl", order == 2 ? 1 : 2);
+        const bool default_mono = order == 1 && acc_smem && wb >= 5 &&
+                                  e->tune_get("bh.eval_unroll", 2) == 2;
+        const bool default_quad = order == 2 && wb <= 3 && npl < 2;
+        TreeState a = *t;
+        if (!frozen && bpl == 2 && e->tune_get("bh.persistent", 1) != 0 &&
+            (emit || default_mono || default_quad))
+            a = split_state(e, emit);
+        if (a.parts > 1) {
+            if (emit)
+                kern = clamp ? bh_split_walk_kernel<true, 5, 1, true, 2, true>
+                             : bh_split_walk_kernel<false, 5, 1, true, 2, true>;
+            else if (default_quad)
+                kern = clamp ? bh_split_walk_kernel<true, 3, 2, false, 1>
+                             : bh_split_walk_kernel<false, 3, 2, false, 1>;
+            else if (npl >= 2)
+                kern = clamp ? bh_split_walk_kernel<true, 5, 1, true, 2>
+                             : bh_split_walk_kernel<false, 5, 1, true, 2>;
+            else
+                kern = clamp ? bh_split_walk_kernel<true, 5, 1, true, 1>
+                             : bh_split_walk_kernel<false, 5, 1, true, 1>;
+        }
         NBG_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-        const int warps = n / (32 * bpl);
         // "bh.test_cap": node tests after which a group walk gives up and
         // its bodies are walked one by one; 0 (the default) sets it to
         // "bh.test_cap_ratio" (default 2) times the median tests of
@@ -1569,34 +1786,42 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
         // the walk is not capped and the pre-pass is skipped.
         t->test_cap = (unsigned long long)std::max<int64_t>(e->tune_get("bh.test_cap", 0), 0);
         if (t->test_cap == 0 && t->curve == 0) t->test_cap = ~0ull;
+        a.test_cap = t->test_cap;
+        // the walk's counters (and, of a shared walk, its groups')
+        NBG_CUDA(e, cudaMemsetAsync(t->fb_count, 0,
+                                    sizeof(WalkCtl) + (a.parts > 1 ? 2 * sizeof(unsigned) * (size_t)warps : 0),
+                                    e->stream));
         if (t->test_cap == 0) {
-            const unsigned ratio = (unsigned)std::max<int64_t>(e->tune_get("bh.test_cap_ratio", 2), 1);
-            const int samples = std::min(warps, kCapSamples);  // both powers of two
-            const size_t csmem = (size_t)kCapSamples * stack_cap * sizeof(int);
+            TreeState tc = *t;
+            tc.cap_ratio = (unsigned)std::max<int64_t>(e->tune_get("bh.test_cap_ratio", 2), 1);
+            tc.cap_samples = std::min(warps, kCapSamples);  // both powers of two
+            tc.cap_stride = warps / tc.cap_samples;
+            const size_t csmem = (size_t)kCapWarps * stack_cap * sizeof(int);
             auto capk = bpl == 4 ? bh_test_cap_kernel<4>
                         : bpl == 2 ? bh_test_cap_kernel<2> : bh_test_cap_kernel<1>;
             NBG_CUDA(e, cudaFuncSetAttribute(capk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)csmem));
             // the cap counts acceptance tests: against the step build's
             // records when those decide acceptance
-            TreeState tc = *t;
             if (frozen) tc.node4 = t->node4_acc;
-            capk<<<1, kCapSamples * 32, csmem, e->stream>>>(n, warps / samples, samples, tc,
-                                                            stack_cap, ratio);
+            capk<<<(unsigned)tc.cap_samples, kCapWarps * 32, csmem, e->stream>>>(n, tc, stack_cap);
             NBG_LAUNCHED(e, "bh_test_cap_kernel");
         }
-        // fb_count[0]: groups handed to the fallback, [1]: the walk's next group
-        NBG_CUDA(e, cudaMemsetAsync(t->fb_count, 0, 2 * sizeof(unsigned), e->stream));
         // "bh.persistent" (default 1): as many CTAs as fit at once; 0: one
         // CTA per kGWWarps groups
-        unsigned blocks = (unsigned)((warps + kGWWarps - 1) / kGWWarps);
+        unsigned blocks = (unsigned)((warps * a.parts + kGWWarps - 1) / kGWWarps);
         if (e->tune_get("bh.persistent", 1) != 0) {
             int per_sm = 0;
             NBG_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGWThreads, smem));
             blocks = std::min(blocks, (unsigned)std::max(per_sm, 1) * (unsigned)e->sm_count);
         }
-        kern<<<blocks, kGWThreads, smem, e->stream>>>(y, f, n, eps2, *t, stack_cap, e->d_err);
+        kern<<<blocks, kGWThreads, smem, e->stream>>>(y, f, n, eps2, a, stack_cap, e->d_err);
         NBG_LAUNCHED(e, "bh_group_walk_kernel");
+        if (a.parts > 1) {
+            auto finish = emit ? bh_walk_finish_kernel<true> : bh_walk_finish_kernel<false>;
+            finish<<<(unsigned)warps, 192, 0, e->stream>>>(y, f, n, a);
+            NBG_LAUNCHED(e, "bh_walk_finish_kernel");
+        }
         if (emit) return NBG_OK;
         auto fb = frozen
             ? (clamp ? bh_body_walk_kernel<true, 2, 1, true> : bh_body_walk_kernel<false, 2, 1, true>)

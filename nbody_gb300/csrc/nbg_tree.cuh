@@ -90,10 +90,31 @@ struct TreeState {
     // The cap is test_cap when that is set, else cap_state[0], set from the
     // test counts of sampled groups by bh_test_cap_kernel.
     int* fb_list = nullptr;                  // [n / 32]
-    unsigned* fb_count = nullptr;            // [2]: queued groups, the walk's next group
+    unsigned* fb_count = nullptr;            // [2]: queued groups, the walk's next group; then WalkCtl's rest
     unsigned long long* cap_state = nullptr; // [1]
     unsigned long long test_cap = 0;
+    // the shared group walk (bh_split_walk_kernel), set per launch: warps per
+    // group, the level under which subtrees are dealt out, the partial sums
+    // [parts][3][n] in leaf order, and the sampled groups that set the cap
+    int parts = 1, top = 0;
+    double* part = nullptr;
+    int* cand_part = nullptr;         // [groups][parts][cand_cap] the parts' band cells
+    unsigned* cand_part_n = nullptr;  // [groups][parts], above cand_cap: too many
+    int cap_samples = 0, cap_stride = 0;
+    unsigned cap_ratio = 0;
 };
+
+// Counters of one walk, at fb_count, zeroed before it.
+constexpr int kCapSamples = 32;  // groups whose node tests set the walk's cap
+struct WalkCtl {
+    unsigned fb_count;           // groups handed to the per-body walk
+    unsigned next;               // next group (or share of one) to take
+    unsigned long long bound;    // ~(an upper bound of the cap), 0 = none yet
+    unsigned finished[kCapSamples];  // sampled groups: node tests + 1, 0 = not known
+    unsigned done;               // sampled groups finished or given up
+    unsigned group[1];           // of a shared walk: [groups] node tests, then [groups] interactions
+};
+inline size_t walk_ctl_words(size_t n) { return sizeof(WalkCtl) / 4 + 2 * (n / 32 + 1); }
 
 // Stack entries per warp of the group and per-body walks: 48 per tree level
 // plus 32 (a step pops 16 entries and pushes at most 32), set per launch
