@@ -834,6 +834,193 @@ nbg_status direct_sym_launch(nbg_engine* e, const double* y, double* f) {
     return NBG_OK;
 }
 
+// ---------------------------------------------------------------------------
+// mixed kernel for small systems
+// ---------------------------------------------------------------------------
+// The symmetric kernel's units (1024 bodies times 128) are too few for a small
+// system: 120 at 5003 bodies, one CTA of four warps each, 23 us for what the
+// FP32 pipe does in 5.  Smaller units cost it an FP64 conversion and atomic
+// per A body and unit (the FP64 pipe takes 16 cycles a warp instruction).
+// Here all ordered pairs are evaluated: the sixteen warps of a CTA hold the
+// same 64 bodies, two a lane, and each takes every sixteenth quad of the
+// others, so the block's sums leave the CTA once.  The (block, quad) pairs are
+// divided evenly over one CTA per SM, whose segments begin and end anywhere.
+// Pairs are packed over the quad's bodies, whose records of four float4 need
+// no duplication.  Bound by the FP32 pipe (11 packed operations a pair with
+// equal masses, 12 else) and, below 4000 bodies, by its two launches.
+constexpr int kSmallWarps = 16;
+constexpr int kSmallThreads = kSmallWarps * 32;
+constexpr int kSmallB = 2;        // bodies per lane, 32 kSmallB a block
+constexpr int kSmallFold = 16;    // quads a warp sums before the sums are folded
+constexpr long long kSmallMin = 32;  // at least so many quads per CTA
+// Up to this size the small-system kernel: fcompute 21 / 10 us at 1000 bodies
+// (symmetric / small), 25 / 14 at 3000, 25 / 21 at 5003, 35 / 35 at 8000,
+// 97 / 107 at 16000.
+constexpr int kSmallMax = 8192;
+
+struct SmallArgs {
+    const float4* quads;  // 4 bodies: (x x x x) (y y y y) (z z z z) (m m m m)
+    double* acc;          // a-part of f: [3][n]
+    double m_uni;         // the common mass (uniform-mass kernel)
+    int n;
+    int nq;               // quads of the n bodies
+    long long units;      // blocks * nq
+    float eps2;
+};
+
+__global__ void pack_small_kernel(const double* __restrict__ y, const double* __restrict__ mass,
+                                  float* __restrict__ out, double* __restrict__ f, int n, int n_pad) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_pad) return;
+    // padding bodies as in pack_sym_kernel
+    float x = 1e18f, yy = 1e18f, z = 1e18f, m = 0.f;
+    if (i < n) {
+        x = (float)y[i];
+        yy = (float)y[n + i];
+        z = (float)y[2 * n + i];
+        m = (float)mass[i];
+        f[i] = y[3 * n + i];
+        f[n + i] = y[4 * n + i];
+        f[2 * n + i] = y[5 * n + i];
+        f[3 * n + i] = 0.0;
+        f[4 * n + i] = 0.0;
+        f[5 * n + i] = 0.0;
+    }
+    float* q = out + (size_t)(i >> 2) * 16 + (i & 3);
+    q[0] = x;
+    q[4] = yy;
+    q[8] = z;
+    q[12] = m;
+}
+
+template <bool CLAMP, bool UNI>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+direct_small_kernel(SmallArgs a) {
+    constexpr int B = kSmallB;
+    __shared__ float2 red[kSmallWarps][3 * B][32];  // sums as hi + lo
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float* scalars = reinterpret_cast<const float*>(a.quads);
+    const long long per = a.units / gridDim.x, rem = a.units % gridDim.x;
+    long long u = blockIdx.x * per + min((long long)blockIdx.x, rem);
+    const long long u1 = u + per + ((long long)blockIdx.x < rem ? 1 : 0);
+    const f2_t eps2 = f2_pack(a.eps2, a.eps2), zero = f2_pack(0.f, 0.f);
+    while (u < u1) {
+        const int blk = (int)(u / a.nq), qa = (int)(u % a.nq);
+        const int qb = (int)min((long long)a.nq, qa + (u1 - u));
+        u += qb - qa;
+        f2_t xi[B], yi[B], zi[B], hi[3 * B], lo[3 * B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int i = (blk * B + b) * 32 + lane;
+            const float* q = scalars + (size_t)(i >> 2) * 16 + (i & 3);
+            const float x = __ldg(q), y = __ldg(q + 4), z = __ldg(q + 8);
+            xi[b] = f2_pack(x, x);
+            yi[b] = f2_pack(y, y);
+            zi[b] = f2_pack(z, z);
+        }
+#pragma unroll
+        for (int k = 0; k < 3 * B; ++k) hi[k] = lo[k] = zero;
+        float4 nX, nY, nZ, nM = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto load = [&](int q) {
+            const float4* p = a.quads + 4 * (size_t)q;
+            nX = __ldg(p);
+            nY = __ldg(p + 1);
+            nZ = __ldg(p + 2);
+            if (!UNI) nM = __ldg(p + 3);
+        };
+        load(min(qa + warp, a.nq - 1));
+        for (int q0 = qa + warp; q0 < qb; q0 += kSmallFold * kSmallWarps) {
+            const int q1 = min(qb, q0 + kSmallFold * kSmallWarps);
+            f2_t ax[B], ay[B], az[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) ax[b] = ay[b] = az[b] = zero;
+#pragma unroll 2
+            for (int q = q0; q < q1; q += kSmallWarps) {
+                const float4 X = nX, Y = nY, Z = nZ, M = nM;
+                load(min(q + kSmallWarps, a.nq - 1));  // in flight over this quad's terms
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    const f2_t x0 = f2_pack(X.x, X.y), x1 = f2_pack(X.z, X.w);
+                    const f2_t y0 = f2_pack(Y.x, Y.y), y1 = f2_pack(Y.z, Y.w);
+                    const f2_t z0 = f2_pack(Z.x, Z.y), z1 = f2_pack(Z.z, Z.w);
+                    if constexpr (UNI) {
+                        pair_uni<CLAMP>(x0, y0, z0, xi[b], yi[b], zi[b], eps2, ax[b], ay[b], az[b]);
+                        pair_uni<CLAMP>(x1, y1, z1, xi[b], yi[b], zi[b], eps2, ax[b], ay[b], az[b]);
+                    } else {
+                        pair2<CLAMP>(x0, y0, z0, f2_pack(M.x, M.y), xi[b], yi[b], zi[b], eps2,
+                                     ax[b], ay[b], az[b]);
+                        pair2<CLAMP>(x1, y1, z1, f2_pack(M.z, M.w), xi[b], yi[b], zi[b], eps2,
+                                     ax[b], ay[b], az[b]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                f2_two_sum(hi[3 * b + 0], lo[3 * b + 0], ax[b]);
+                f2_two_sum(hi[3 * b + 1], lo[3 * b + 1], ay[b]);
+                f2_two_sum(hi[3 * b + 2], lo[3 * b + 2], az[b]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3 * B; ++k) {
+            float h0, h1, l0, l1;
+            f2_unpack(hi[k], h0, h1);
+            f2_unpack(lo[k], l0, l1);
+            // (in FP32: the FP64 pipe takes 16 cycles per warp instruction)
+            const float s1 = h0 + h1, b1 = s1 - h0;
+            red[warp][k][lane] = make_float2(s1, ((h0 - (s1 - b1)) + (h1 - b1)) + (l0 + l1));
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < 96 * B; t += kSmallThreads) {
+            const int k = t >> 5, i = (blk * B + k / 3) * 32 + lane;
+            float2 s = red[0][k][lane];
+#pragma unroll
+            for (int w = 1; w < kSmallWarps; ++w) {
+                const float2 p = red[w][k][lane];
+                const float s1 = s.x + p.x, b1 = s1 - s.x;
+                s = make_float2(s1, s.y + (((s.x - (s1 - b1)) + (p.x - b1)) + p.y));
+            }
+            const double v = (double)s.x + (double)s.y;
+            if (i < a.n) atomicAdd(a.acc + (size_t)(k % 3) * a.n + i, UNI ? a.m_uni * v : v);
+        }
+        __syncthreads();
+    }
+}
+
+nbg_status direct_small_launch(nbg_engine* e, const double* y, double* f) {
+    const int n = (int)e->count;
+    constexpr int B = kSmallB;
+    const int n_pad = (n + 32 * B - 1) / (32 * B) * (32 * B);
+    if (!reserve_scratch(e, (size_t)n_pad * sizeof(float4)))
+        return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
+    pack_small_kernel<<<(unsigned)(n_pad + 127) / 128, 128, 0, e->stream>>>(
+        y, e->d_mass, reinterpret_cast<float*>(e->d_xyzm), f, n, n_pad);
+    NBG_LAUNCHED(e, "pack_small_kernel");
+    const bool clamp = !(e->params.softening > 0.0);
+    const bool uni = e->uniform_mass && e->tune_get("direct.uniform_mass", 1) != 0;
+    using SmallKernel = void (*)(SmallArgs);
+    SmallKernel kern =
+        uni ? (clamp ? direct_small_kernel<true, true> : direct_small_kernel<false, true>)
+            : (clamp ? direct_small_kernel<true, false> : direct_small_kernel<false, false>);
+    int occ = 0;
+    NBG_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kSmallThreads, 0));
+    SmallArgs a;
+    a.quads = e->d_xyzm;
+    a.acc = f + 3 * (size_t)n;
+    a.m_uni = e->mass_value;
+    a.n = n;
+    a.nq = (n + 3) / 4;
+    a.units = (long long)(n_pad / (32 * B)) * a.nq;
+    a.eps2 = (float)(e->params.softening * e->params.softening);
+    // at least kSmallMin quads a CTA
+    const long long fit = (a.units + kSmallMin - 1) / kSmallMin;
+    const long long grid = std::min((long long)e->sm_count * std::max(occ, 1), std::max(fit, 1LL));
+    ProfScope ps(e, NBG_K_DIRECT);
+    kern<<<(unsigned)grid, kSmallThreads, 0, e->stream>>>(a);
+    NBG_LAUNCHED(e, "direct_small_kernel");
+    return NBG_OK;
+}
+
 // Which FP64 kernel: the split path from kSplitMin bodies on, where its five
 // launches and the FP64 share of its pairs cost less than the FP64 pipe's 16
 // operations a pair (1024 bodies: 46 us against 100; 1536: 91 against 84;
@@ -886,7 +1073,12 @@ nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
     if (e->params.precision == NBG_PREC_FP64) return direct_fp64_launch(e, y, f);
 
     // ---- mixed precision ----
-    if (e->tune_get("direct.symmetric", 1) != 0) return direct_sym_launch(e, y, f);
+    if (e->tune_get("direct.symmetric", 1) != 0) {
+        // ("direct.sym_g" asks for the symmetric kernel of that shape)
+        const bool small = n <= kSmallMax && e->tune_get("direct.sym_g", 0) == 0;
+        return e->tune_get("direct.small", small) != 0 ? direct_small_launch(e, y, f)
+                                                       : direct_sym_launch(e, y, f);
+    }
     const int n_jt = (n + kT - 1) / kT;
     const int n_pad = n_jt * kT;
     const size_t need = (size_t)n_pad * sizeof(Body2);

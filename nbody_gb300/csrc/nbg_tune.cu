@@ -52,6 +52,8 @@ namespace {
 
 std::vector<Candidate> direct_candidates() {
     std::vector<Candidate> c;
+    c.push_back({{"direct.symmetric", 1}, {"direct.small", 1}});
+    const size_t first = c.size();
     for (int bps : {0, 3, 2})
         c.push_back({{"direct.symmetric", 1}, {"direct.sym_blocks", 4}, {"direct.blocks_per_sm", bps}});
     c.push_back({{"direct.symmetric", 1}, {"direct.sym_blocks", 5}, {"direct.blocks_per_sm", 0}});
@@ -59,6 +61,7 @@ std::vector<Candidate> direct_candidates() {
         c.push_back({{"direct.symmetric", 1}, {"direct.sym_blocks", 4}, {"direct.sym_unroll", ru},
                      {"direct.blocks_per_sm", 0}});
     c.push_back({{"direct.symmetric", 1}, {"direct.sym_g", 3}, {"direct.blocks_per_sm", 0}});
+    for (size_t i = first; i < c.size(); ++i) c[i].push_back({"direct.small", 0});
     for (int g : {4, 2})
         for (int unr : {2, 4, 8}) {
             if (g == 4 && unr == 8) continue;  // not instantiated
