@@ -50,6 +50,7 @@ __device__ __forceinline__ int next_down(int idx) { return (idx >> (__ffs(~idx) 
 __global__ void bh_walk_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                                     double* __restrict__ f, int n, int nested, TreeState t,
                                     unsigned* err) {
+    if (!after_previous()) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= n) return;
     const size_t sz = t.size;
@@ -158,6 +159,7 @@ struct SplitNode {
 };
 
 __global__ void __launch_bounds__(256) split_nodes_kernel(SplitSystem s, TreeState t) {
+    if (!after_previous()) return;
     const int ex = split_exponent(s);
     for (size_t i = 1 + blockIdx.x * (size_t)256 + threadIdx.x; i < t.size; i += (size_t)gridDim.x * 256) {
         // with masses of both signs a centre may lie outside the bodies'
@@ -195,6 +197,7 @@ __device__ __noinline__ bool accept_fp64(const TreeState& t, size_t node, size_t
 }
 
 __global__ void __launch_bounds__(32, 16) bh_walk_split_kernel(SplitWalkArgs a) {
+    if (!after_previous()) return;
     __shared__ uint3 stack[kSWStack];
     __shared__ uint3 list[kSWList + 1];  // node, bodies that accepted it (two masks)
     __shared__ unsigned queue[2][kSWQ][32];
@@ -428,6 +431,7 @@ __global__ void __launch_bounds__(32, 16) bh_walk_split_kernel(SplitWalkArgs a) 
 
 __global__ void __launch_bounds__(128)
 split_walk_sum_kernel(SplitWalkArgs a, const double* __restrict__ y, double* __restrict__ f) {
+    if (!after_previous()) return;
     const size_t n = (size_t)a.s.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
     if (at >= 3 * n) return;
     const int b = a.t.body_n[n + at % n];
@@ -444,6 +448,7 @@ template <bool CLAMP>
 __global__ void __launch_bounds__(256)
 bh_walk_mixed_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2,
                      TreeState t, unsigned* err) {
+    if (!after_previous()) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     if ((tid & ~31) >= n) return;  // whole warps past the last body
@@ -1118,6 +1123,7 @@ template <bool CLAMP, int MINB, int BPL, int ORDER, int EUNR = 2, bool SMACC = f
 __global__ void __launch_bounds__(kGWThreads, MINB)
 bh_group_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2v,
                      TreeState t, int stack_cap, unsigned* err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int groups = n / (32 * BPL);
@@ -1144,6 +1150,7 @@ template <bool CLAMP, int MINB, int ORDER, bool SMACC, int NPL, bool EMIT = fals
 __global__ void __launch_bounds__(kGWThreads, MINB)
 bh_split_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2v,
                      TreeState t, int stack_cap, unsigned* err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int tasks = n / 64 * t.parts;
@@ -1163,6 +1170,7 @@ bh_split_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n
 template <bool EMIT>
 __global__ void __launch_bounds__(192)
 bh_walk_finish_kernel(const double* __restrict__ y, double* __restrict__ f, int n, TreeState t) {
+    if (!after_previous()) return;
     const WalkCtl* ctl = reinterpret_cast<const WalkCtl*>(t.fb_count);
     const int gw = blockIdx.x, tid = threadIdx.x;
     const unsigned long long cap = t.test_cap != 0 ? t.test_cap : t.cap_state[0];
@@ -1211,6 +1219,7 @@ constexpr int kCapTop = 6;
 template <int BPL>
 __global__ void __launch_bounds__(kCapWarps * 32, 1)
 bh_test_cap_kernel(int n, TreeState t, int stack_cap) {
+    if (!after_previous()) return;
     extern __shared__ int cap_stacks[];
     __shared__ unsigned total;
     __shared__ int stopped;
@@ -1322,6 +1331,7 @@ template <bool CLAMP, int BPL, int ORDER, bool FROZEN = false>
 __global__ void __launch_bounds__(kGWThreads)
 bh_body_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2,
                     TreeState t, int stack_cap, unsigned* err) {
+    if (!after_previous()) return;
     extern __shared__ int body_stacks[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -1437,6 +1447,7 @@ bh_body_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n,
 // M = sum over children of M_c + m_c d d^T, d = child centre - node centre);
 // leaves have none.
 __global__ void quad_leaf_kernel(float4* quad, int n) {
+    if (!after_previous()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         quad[2 * (size_t)(n + p)] = make_float4(0.f, 0.f, 0.f, 0.f);
         quad[2 * (size_t)(n + p) + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1470,6 +1481,7 @@ __device__ __forceinline__ void quad_node(size_t idx, TreeState& t) {
 // owns the subtree under node 2^lv_lo + b (at most 9 levels, 256 nodes at
 // its bottom), a block barrier between levels.
 __global__ void __launch_bounds__(256) quad_levels_kernel(int lv_lo, int lv_hi, TreeState t) {
+    if (!after_previous()) return;
     const size_t root = ((size_t)1 << lv_lo) + blockIdx.x;
     for (int lv = lv_hi - 1; lv >= lv_lo; --lv) {
         const int span = 1 << (lv - lv_lo);
@@ -1485,12 +1497,12 @@ nbg_status tree_quadrupoles(nbg_engine* e) {
     if (t->quad == nullptr) {
         NBG_CUDA(e, cudaMalloc(&t->quad, 2 * t->size * sizeof(float4)));
         // leaves have no moments; only inner nodes are written afterwards
-        quad_leaf_kernel<<<grid_for(n, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(t->quad, n);
+        queued(quad_leaf_kernel, grid_for(n, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(t->quad, n);
         NBG_LAUNCHED(e, "quad_leaf_kernel");
     }
     for (int hi = t->levels; hi > 0;) {
         const int lo = std::max(0, hi - 9);
-        quad_levels_kernel<<<1u << lo, 256, 0, e->stream>>>(lo, hi, *t);
+        queued(quad_levels_kernel, 1u << lo, 256, 0, e->stream)(lo, hi, *t);
         NBG_LAUNCHED(e, "quad_levels_kernel");
         hi = lo;
     }
@@ -1502,6 +1514,7 @@ nbg_status tree_quadrupoles(nbg_engine* e) {
 namespace {
 // Residual of each leaf's FP32 position (frozen acceptance): lo = y - hi.
 __global__ void leaf_lo_kernel(const double* __restrict__ y, int n, TreeState t) {
+    if (!after_previous()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const int b = t.body_n[n + p];
         const float4 hi = t.node4[n + p];
@@ -1542,7 +1555,7 @@ nbg_status bh_tree(nbg_engine* e, uint64_t step, const double* y, bool fp64_node
         if (tt->leaf_lo == nullptr)
             NBG_CUDA(e, cudaMalloc(&tt->leaf_lo, tt->n * sizeof(float4)));
         const int n = (int)tt->n;
-        leaf_lo_kernel<<<grid_for(n, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
+        queued(leaf_lo_kernel, grid_for(n, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(
             y, n, *tt);
         NBG_LAUNCHED(e, "leaf_lo_kernel");
     }
@@ -1570,16 +1583,16 @@ nbg_status bh_fcompute(nbg_engine* e, uint64_t step, const double* y, double* f)
             if (s != NBG_OK) return s;
             a.t = *e->tree;
             a.part = reinterpret_cast<double*>(reinterpret_cast<char*>(e->d_xyzm) + system);
-            split_nodes_kernel<<<grid_for(2 * (size_t)n, 256, (unsigned)e->sm_count * 8u), 256, 0,
-                                 e->stream>>>(a.s, a.t);
+            queued(split_nodes_kernel, grid_for(2 * (size_t)n, 256, (unsigned)e->sm_count * 8u), 256, 0,
+                                 e->stream)(a.s, a.t);
             NBG_LAUNCHED(e, "split_nodes_kernel");
-            bh_walk_split_kernel<<<dim3((unsigned)groups, (unsigned)a.parts), 32, 0, e->stream>>>(a);
+            queued(bh_walk_split_kernel, dim3((unsigned)groups, (unsigned)a.parts), 32, 0, e->stream)(a);
             NBG_LAUNCHED(e, "bh_walk_split_kernel");
-            split_walk_sum_kernel<<<(unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream>>>(a, y, f);
+            queued(split_walk_sum_kernel, (unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream)(a, y, f);
             NBG_LAUNCHED(e, "split_walk_sum_kernel");
             return NBG_OK;
         }
-        bh_walk_fp64_kernel<<<(n + 127) / 128, 128, 0, e->stream>>>(
+        queued(bh_walk_fp64_kernel, (n + 127) / 128, 128, 0, e->stream)(
             y, e->d_mass, f, n, e->params.traverse_type == NBG_TRAVERSE_NESTED_TREE ? 1 : 0,
             *e->tree, e->d_err);
         NBG_LAUNCHED(e, "bh_walk_fp64_kernel");
@@ -1804,7 +1817,7 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
             // the cap counts acceptance tests: against the step build's
             // records when those decide acceptance
             if (frozen) tc.node4 = t->node4_acc;
-            capk<<<(unsigned)tc.cap_samples, kCapWarps * 32, csmem, e->stream>>>(n, tc, stack_cap);
+            queued(capk, (unsigned)tc.cap_samples, kCapWarps * 32, csmem, e->stream)(n, tc, stack_cap);
             NBG_LAUNCHED(e, "bh_test_cap_kernel");
         }
         // "bh.persistent" (default 1): as many CTAs as fit at once; 0: one
@@ -1815,11 +1828,11 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
             NBG_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGWThreads, smem));
             blocks = std::min(blocks, (unsigned)std::max(per_sm, 1) * (unsigned)e->sm_count);
         }
-        kern<<<blocks, kGWThreads, smem, e->stream>>>(y, f, n, eps2, a, stack_cap, e->d_err);
+        queued(kern, blocks, kGWThreads, smem, e->stream)(y, f, n, eps2, a, stack_cap, e->d_err);
         NBG_LAUNCHED(e, "bh_group_walk_kernel");
         if (a.parts > 1) {
             auto finish = emit ? bh_walk_finish_kernel<true> : bh_walk_finish_kernel<false>;
-            finish<<<(unsigned)warps, 192, 0, e->stream>>>(y, f, n, a);
+            queued(finish, (unsigned)warps, 192, 0, e->stream)(y, f, n, a);
             NBG_LAUNCHED(e, "bh_walk_finish_kernel");
         }
         if (emit) return NBG_OK;
@@ -1834,7 +1847,7 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
                      : (bpl == 2 ? bh_body_walk_kernel<false, 2, 1> : bh_body_walk_kernel<false, 1, 1>));
         const size_t fsmem = (size_t)kGWWarps * stack_cap * sizeof(int);
         NBG_CUDA(e, cudaFuncSetAttribute(fb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
-        fb<<<(unsigned)e->sm_count * 8u, kGWThreads, fsmem, e->stream>>>(y, f, n, eps2, *t, stack_cap,
+        queued(fb, (unsigned)e->sm_count * 8u, kGWThreads, fsmem, e->stream)(y, f, n, eps2, *t, stack_cap,
                                                                      e->d_err);
         NBG_LAUNCHED(e, "bh_body_walk_kernel");
         return NBG_OK;
@@ -1846,10 +1859,10 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
     // every warp is full; n is a power of two, so only n < 32 has such lanes
     const int threads = ((n + 31) / 32) * 32;
     if (clamp)
-        bh_walk_mixed_kernel<true><<<(threads + 255) / 256, 256, 0, e->stream>>>(y, f, n, eps2, *t,
+        queued(bh_walk_mixed_kernel<true>, (threads + 255) / 256, 256, 0, e->stream)(y, f, n, eps2, *t,
                                                                                e->d_err);
     else
-        bh_walk_mixed_kernel<false><<<(threads + 255) / 256, 256, 0, e->stream>>>(y, f, n, eps2, *t,
+        queued(bh_walk_mixed_kernel<false>, (threads + 255) / 256, 256, 0, e->stream)(y, f, n, eps2, *t,
                                                                                 e->d_err);
     NBG_LAUNCHED(e, "bh_walk_mixed_kernel");
     return NBG_OK;

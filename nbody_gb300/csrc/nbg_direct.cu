@@ -75,6 +75,7 @@ constexpr int kF64Threads = 32;  // one warp per CTA: the fewest idle SMs in the
 __global__ void __launch_bounds__(kF64Threads)
 direct_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                    double* __restrict__ f, int n) {
+    if (!after_previous()) return;
     const int lane = threadIdx.x & 31;
     const int i = (int)((blockIdx.x * kF64Threads + threadIdx.x) >> 5);
     if (i >= n) return;
@@ -129,6 +130,7 @@ struct SplitArgs {
 
 template <bool UNI>
 __global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
+    if (!after_previous()) return;
     __shared__ __align__(16) float4 tile[kSplitTile][6];  // every word twice, for FP32x2
     __shared__ unsigned queue[2][kSplitQ][kSplitT];
     const int tid = threadIdx.x;
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(kSplitT, 4) split_force_kernel(SplitArgs a) {
 }
 
 __global__ void __launch_bounds__(128) split_reduce_kernel(SplitArgs a) {
+    if (!after_previous()) return;
     const size_t sn = (size_t)a.s.n, at = (size_t)blockIdx.x * 128 + threadIdx.x;
     if (at >= 3 * sn) return;
     double s = 0.0;
@@ -262,6 +265,7 @@ struct Body2 {  // one body in duplicated form, 32 bytes
 __global__ void pack_mixed_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                                   Body2* __restrict__ out, double* __restrict__ f, int n,
                                   int n_pad) {
+    if (!after_previous()) return;
     int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pad; i += stride) {
         Body2 b;
@@ -308,6 +312,7 @@ __device__ __forceinline__ void issue_tile(Body2* tiles, uint64_t* full, int s, 
 template <bool CLAMP, int G, int UNR>
 __global__ void __launch_bounds__(kThreadsMixed, G >= 4 ? 4 : kMinBlocksMixed)
 direct_mixed_kernel(MixedArgs a) {
+    if (!after_previous()) return;
     constexpr int kIB = kThreadsMixed * 2 * G;
     constexpr int kSlots = 6 * G;  // (hi, lo) x 3 components x G pairs
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -503,6 +508,7 @@ __device__ __forceinline__ size_t sym_xy(int i) { return (size_t)(i >> 7) * 256 
 __global__ void pack_sym_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                                 float4* __restrict__ out, double* __restrict__ f, int n,
                                 int n_pad) {
+    if (!after_previous()) return;
     int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pad; i += stride) {
         // padding bodies: zero mass, and parked at 1e18 on every axis, where
@@ -585,6 +591,7 @@ __device__ __forceinline__ void sym_issue(float4* tiles, uint64_t* full, int s, 
 template <bool CLAMP, int MINB, int RUNR, int G = 4, bool UNI = false>
 __global__ void __launch_bounds__(kSymThreads, MINB)
 direct_sym_kernel(SymArgs a) {
+    if (!after_previous()) return;
     constexpr int kSymRange = sym_range(G);
     constexpr int kSymTilesPerRange = kSymRange / kSymT;
     constexpr int kSlots = 6 * G;
@@ -778,7 +785,7 @@ nbg_status direct_sym_launch(nbg_engine* e, const double* y, double* f) {
     if (!reserve_scratch(e, need))
         return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
     float4* bodies = reinterpret_cast<float4*>(e->d_xyzm);
-    pack_sym_kernel<<<grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
+    queued(pack_sym_kernel, grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(
         y, e->d_mass, bodies, f, n, n_pad);
     NBG_LAUNCHED(e, "pack_sym_kernel");
     const bool clamp = !(e->params.softening > 0.0);
@@ -829,7 +836,7 @@ nbg_status direct_sym_launch(nbg_engine* e, const double* y, double* f) {
     long long grid = (long long)e->sm_count * occ;
     if (grid > a.units) grid = a.units;
     ProfScope ps(e, NBG_K_DIRECT);
-    kern<<<(unsigned)grid, kSymThreads, smem, e->stream>>>(a);
+    queued(kern, (unsigned)grid, kSymThreads, smem, e->stream)(a);
     NBG_LAUNCHED(e, "direct_sym_kernel");
     return NBG_OK;
 }
@@ -870,6 +877,7 @@ struct SmallArgs {
 
 __global__ void pack_small_kernel(const double* __restrict__ y, const double* __restrict__ mass,
                                   float* __restrict__ out, double* __restrict__ f, int n, int n_pad) {
+    if (!after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
     // padding bodies as in pack_sym_kernel
@@ -896,6 +904,7 @@ __global__ void pack_small_kernel(const double* __restrict__ y, const double* __
 template <bool CLAMP, bool UNI>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 direct_small_kernel(SmallArgs a) {
+    if (!after_previous()) return;
     constexpr int B = kSmallB;
     __shared__ float2 red[kSmallWarps][3 * B][32];  // sums as hi + lo
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -993,7 +1002,7 @@ nbg_status direct_small_launch(nbg_engine* e, const double* y, double* f) {
     const int n_pad = (n + 32 * B - 1) / (32 * B) * (32 * B);
     if (!reserve_scratch(e, (size_t)n_pad * sizeof(float4)))
         return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
-    pack_small_kernel<<<(unsigned)(n_pad + 127) / 128, 128, 0, e->stream>>>(
+    queued(pack_small_kernel, (unsigned)(n_pad + 127) / 128, 128, 0, e->stream)(
         y, e->d_mass, reinterpret_cast<float*>(e->d_xyzm), f, n, n_pad);
     NBG_LAUNCHED(e, "pack_small_kernel");
     const bool clamp = !(e->params.softening > 0.0);
@@ -1016,7 +1025,7 @@ nbg_status direct_small_launch(nbg_engine* e, const double* y, double* f) {
     const long long fit = (a.units + kSmallMin - 1) / kSmallMin;
     const long long grid = std::min((long long)e->sm_count * std::max(occ, 1), std::max(fit, 1LL));
     ProfScope ps(e, NBG_K_DIRECT);
-    kern<<<(unsigned)grid, kSmallThreads, 0, e->stream>>>(a);
+    queued(kern, (unsigned)grid, kSmallThreads, 0, e->stream)(a);
     NBG_LAUNCHED(e, "direct_small_kernel");
     return NBG_OK;
 }
@@ -1046,7 +1055,7 @@ nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
     split = split && reserve_scratch(e, system + (size_t)a.ranges * 3 * n * sizeof(double));
     if (!split) {
         const unsigned warps = kF64Threads / 32;
-        direct_fp64_kernel<<<((unsigned)n + warps - 1) / warps, kF64Threads, 0, e->stream>>>(
+        queued(direct_fp64_kernel, ((unsigned)n + warps - 1) / warps, kF64Threads, 0, e->stream)(
             y, e->d_mass, f, n);
         NBG_LAUNCHED(e, "direct_fp64_kernel");
         return NBG_OK;
@@ -1057,11 +1066,11 @@ nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
     if (s != NBG_OK) return s;
     const dim3 grid((unsigned)blocks, (unsigned)a.ranges);
     if (e->uniform_mass)
-        split_force_kernel<true><<<grid, kSplitT, 0, e->stream>>>(a);
+        queued(split_force_kernel<true>, grid, kSplitT, 0, e->stream)(a);
     else
-        split_force_kernel<false><<<grid, kSplitT, 0, e->stream>>>(a);
+        queued(split_force_kernel<false>, grid, kSplitT, 0, e->stream)(a);
     NBG_LAUNCHED(e, "split_force_kernel");
-    split_reduce_kernel<<<(unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream>>>(a);
+    queued(split_reduce_kernel, (unsigned)((3 * (size_t)n + 127) / 128), 128, 0, e->stream)(a);
     NBG_LAUNCHED(e, "split_reduce_kernel");
     return NBG_OK;
 }
@@ -1085,7 +1094,7 @@ nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
     if (!reserve_scratch(e, need))
         return cuda_error(e, cudaErrorMemoryAllocation, "the packed bodies' buffer");
     Body2* bodies = reinterpret_cast<Body2*>(e->d_xyzm);
-    pack_mixed_kernel<<<grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
+    queued(pack_mixed_kernel, grid_for(n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(
         y, e->d_mass, bodies, f, n, n_pad);
     NBG_LAUNCHED(e, "pack_mixed_kernel");
 
@@ -1114,7 +1123,7 @@ nbg_status direct_fcompute(nbg_engine* e, const double* y, double* f) {
     long long grid = (long long)e->sm_count * occ;
     if (grid > a.units) grid = a.units;
     ProfScope ps(e, NBG_K_DIRECT);
-    kern<<<(unsigned)grid, kThreadsMixed, smem, e->stream>>>(a);
+    queued(kern, (unsigned)grid, kThreadsMixed, smem, e->stream)(a);
     NBG_LAUNCHED(e, "direct_mixed_kernel");
     return NBG_OK;
 }
@@ -1210,7 +1219,7 @@ extern "C" nbg_status nbg_direct_mixed_noalloc(const double* y, const double* ma
         cudaGetLastError();
         return NBG_ERR_CUDA;
     }
-    pack_mixed_kernel<<<grid_for(n_pad, 256, (unsigned)d.sm_count * 8u), 256, 0, st>>>(
+    queued(pack_mixed_kernel, grid_for(n_pad, 256, (unsigned)d.sm_count * 8u), 256, 0, st)(
         y, mass, d.bodies, f, nn, n_pad);
     MixedArgs a;
     a.bodies = d.bodies;
@@ -1223,7 +1232,7 @@ extern "C" nbg_status nbg_direct_mixed_noalloc(const double* y, const double* ma
     a.err = d.err;
     long long grid = (long long)d.sm_count * occ;
     if (grid > a.units) grid = a.units;
-    kern<<<(unsigned)grid, kThreadsMixed, smem, st>>>(a);
+    queued(kern, (unsigned)grid, kThreadsMixed, smem, st)(a);
     if (cudaGetLastError() != cudaSuccess) return NBG_ERR_CUDA;
 
     // Synchronous: the result is in f when this returns, and a device-side

@@ -145,6 +145,40 @@ struct ProfScope {
     ~ProfScope() { prof_end(e, kid, ev); }
 };
 
+// ---- launches ---------------------------------------------------------------
+// queued(kernel, grid, block, smem, stream)(arguments): a launch whose set-up
+// overlaps the previous kernel's end (programmatic stream serialisation); the
+// kernel itself waits for that end in after_previous(), its first statement,
+// so the order of all memory accesses is that of ordinary launches.  It saves
+// 2.5 to 3 us between two kernels: fcompute of 1000 bodies (2 kernels) 10.6 ->
+// 5.9 us, a Barnes-Hut Euler step of 1024 bodies (9 kernels) 98 -> 76 us, of
+// 2^17 (33 kernels) 530 -> 466 us.
+template <class... P>
+struct Queued {
+    void (*kernel)(P...);
+    dim3 grid, block;
+    size_t smem;
+    cudaStream_t stream;
+    template <class... A>
+    void operator()(A&&... args) const {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // (errors: NBG_LAUNCHED)
+    }
+};
+template <class... P>
+Queued<P...> queued(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
+    return {kernel, grid, block, smem, stream};
+}
+
 // ---- grid helpers ----------------------------------------------------------
 inline unsigned grid_for(size_t n, unsigned block, unsigned cap) {
     size_t g = (n + block - 1) / block;

@@ -48,6 +48,7 @@ using namespace mlp;
 // node moments and features
 // ---------------------------------------------------------------------------
 __global__ void moments_leaf_kernel(double* mom, size_t sz, int n) {
+    if (!after_previous()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
         for (int q = 0; q < 6; ++q) mom[q * sz + n + p] = 0.0;
 }
@@ -55,6 +56,7 @@ __global__ void moments_leaf_kernel(double* mom, size_t sz, int n) {
 // Parallel-axis combination: Q = Q_l + Q_r + m_l d_l d_l^T + m_r d_r d_r^T,
 // d = child centre - parent centre.  Order (xx, yy, zz, xy, xz, yz).
 __global__ void moments_level_kernel(int first, int count, TreeState t, double* mom) {
+    if (!after_previous()) return;
     const size_t sz = t.size;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const size_t idx = (size_t)first + k;
@@ -79,6 +81,7 @@ __global__ void moments_level_kernel(int first, int count, TreeState t, double* 
 // feat[3 * idx + 0..2] = (Qxx, Qyy, Qzz, Qxy)/(m s^2), (Qxz, Qyz)/(m s^2), ex, ey,
 //                        ez, ox, oy, oz
 __global__ void features_kernel(TreeState t, const double* mom, double lambda) {
+    if (!after_previous()) return;
     const size_t sz = t.size;
     for (size_t idx = 1 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < sz;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -122,6 +125,7 @@ __device__ __forceinline__ float wat(const float* w, int layer, int k, int n) {
 
 __global__ void make_frags_kernel(const float* __restrict__ w, uint2* __restrict__ frag,
                                   float* __restrict__ bias) {
+    if (!after_previous()) return;
     const int tile = blockIdx.x;  // 0 .. kTiles-1
     const int lane = threadIdx.x;
     int layer, kt, nt;
@@ -256,6 +260,7 @@ train_kernel(const float* __restrict__ x, const float* __restrict__ tg, const in
              size_t b0, size_t bsize, const uint2* __restrict__ frag_g,
              const float* __restrict__ bias_g, float* __restrict__ grad_part,
              double* __restrict__ loss_part, float wnorm) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
     for (int i = threadIdx.x; i < kFragWords; i += blockDim.x) S.frag[i] = frag_g[i];
@@ -460,6 +465,7 @@ train_kernel(const float* __restrict__ x, const float* __restrict__ tg, const in
 __global__ void grad_reduce_kernel(const float* __restrict__ grad_part, int blocks,
                                    float* __restrict__ grad, const double* __restrict__ loss_part,
                                    double* __restrict__ loss) {
+    if (!after_previous()) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
         float v = grad_part[i];
         for (int b = 1; b < blocks; ++b) v += grad_part[(size_t)b * kParams + i];
@@ -474,6 +480,7 @@ __global__ void grad_reduce_kernel(const float* __restrict__ grad_part, int bloc
 
 __global__ void adam_kernel(float* w, float* grad, float* m1, float* m2, float lr, float b1,
                             float b2, float eps, float c1, float c2, int n) {
+    if (!after_previous()) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gr = grad[i];
         const float a = b1 * m1[i] + (1.f - b1) * gr;
@@ -503,6 +510,7 @@ __global__ void sample_pairs_kernel(const int* __restrict__ leaves, int nb, Tree
                                     int* __restrict__ pairs, unsigned* __restrict__ counts,
                                     const unsigned long long* __restrict__ first,
                                     unsigned long long cap) {
+    if (!after_previous()) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nb) return;
     const int leaf = leaves[k];
@@ -545,6 +553,7 @@ __global__ void sample_targets_kernel(const int* __restrict__ pairs, size_t npai
                                       TreeState t, int n, int levels, double lambda, double eps2,
                                       float* __restrict__ xo, float* __restrict__ to,
                                       int* __restrict__ meta) {
+    if (!after_previous()) return;
     const int lane = threadIdx.x & 31;
     const size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= npairs) return;
@@ -610,6 +619,7 @@ __global__ void __launch_bounds__(kWalkThreads)
 learned_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2,
                     float band2, float inv_lambda, TreeState t, const uint2* __restrict__ frag_g,
                     const float* __restrict__ bias_g, unsigned* err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WalkSmem& S = *reinterpret_cast<WalkSmem*>(smem_raw);
     for (int i = threadIdx.x; i < kFragWords; i += blockDim.x) S.frag[i] = frag_g[i];
@@ -755,6 +765,7 @@ learned_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n,
 __global__ void __launch_bounds__(128)
 predict_kernel(const float* __restrict__ x, size_t count, float* __restrict__ out,
                const uint2* __restrict__ frag_g, const float* __restrict__ bias_g) {
+    if (!after_previous()) return;
     __shared__ uint2 frag[kFragWords];
     __shared__ float bias[kBias];
     __shared__ uint32_t xs[4][32 * 8];
@@ -795,7 +806,7 @@ nbg_status learn_alloc(nbg_engine* e) {
 
 nbg_status rebuild_frags(nbg_engine* e) {
     LearnState* L = e->learn;
-    make_frags_kernel<<<kTiles, 32, 0, e->stream>>>(L->w, L->frag, L->bias);
+    queued(make_frags_kernel, kTiles, 32, 0, e->stream)(L->w, L->frag, L->bias);
     NBG_LAUNCHED(e, "make_frags_kernel");
     return tc_rebuild_weights(e);
 }
@@ -816,15 +827,15 @@ nbg_status tree_features(nbg_engine* e) {
     }
     const int n = (int)t->n;
     const unsigned g = grid_for(n, 256, (unsigned)e->sm_count * 8u);
-    moments_leaf_kernel<<<g, 256, 0, e->stream>>>(L->mom, sz, n);
+    queued(moments_leaf_kernel, g, 256, 0, e->stream)(L->mom, sz, n);
     NBG_LAUNCHED(e, "moments_leaf_kernel");
     for (int lv = t->levels - 1; lv >= 0; --lv) {
         const int first = 1 << lv;
-        moments_level_kernel<<<grid_for(first, 256, (unsigned)e->sm_count * 8u), 256, 0,
-                               e->stream>>>(first, first, *t, L->mom);
+        queued(moments_level_kernel, grid_for(first, 256, (unsigned)e->sm_count * 8u), 256, 0,
+                               e->stream)(first, first, *t, L->mom);
         NBG_LAUNCHED(e, "moments_level_kernel");
     }
-    features_kernel<<<grid_for(sz, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(
+    queued(features_kernel, grid_for(sz, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(
         *t, L->mom, t->lambda);
     NBG_LAUNCHED(e, "features_kernel");
     return NBG_OK;
@@ -877,7 +888,7 @@ nbg_status learned_walk(nbg_engine* e, const double* y, double* f) {
     auto kern = group ? learned_walk_kernel<true> : learned_walk_kernel<false>;
     NBG_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int threads = ((n + 31) / 32) * 32;
-    kern<<<(threads + kWalkThreads - 1) / kWalkThreads, kWalkThreads, smem, e->stream>>>(
+    queued(kern, (threads + kWalkThreads - 1) / kWalkThreads, kWalkThreads, smem, e->stream)(
         y, f, n, eps2, band2, (float)(1.0 / lam_l), *t, e->learn->frag, e->learn->bias, e->d_err);
     NBG_LAUNCHED(e, "learned_walk_kernel");
     return NBG_OK;
@@ -1033,7 +1044,7 @@ nbg_status nbg_learn_generate(nbg_engine* e, size_t max_samples, uint64_t seed,
     DevScratch s_counts, s_first;
     NBG_CUDA(e, cudaMalloc(&s_counts.p, nb * sizeof(unsigned)));
     NBG_CUDA(e, cudaMalloc(&s_first.p, nb * sizeof(unsigned long long)));
-    sample_pairs_kernel<false><<<(nb + 127) / 128, 128, 0, e->stream>>>(
+    queued(sample_pairs_kernel<false>, (nb + 127) / 128, 128, 0, e->stream)(
         d_bodies, nb, *t, n, band2, max_subtree_log2, t->levels, nullptr, s_counts.as<unsigned>(),
         nullptr, 0ull);
     NBG_LAUNCHED(e, "sample_pairs_kernel");
@@ -1049,7 +1060,7 @@ nbg_status nbg_learn_generate(nbg_engine* e, size_t max_samples, uint64_t seed,
     }
     NBG_CUDA(e, cudaMemcpyAsync(s_first.p, first.data(), nb * sizeof(unsigned long long),
                                 cudaMemcpyHostToDevice, e->stream));
-    sample_pairs_kernel<true><<<(nb + 127) / 128, 128, 0, e->stream>>>(
+    queued(sample_pairs_kernel<true>, (nb + 127) / 128, 128, 0, e->stream)(
         d_bodies, nb, *t, n, band2, max_subtree_log2, t->levels, L->pairs, nullptr,
         s_first.as<unsigned long long>(), (unsigned long long)max_samples);
     NBG_LAUNCHED(e, "sample_pairs_kernel");
@@ -1057,7 +1068,7 @@ nbg_status nbg_learn_generate(nbg_engine* e, size_t max_samples, uint64_t seed,
     if (np > 0) {
         const double eps2 = e->params.softening * e->params.softening;
         const size_t threads = np * 32;
-        sample_targets_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, e->stream>>>(
+        queued(sample_targets_kernel, (unsigned)((threads + 255) / 256), 256, 0, e->stream)(
             L->pairs, np, y, e->d_mass, *t, n, t->levels, lam_l, eps2, L->x + L->count * 16,
             L->t + L->count * 4, L->meta + L->count * 2);
         NBG_LAUNCHED(e, "sample_targets_kernel");
@@ -1112,10 +1123,10 @@ static nbg_status run_train_pass(nbg_engine* e, const float* x, const float* t, 
         NBG_CUDA(e, cudaMalloc(&L->loss_part, (size_t)grid * sizeof(double)));
         L->part_blocks = (int)grid;
     }
-    train_kernel<<<grid, kTrainWarps * 32, smem, e->stream>>>(
+    queued(train_kernel, grid, kTrainWarps * 32, smem, e->stream)(
         x, t, order, b0, bsize, L->frag, L->bias, L->grad_part, L->loss_part, wnorm);
     NBG_LAUNCHED(e, "train_kernel");
-    grad_reduce_kernel<<<(kParams + 255) / 256, 256, 0, e->stream>>>(L->grad_part, (int)grid,
+    queued(grad_reduce_kernel, (kParams + 255) / 256, 256, 0, e->stream)(L->grad_part, (int)grid,
                                                                        L->grad, L->loss_part,
                                                                        L->loss);
     NBG_LAUNCHED(e, "grad_reduce_kernel");
@@ -1203,7 +1214,7 @@ nbg_status nbg_learn_train(nbg_engine* e, int epochs, size_t batch, double lr, u
             L->adam_step++;
             const double c1 = 1.0 - std::pow(0.9, (double)L->adam_step);
             const double c2 = 1.0 - std::pow(0.999, (double)L->adam_step);
-            adam_kernel<<<(kParams + adam_threads - 1) / adam_threads, adam_threads, 0, e->stream>>>(
+            queued(adam_kernel, (kParams + adam_threads - 1) / adam_threads, adam_threads, 0, e->stream)(
                 L->w, L->grad, L->m1, L->m2, (float)lr_t, 0.9f, 0.999f, 1e-8f, (float)c1,
                 (float)c2, kParams);
             NBG_LAUNCHED(e, "adam_kernel");
@@ -1275,7 +1286,7 @@ nbg_status nbg_learn_predict(nbg_engine* e, const float* x, size_t count, float*
     float* dout = sout.as<float>();
     NBG_CUDA(e, cudaMemcpyAsync(dx, x, count * 16 * sizeof(float), cudaMemcpyHostToDevice, e->stream));
     const size_t warps = (count + 31) / 32;
-    predict_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, e->stream>>>(dx, count, dout, e->learn->frag,
+    queued(predict_kernel, (unsigned)((warps + 3) / 4), 128, 0, e->stream)(dx, count, dout, e->learn->frag,
                                                                     e->learn->bias);
     NBG_LAUNCHED(e, "predict_kernel");
     std::vector<float> tmp(count * 4);

@@ -96,6 +96,7 @@ __device__ __forceinline__ float bf16_round(float x) {
 // carry GELU's factor 1/2 (exact in BF16): the epilogue forms 2 GELU(z) =
 // z + z tanh(u) with one FMA, and the products are the same bit for bit.
 __global__ void make_tc_weights_kernel(const float* __restrict__ w, uint32_t* __restrict__ tcw) {
+    if (!after_previous()) return;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     constexpr int q1 = 64 * 8, q2 = q1 + 64 * 32, q3 = q2 + 16 * 32;
     if (q < q1) {  // W1^T: n < 64, K = 16
@@ -291,6 +292,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
 learned_tc_kernel(double* __restrict__ f, int n, int groups, TreeState t,
                   const uint32_t* __restrict__ tcw, float inv_lambda,
                   unsigned* __restrict__ next, unsigned* __restrict__ err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(smem_tc);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -463,6 +465,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
 predict_tc_kernel(const float* __restrict__ x, int count, float* __restrict__ out,
                   float* __restrict__ acc_out, const uint32_t* __restrict__ tcw,
                   unsigned* __restrict__ next, unsigned* __restrict__ err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(smem_tc);
     const int tid = threadIdx.x;
@@ -516,6 +519,7 @@ learned_body_walk_kernel(const double* __restrict__ y, double* __restrict__ f, i
                          float band2, float inv_lambda, TreeState t, int stack_cap,
                          const uint2* __restrict__ frag_g, const float* __restrict__ bias_g,
                          unsigned* err) {
+    if (!after_previous()) return;
     extern __shared__ __align__(128) unsigned char smem_lb[];
     LbSmem& S = *reinterpret_cast<LbSmem*>(smem_lb);
     int* stacks = reinterpret_cast<int*>(smem_lb + sizeof(LbSmem));
@@ -639,7 +643,7 @@ nbg_status tc_rebuild_weights(nbg_engine* e) {
     LearnState* L = e->learn;
     if (L->tcw == nullptr) NBG_CUDA(e, cudaMalloc(&L->tcw, kTcwWords * sizeof(uint32_t)));
     const int threads = 64 * 8 + 64 * 32 + 16 * 32 + 144;
-    make_tc_weights_kernel<<<(threads + 255) / 256, 256, 0, e->stream>>>(L->w, L->tcw);
+    queued(make_tc_weights_kernel, (threads + 255) / 256, 256, 0, e->stream)(L->w, L->tcw);
     NBG_LAUNCHED(e, "make_tc_weights_kernel");
     return NBG_OK;
 }
@@ -702,7 +706,7 @@ nbg_status learned_tc_walk(nbg_engine* e, const double* y, double* f) {
     const size_t lsmem = sizeof(LbSmem) + (size_t)kLbWarps * stack_cap * sizeof(int);
     auto lb = clamp ? learned_body_walk_kernel<true> : learned_body_walk_kernel<false>;
     NBG_CUDA(e, cudaFuncSetAttribute(lb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem));
-    lb<<<(unsigned)e->sm_count * 4u, kLbWarps * 32, lsmem, e->stream>>>(
+    queued(lb, (unsigned)e->sm_count * 4u, kLbWarps * 32, lsmem, e->stream)(
         y, f, n, eps2, band2, inv_lambda, *t, stack_cap, L->frag, L->bias, e->d_err);
     NBG_LAUNCHED(e, "learned_body_walk_kernel");
     // band rows on the tensor cores
@@ -716,7 +720,7 @@ nbg_status learned_tc_walk(nbg_engine* e, const double* y, double* f) {
     tt.band2 = band2;
     const unsigned blocks =
         (unsigned)std::min<long>(groups, (long)kTcBlocksPerSm * e->sm_count);
-    learned_tc_kernel<<<blocks, kTcThreads, tc_smem_bytes(), e->stream>>>(
+    queued(learned_tc_kernel, blocks, kTcThreads, tc_smem_bytes(), e->stream)(
         f, n, groups, tt, L->tcw, inv_lambda, L->tc_next, e->d_err);
     NBG_LAUNCHED(e, "learned_tc_kernel");
     return NBG_OK;
@@ -747,7 +751,7 @@ static nbg_status predict_tc(nbg_engine* e, const float* x, size_t count, float*
     NBG_CUDA(e, cudaMemsetAsync(L->tc_next, 0, sizeof(unsigned), e->stream));
     const long units = (long)((count + kTcRows - 1) / kTcRows);
     const unsigned blocks = (unsigned)std::min<long>(units, (long)kTcBlocksPerSm * e->sm_count);
-    predict_tc_kernel<<<blocks, kTcThreads, tc_smem_bytes(), e->stream>>>(
+    queued(predict_tc_kernel, blocks, kTcThreads, tc_smem_bytes(), e->stream)(
         dx, (int)count, dout, dacc, L->tcw, L->tc_next, e->d_err);
     NBG_LAUNCHED(e, "predict_tc_kernel");
     if (acc != nullptr)

@@ -58,6 +58,7 @@ struct SplitSystem {
 };
 
 __global__ void __launch_bounds__(256) split_extent_kernel(SplitSystem a) {
+    if (!after_previous()) return;
     unsigned long long m = 0;
     const size_t n3 = 3 * (size_t)a.n;
     for (size_t i = blockIdx.x * 256 + threadIdx.x; i < n3; i += (size_t)gridDim.x * 256)
@@ -84,6 +85,7 @@ __device__ __forceinline__ int split_exponent(const SplitSystem& a) {
 }
 
 __global__ void __launch_bounds__(256) split_pack_kernel(SplitSystem a) {
+    if (!after_previous()) return;
     const int ex = split_exponent(a);
     for (int i = blockIdx.x * 256 + threadIdx.x; i < a.n_pad; i += gridDim.x * 256) {
         SplitBody b;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitSystem a) {
 // CTA against one of kSplitEst ranges, in FP32x2.
 template <bool POT>
 __global__ void __launch_bounds__(kSplitT) split_estimate_kernel(SplitSystem a) {
+    if (!after_previous()) return;
     __shared__ __align__(16) float4 tile[kSplitT][2];
     const int tid = threadIdx.x;
     const int i0 = blockIdx.x * 2 * kSplitT + tid, i1 = i0 + kSplitT;  // < n_pad
@@ -233,12 +236,12 @@ nbg_status split_prepare(nbg_engine* e, SplitSystem* a, const double* y, const d
     a->bodies = static_cast<SplitBody*>(at);
     a->extent = reinterpret_cast<unsigned long long*>(a->bodies + a->n_pad);
     a->est = reinterpret_cast<float*>(a->extent + kSplitExtents);
-    split_extent_kernel<<<kSplitExtents, 256, 0, e->stream>>>(*a);
+    queued(split_extent_kernel, kSplitExtents, 256, 0, e->stream)(*a);
     NBG_LAUNCHED(e, "split_extent_kernel");
-    split_pack_kernel<<<grid_for(a->n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream>>>(*a);
+    queued(split_pack_kernel, grid_for(a->n_pad, 256, (unsigned)e->sm_count * 8u), 256, 0, e->stream)(*a);
     NBG_LAUNCHED(e, "split_pack_kernel");
     const dim3 grid((unsigned)(a->n_pad / (2 * kSplitT)), kSplitEst);
-    split_estimate_kernel<POT><<<grid, kSplitT, 0, e->stream>>>(*a);
+    queued(split_estimate_kernel<POT>, grid, kSplitT, 0, e->stream)(*a);
     NBG_LAUNCHED(e, "split_estimate_kernel");
     return NBG_OK;
 }

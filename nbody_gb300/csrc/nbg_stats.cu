@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(kStatThreads)
 stats_linear_kernel(const double* __restrict__ y, const double* __restrict__ mass, size_t stride,
                     const long long* __restrict__ off, const int* __restrict__ cnt, int n_single,
                     double* __restrict__ lin) {
+    if (!after_previous()) return;
     __shared__ double sh[kStatThreads / 32];
     const int s = blockIdx.x;
     const long long o = off != nullptr ? off[s] : 0;
@@ -83,6 +84,7 @@ stats_linear_kernel(const double* __restrict__ y, const double* __restrict__ mas
 __global__ void __launch_bounds__(32 * (kLinSums + 1))
 stats_finish_kernel(const double* __restrict__ lin, int parts, const double* __restrict__ pot,
                     int npot, double* __restrict__ out) {
+    if (!after_previous()) return;
     __shared__ double res[kLinSums + 1];
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double v = 0.0;
@@ -146,6 +148,7 @@ stats_potential_kernel(const double* __restrict__ y, const double* __restrict__ 
                        const long long* __restrict__ off, const int* __restrict__ cnt,
                        const PairUnit* __restrict__ units, double eps2,
                        double* __restrict__ out) {
+    if (!after_previous()) return;
     __shared__ double tx[kStatThreads], ty[kStatThreads], tz[kStatThreads], tm[kStatThreads];
     __shared__ double sh[kStatThreads / 32];
     const PairUnit u = units[blockIdx.x];
@@ -218,6 +221,7 @@ struct PotArgs {
 
 template <bool SOFT>
 __global__ void __launch_bounds__(kSplitT, 4) split_potential_kernel(PotArgs a) {
+    if (!after_previous()) return;
     __shared__ __align__(16) float4 tile[kSplitTile][6];
     __shared__ unsigned queue[2][kSplitQ][kSplitT];
     __shared__ double sh[kSplitT / 32];
@@ -348,6 +352,7 @@ template <bool SOFT>
 __global__ void __launch_bounds__(32)
 pot_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass, int n, double eps2,
                 double* __restrict__ part) {
+    if (!after_previous()) return;
     const int i = blockIdx.x, lane = threadIdx.x;
     const size_t sn = (size_t)n;
     const double x1 = y[i], y1 = y[sn + i], z1 = y[2 * sn + i];
@@ -390,7 +395,7 @@ nbg_status stats_single(nbg_engine* e, const double* y, const double* mass, int 
     a.part = reinterpret_cast<double*>(reinterpret_cast<char*>(e->d_xyzm) + system);
     double* lin = a.part + npot;
     double* res = lin + (size_t)parts * kLinSums;
-    stats_linear_kernel<<<dim3(1, (unsigned)parts), kStatThreads, 0, e->stream>>>(
+    queued(stats_linear_kernel, dim3(1, (unsigned)parts), kStatThreads, 0, e->stream)(
         y, mass, (size_t)n, nullptr, nullptr, n, lin);
     NBG_LAUNCHED(e, "stats_linear_kernel");
     if (split) {
@@ -398,18 +403,18 @@ nbg_status stats_single(nbg_engine* e, const double* y, const double* mass, int 
         if (s != NBG_OK) return s;
         const dim3 grid((unsigned)a.blocks, (unsigned)rows);
         if (eps2 > 0.0)
-            split_potential_kernel<true><<<grid, kSplitT, 0, e->stream>>>(a);
+            queued(split_potential_kernel<true>, grid, kSplitT, 0, e->stream)(a);
         else
-            split_potential_kernel<false><<<grid, kSplitT, 0, e->stream>>>(a);
+            queued(split_potential_kernel<false>, grid, kSplitT, 0, e->stream)(a);
         NBG_LAUNCHED(e, "split_potential_kernel");
     } else {
         if (eps2 > 0.0)
-            pot_fp64_kernel<true><<<(unsigned)n, 32, 0, e->stream>>>(y, mass, n, eps2, a.part);
+            queued(pot_fp64_kernel<true>, (unsigned)n, 32, 0, e->stream)(y, mass, n, eps2, a.part);
         else
-            pot_fp64_kernel<false><<<(unsigned)n, 32, 0, e->stream>>>(y, mass, n, eps2, a.part);
+            queued(pot_fp64_kernel<false>, (unsigned)n, 32, 0, e->stream)(y, mass, n, eps2, a.part);
         NBG_LAUNCHED(e, "pot_fp64_kernel");
     }
-    stats_finish_kernel<<<1, 32 * (kLinSums + 1), 0, e->stream>>>(lin, parts, a.part,
+    queued(stats_finish_kernel, 1, 32 * (kLinSums + 1), 0, e->stream)(lin, parts, a.part,
                                                                   npot, res);
     NBG_LAUNCHED(e, "stats_finish_kernel");
     NBG_CUDA(e, cudaMemcpyAsync(out, res, 12 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
@@ -435,15 +440,15 @@ nbg_status stats_segments(nbg_engine* e, const double* y, const double* mass, si
     NBG_CUDA(e, cudaMemsetAsync(d_out, 0, 12 * (size_t)nsys * sizeof(double), e->stream));
     DevScratch lin;
     NBG_CUDA(e, cudaMalloc(&lin.p, (size_t)nsys * kLinSums * sizeof(double)));
-    stats_linear_kernel<<<nsys, kStatThreads, 0, e->stream>>>(y, mass, stride, d_off, d_cnt, 0,
+    queued(stats_linear_kernel, nsys, kStatThreads, 0, e->stream)(y, mass, stride, d_off, d_cnt, 0,
                                                               lin.as<double>());
     NBG_LAUNCHED(e, "stats_linear_kernel");
-    stats_finish_kernel<<<nsys, 32 * (kLinSums + 1), 0, e->stream>>>(lin.as<double>(), 1, nullptr, 0,
+    queued(stats_finish_kernel, nsys, 32 * (kLinSums + 1), 0, e->stream)(lin.as<double>(), 1, nullptr, 0,
                                                                      d_out);
     NBG_LAUNCHED(e, "stats_finish_kernel");
     if (!units.empty()) {
         auto kern = eps2 > 0.0 ? stats_potential_kernel<true> : stats_potential_kernel<false>;
-        kern<<<(unsigned)units.size(), kStatThreads, 0, e->stream>>>(y, mass, stride, d_off, d_cnt,
+        queued(kern, (unsigned)units.size(), kStatThreads, 0, e->stream)(y, mass, stride, d_off, d_cnt,
                                                                      d_units, eps2, d_out);
         NBG_LAUNCHED(e, "stats_potential_kernel");
     }

@@ -34,6 +34,7 @@
 #include <cstring>
 
 #include "nbg_tree.cuh"
+#include "nbg_ptx.cuh"
 
 namespace nbg {
 namespace {
@@ -64,6 +65,7 @@ __device__ __forceinline__ unsigned digit_peers(unsigned dig) {
 
 __global__ void init_keys_kernel(const double* __restrict__ coord, int n,
                                  uint64_t* __restrict__ keys, int* __restrict__ vals) {
+    if (!after_previous()) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         keys[i] = order_key(coord[i]);
         vals[i] = i;
@@ -78,6 +80,7 @@ __device__ __forceinline__ double order_key_inverse(uint64_t k) {
 
 // box[0..2] = min order keys, box[3..5] = max order keys of x, y, z.
 __global__ void bbox_kernel(const double* __restrict__ y, int n, unsigned long long* box) {
+    if (!after_previous()) return;
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         for (int d = 0; d < 3; ++d) {
@@ -154,6 +157,7 @@ __global__ void morton_keys_kernel(const double* __restrict__ y, int n,
                                    const unsigned long long* __restrict__ box,
                                    uint64_t* __restrict__ keys, int* __restrict__ vals,
                                    int hilbert) {
+    if (!after_previous()) return;
     // the box's corner and scale, once per CTA
     __shared__ double s_lo[3], s_scale[3];
     if (threadIdx.x < 3) {
@@ -180,6 +184,7 @@ __global__ void morton_keys_kernel(const double* __restrict__ y, int n,
 // Per-block digit histogram: hist[digit * nblocks + block].
 __global__ void __launch_bounds__(kSortThreads)
 radix_hist_kernel(const uint64_t* __restrict__ keys, int n, int shift, unsigned* __restrict__ hist) {
+    if (!after_previous()) return;
     __shared__ unsigned h[kDigits];
     for (int d = threadIdx.x; d < kDigits; d += kSortThreads) h[d] = 0;
     __syncthreads();
@@ -197,6 +202,7 @@ radix_hist_kernel(const uint64_t* __restrict__ keys, int n, int shift, unsigned*
 // prefix of the totals (the digit base) itself.
 __global__ void __launch_bounds__(512)
 radix_digit_scan_kernel(unsigned* __restrict__ hist, int nblocks, unsigned* __restrict__ totals) {
+    if (!after_previous()) return;
     __shared__ unsigned warp_tot[16];
     __shared__ unsigned carry;
     const int d = blockIdx.x;
@@ -235,6 +241,7 @@ __global__ void __launch_bounds__(kSortThreads)
 radix_scatter_kernel(const uint64_t* __restrict__ kin, const int* __restrict__ vin,
                      uint64_t* __restrict__ kout, int* __restrict__ vout, int n, int shift,
                      const unsigned* __restrict__ offsets, const unsigned* __restrict__ totals) {
+    if (!after_previous()) return;
     constexpr int kWarpsS = kSortThreads / 32;
     __shared__ unsigned cnt[kWarpsS][kDigits];
     __shared__ unsigned gbase[kDigits];  // global start of this block's run of each digit
@@ -355,6 +362,7 @@ struct ClusterSortArgs {
 
 template <int ITEMS>
 __global__ void __launch_bounds__(kCSThreads, 1) cluster_sort_kernel(ClusterSortArgs a) {
+    if (!after_previous()) return;
     constexpr int kCSTile = kCSThreads * ITEMS;  // keys per CTA
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ClusterSortSmem<ITEMS>& S = *reinterpret_cast<ClusterSortSmem<ITEMS>*>(smem_raw);
@@ -476,6 +484,7 @@ __global__ void __launch_bounds__(kCSThreads, 1) cluster_sort_kernel(ClusterSort
 // split-axis list.
 __global__ void split_flag_kernel(const int* __restrict__ list, int n, int S,
                                   unsigned char* __restrict__ flag) {
+    if (!after_previous()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
         flag[list[p]] = (unsigned char)((p & (S - 1)) < (S >> 1));
 }
@@ -491,6 +500,7 @@ struct PartArgs {
 };
 
 __global__ void __launch_bounds__(256) part_count_kernel(PartArgs a) {
+    if (!after_previous()) return;
     const int* in = a.in[blockIdx.y];
     int c = 0;
     const int base = blockIdx.x * kPartTile;
@@ -512,6 +522,7 @@ __global__ void __launch_bounds__(256) part_count_kernel(PartArgs a) {
 // Stable partition of each segment by flag: left entries keep their order in
 // [seg, seg + S/2), right entries in [seg + S/2, seg + S).
 __global__ void __launch_bounds__(256) part_scatter_kernel(PartArgs a) {
+    if (!after_previous()) return;
     constexpr int kItems = kPartTile / 256;
     __shared__ int excl[kPartTile];  // exclusive count of lefts before each tile slot
     __shared__ int wsum[8];
@@ -598,6 +609,7 @@ struct LocalSmem {
 __global__ void __launch_bounds__(kLocalThreads)
 kd_local_kernel(const int* __restrict__ l0, const int* __restrict__ l1, const int* __restrict__ l2,
                 int* __restrict__ loc, int* __restrict__ order, int n, int lv) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LocalSmem& S = *reinterpret_cast<LocalSmem*>(smem_raw);
     const int seg = min(n, kLocalTile), base = blockIdx.x * seg;
@@ -673,6 +685,7 @@ kd_local_kernel(const int* __restrict__ l0, const int* __restrict__ l1, const in
 template <bool F32>
 __global__ void leaf_init_kernel(const int* __restrict__ order, const double* __restrict__ y,
                                  const double* __restrict__ mass, int n, TreeState t) {
+    if (!after_previous()) return;
     const size_t sz = t.size;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const int b = order[p];
@@ -706,6 +719,7 @@ __global__ void leaf_init_kernel(const int* __restrict__ order, const double* __
 // Refit leaves: new positions, same bodies (nbody/nbody_space_heap.cpp:45-53).
 template <bool F32>
 __global__ void leaf_refit_kernel(const double* __restrict__ y, int n, TreeState t) {
+    if (!after_previous()) return;
     const size_t sz = t.size;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const size_t idx = (size_t)n + p;
@@ -852,11 +866,11 @@ nbg_status radix_sort(nbg_engine* e, TreeState* t, int n, int first_pass = 0) {
     for (int pass = first_pass; pass < 8; ++pass) {
         const int shift = 8 * pass;
         const int src = pass & 1, dst = src ^ 1;
-        radix_hist_kernel<<<nblocks, kSortThreads, 0, e->stream>>>(t->keys[src], n, shift, t->hist);
+        queued(radix_hist_kernel, nblocks, kSortThreads, 0, e->stream)(t->keys[src], n, shift, t->hist);
         NBG_LAUNCHED(e, "radix_hist_kernel");
-        radix_digit_scan_kernel<<<kDigits, 512, 0, e->stream>>>(t->hist, nblocks, t->totals);
+        queued(radix_digit_scan_kernel, kDigits, 512, 0, e->stream)(t->hist, nblocks, t->totals);
         NBG_LAUNCHED(e, "radix_digit_scan_kernel");
-        radix_scatter_kernel<<<nblocks, kSortThreads, 0, e->stream>>>(
+        queued(radix_scatter_kernel, nblocks, kSortThreads, 0, e->stream)(
             t->keys[src], t->vals[src], t->keys[dst], t->vals[dst], n, shift, t->hist, t->totals);
         NBG_LAUNCHED(e, "radix_scatter_kernel");
     }
@@ -869,18 +883,20 @@ nbg_status cluster_sort_launch(nbg_engine* e, const ClusterSortArgs& a, int axes
     const size_t smem = sizeof(ClusterSortSmem<ITEMS>);
     NBG_CUDA(e, cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kCSCtas;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kCSCtas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kCSCtas, (unsigned)axes);
     cfg.blockDim = dim3(kCSThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = e->stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;  // (as queued() launches, which take no cluster)
     NBG_CUDA(e, cudaLaunchKernelEx(&cfg, cluster_sort_kernel<ITEMS>, a));
     NBG_LAUNCHED(e, "cluster_sort_kernel");
     return NBG_OK;
@@ -904,6 +920,7 @@ constexpr int kFusedLevels = 9;
 template <bool F32>
 __global__ void __launch_bounds__(256)
 update_levels_fused_kernel(int lv_lo, int lv_hi, double lambda2, TreeState t) {
+    if (!after_previous()) return;
     const size_t root = ((size_t)1 << lv_lo) + blockIdx.x;
     for (int lv = lv_hi - 1; lv >= lv_lo; --lv) {
         const int span = 1 << (lv - lv_lo);
@@ -921,9 +938,9 @@ nbg_status update_levels(nbg_engine* e, TreeState* t) {
     for (int hi = t->levels; hi > 0;) {
         const int lo = std::max(0, hi - kFusedLevels);
         if (t->f32)
-            update_levels_fused_kernel<true><<<1u << lo, 256, 0, e->stream>>>(lo, hi, lambda2, *t);
+            queued(update_levels_fused_kernel<true>, 1u << lo, 256, 0, e->stream)(lo, hi, lambda2, *t);
         else
-            update_levels_fused_kernel<false><<<1u << lo, 256, 0, e->stream>>>(lo, hi, lambda2, *t);
+            queued(update_levels_fused_kernel<false>, 1u << lo, 256, 0, e->stream)(lo, hi, lambda2, *t);
         NBG_LAUNCHED(e, "update_levels_fused_kernel");
         hi = lo;
     }
@@ -981,9 +998,9 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         // box = {min keys: all ones, max keys: zero}
         NBG_CUDA(e, cudaMemsetAsync(t->box, 0xFF, 3 * sizeof(unsigned long long), e->stream));
         NBG_CUDA(e, cudaMemsetAsync(t->box + 3, 0, 3 * sizeof(unsigned long long), e->stream));
-        bbox_kernel<<<std::min(g, (unsigned)e->sm_count * 2u), 256, 0, e->stream>>>(y, n, t->box);
+        queued(bbox_kernel, std::min(g, (unsigned)e->sm_count * 2u), 256, 0, e->stream)(y, n, t->box);
         NBG_LAUNCHED(e, "bbox_kernel");
-        morton_keys_kernel<<<g, 256, 0, e->stream>>>(y, n, t->box, t->keys[0], t->vals[0],
+        queued(morton_keys_kernel, g, 256, 0, e->stream)(y, n, t->box, t->keys[0], t->vals[0],
                                                      curve == 2 ? 1 : 0);
         NBG_LAUNCHED(e, "morton_keys_kernel");
         // the key bits from 16 up (47 of 63: the curve down to cells of
@@ -995,9 +1012,9 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
             s = radix_sort(e, t, n, 2);
         if (s != NBG_OK) return s;
         if (t->f32)
-            leaf_init_kernel<true><<<g, 256, 0, e->stream>>>(t->vals[0], y, e->d_mass, n, *t);
+            queued(leaf_init_kernel<true>, g, 256, 0, e->stream)(t->vals[0], y, e->d_mass, n, *t);
         else
-            leaf_init_kernel<false><<<g, 256, 0, e->stream>>>(t->vals[0], y, e->d_mass, n, *t);
+            queued(leaf_init_kernel<false>, g, 256, 0, e->stream)(t->vals[0], y, e->d_mass, n, *t);
         NBG_LAUNCHED(e, "leaf_init_kernel");
         s = update_levels(e, t);
         if (s != NBG_OK) return s;
@@ -1013,7 +1030,7 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         if (s != NBG_OK) return s;
     }
     for (int d = 0; d < 3 && n > kCSMax; ++d) {
-        init_keys_kernel<<<g, 256, 0, e->stream>>>(y + (size_t)d * n, n, t->keys[0], t->vals[0]);
+        queued(init_keys_kernel, g, 256, 0, e->stream)(y + (size_t)d * n, n, t->keys[0], t->vals[0]);
         NBG_LAUNCHED(e, "init_keys_kernel");
         nbg_status s = radix_sort(e, t, n);
         if (s != NBG_OK) return s;
@@ -1026,7 +1043,7 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
     for (; (n >> lv) > kLocalTile; ++lv) {
         const int S = n >> lv;
         const int d = lv % 3;
-        split_flag_kernel<<<g, 256, 0, e->stream>>>(t->lists[d], n, S, t->flag);
+        queued(split_flag_kernel, g, 256, 0, e->stream)(t->lists[d], n, S, t->flag);
         NBG_LAUNCHED(e, "split_flag_kernel");
         const int e0 = (d + 1) % 3, e1 = (d + 2) % 3;
         PartArgs a;
@@ -1039,9 +1056,9 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         a.ntiles = ntiles;
         a.n = n;
         a.S = S;
-        part_count_kernel<<<dim3(ntiles, 2), 256, 0, e->stream>>>(a);
+        queued(part_count_kernel, dim3(ntiles, 2), 256, 0, e->stream)(a);
         NBG_LAUNCHED(e, "part_count_kernel");
-        part_scatter_kernel<<<dim3(ntiles, 2), 256, 0, e->stream>>>(a);
+        queued(part_scatter_kernel, dim3(ntiles, 2), 256, 0, e->stream)(a);
         NBG_LAUNCHED(e, "part_scatter_kernel");
         int* tmp0 = t->lists[e0];
         int* tmp1 = t->lists[e1];
@@ -1052,14 +1069,14 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
     }
     NBG_CUDA(e, cudaFuncSetAttribute(kd_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(LocalSmem)));
-    kd_local_kernel<<<std::max(1, n / kLocalTile), kLocalThreads, sizeof(LocalSmem), e->stream>>>(
+    queued(kd_local_kernel, std::max(1, n / kLocalTile), kLocalThreads, sizeof(LocalSmem), e->stream)(
         t->lists[0], t->lists[1], t->lists[2], t->spare[0], t->spare[1], n, lv);
     NBG_LAUNCHED(e, "kd_local_kernel");
     // 3. leaves, then the bottom-up update
     if (t->f32)
-        leaf_init_kernel<true><<<g, 256, 0, e->stream>>>(t->spare[1], y, e->d_mass, n, *t);
+        queued(leaf_init_kernel<true>, g, 256, 0, e->stream)(t->spare[1], y, e->d_mass, n, *t);
     else
-        leaf_init_kernel<false><<<g, 256, 0, e->stream>>>(t->spare[1], y, e->d_mass, n, *t);
+        queued(leaf_init_kernel<false>, g, 256, 0, e->stream)(t->spare[1], y, e->d_mass, n, *t);
     NBG_LAUNCHED(e, "leaf_init_kernel");
     nbg_status s = update_levels(e, t);
     if (s != NBG_OK) return s;
@@ -1074,9 +1091,9 @@ nbg_status tree_refit(nbg_engine* e, const double* y, double lambda) {
     ProfScope ps(e, NBG_K_TREE_BUILD);
     const unsigned g = grid_for(n, 256, (unsigned)e->sm_count * 8u);
     if (t->f32)
-        leaf_refit_kernel<true><<<g, 256, 0, e->stream>>>(y, n, *t);
+        queued(leaf_refit_kernel<true>, g, 256, 0, e->stream)(y, n, *t);
     else
-        leaf_refit_kernel<false><<<g, 256, 0, e->stream>>>(y, n, *t);
+        queued(leaf_refit_kernel<false>, g, 256, 0, e->stream)(y, n, *t);
     NBG_LAUNCHED(e, "leaf_refit_kernel");
     return update_levels(e, t);
 }

@@ -6,6 +6,7 @@
 // an RK stage that combines i k-buffers reads each of them once and writes the
 // result once.  All kernels are HBM-bound: 8 bytes per element per operand.
 #include "nbg_internal.cuh"
+#include "nbg_ptx.cuh"
 
 namespace nbg {
 namespace {
@@ -13,6 +14,7 @@ namespace {
 constexpr unsigned kThreads = 256;
 
 __global__ void fill_kernel(double* __restrict__ a, double v, size_t n) {
+    if (!after_previous()) return;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) a[i] = v;
 }
@@ -22,6 +24,7 @@ __global__ void fill_kernel(double* __restrict__ a, double v, size_t n) {
 template <int MODE>
 __global__ void axpy_n_kernel(double* __restrict__ a, const double* __restrict__ base,
                               Terms t, size_t n) {
+    if (!after_previous()) return;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         double acc;
@@ -43,6 +46,7 @@ __global__ void axpy_n_kernel(double* __restrict__ a, const double* __restrict__
 // corr = (s - a) - corrected; a = s.  Explicit roundings, no contraction.
 __global__ void axpy_n_corr_kernel(double* __restrict__ a, double* __restrict__ corr, Terms t,
                                    size_t n) {
+    if (!after_previous()) return;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         double ai = a[i];
@@ -63,6 +67,7 @@ __global__ void axpy_n_corr_kernel(double* __restrict__ a, double* __restrict__ 
 // the bits and one atomicMax per block give the exact result.
 __global__ void maxabs_kernel(const double* __restrict__ a, size_t n,
                               unsigned long long* __restrict__ out) {
+    if (!after_previous()) return;
     unsigned long long m = 0ull;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -89,6 +94,7 @@ __global__ void maxabs_kernel(const double* __restrict__ a, size_t n,
 // Periodic wrap of positions into [-b, b] (nbody/nbody_engine_cuda_impl.cu:724-747,
 // nbody/nbody_engine_simple.cpp:175-199).
 __global__ void clamp_kernel(double* __restrict__ y, double b, size_t n) {
+    if (!after_previous()) return;
     double diam = 2.0 * b;
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -109,7 +115,7 @@ unsigned vec_grid(nbg_engine* e, size_t n) {
 nbg_status launch_fill(nbg_engine* e, double* a, double v, size_t n) {
     if (n == 0) return NBG_OK;
     ProfScope ps(e, NBG_K_VECOPS);
-    fill_kernel<<<vec_grid(e, n), kThreads, 0, e->stream>>>(a, v, n);
+    queued(fill_kernel, vec_grid(e, n), kThreads, 0, e->stream)(a, v, n);
     NBG_LAUNCHED(e, "fill_kernel");
     return NBG_OK;
 }
@@ -120,11 +126,11 @@ nbg_status launch_axpy_n(nbg_engine* e, double* a, const double* base, int mode,
     ProfScope ps(e, NBG_K_VECOPS);
     unsigned g = vec_grid(e, n);
     if (mode == kBasePtr)
-        axpy_n_kernel<1><<<g, kThreads, 0, e->stream>>>(a, base, t, n);
+        queued(axpy_n_kernel<1>, g, kThreads, 0, e->stream)(a, base, t, n);
     else if (mode == kBaseZero)
-        axpy_n_kernel<2><<<g, kThreads, 0, e->stream>>>(a, nullptr, t, n);
+        queued(axpy_n_kernel<2>, g, kThreads, 0, e->stream)(a, nullptr, t, n);
     else
-        axpy_n_kernel<0><<<g, kThreads, 0, e->stream>>>(a, nullptr, t, n);
+        queued(axpy_n_kernel<0>, g, kThreads, 0, e->stream)(a, nullptr, t, n);
     NBG_LAUNCHED(e, "axpy_n_kernel");
     return NBG_OK;
 }
@@ -132,7 +138,7 @@ nbg_status launch_axpy_n(nbg_engine* e, double* a, const double* base, int mode,
 nbg_status launch_axpy_n_corr(nbg_engine* e, double* a, double* corr, const Terms& t, size_t n) {
     if (n == 0) return NBG_OK;
     ProfScope ps(e, NBG_K_VECOPS);
-    axpy_n_corr_kernel<<<vec_grid(e, n), kThreads, 0, e->stream>>>(a, corr, t, n);
+    queued(axpy_n_corr_kernel, vec_grid(e, n), kThreads, 0, e->stream)(a, corr, t, n);
     NBG_LAUNCHED(e, "axpy_n_corr_kernel");
     return NBG_OK;
 }
@@ -140,7 +146,7 @@ nbg_status launch_axpy_n_corr(nbg_engine* e, double* a, double* corr, const Term
 nbg_status launch_maxabs(nbg_engine* e, const double* a, size_t n) {
     ProfScope ps(e, NBG_K_VECOPS);
     NBG_CUDA(e, cudaMemsetAsync(e->d_scalar, 0, sizeof(unsigned long long), e->stream));
-    maxabs_kernel<<<vec_grid(e, n), kThreads, 0, e->stream>>>(a, n, e->d_scalar);
+    queued(maxabs_kernel, vec_grid(e, n), kThreads, 0, e->stream)(a, n, e->d_scalar);
     NBG_LAUNCHED(e, "maxabs_kernel");
     return NBG_OK;
 }
@@ -148,7 +154,7 @@ nbg_status launch_maxabs(nbg_engine* e, const double* a, size_t n) {
 nbg_status launch_clamp(nbg_engine* e, double* y, double b, size_t n) {
     if (n == 0) return NBG_OK;
     ProfScope ps(e, NBG_K_VECOPS);
-    clamp_kernel<<<vec_grid(e, n), kThreads, 0, e->stream>>>(y, b, n);
+    queued(clamp_kernel, vec_grid(e, n), kThreads, 0, e->stream)(y, b, n);
     NBG_LAUNCHED(e, "clamp_kernel");
     return NBG_OK;
 }
