@@ -1619,23 +1619,25 @@ namespace {
 using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, unsigned*);
 
 // Warps per group of the default walk, and the state of such a walk with its
-// scratch (the parts' sums and, with emit, their band cells): a.parts is 1
-// where the groups fill half of the resident warps (20 per SM) or there is no
-// scratch.  A whole Euler step, one part against the number chosen here: 1024
-// bodies 128 / 98 us (16 parts), 16384 bodies 266 / 180 us (16), 2^16 bodies
-// 436 / 373 us (4; 385 with 8), and where one is kept, 2^17 bodies 528 / 532 us
-// (2), 2^17 with quadrupoles at ratio 1.3 468 / 524 us, 2^18 722 / 752 us: what
-// the parts save there their finish kernel and the doubled top of the tree cost.
+// scratch (the parts' sums and, with emit, their band cells).  By default
+// enough warps for ratio / 2 times the resident ones (20 per SM): a larger
+// ratio means more work per group to set against the second kernel and the top
+// of the tree, which every part walks.  fcompute with 1, 2, 4, 8 and 16 parts,
+// us: 2^10 bodies 98, 81, 77, 72, 69; 2^14 243, 191, 160, 155, 158; 2^16 at
+// ratio 1.3 242, 238, 253, at ratio 2 353, 328, 307, 311, at ratio 4 with
+// quadrupoles 1202, 923, 860, 820, 852; 2^17 at ratio 1.3 289, 307, at ratio 2
+// 440, 403, 411, at ratio 4 with quadrupoles 1767, 1666, 1562, 1550.
 TreeState split_state(nbg_engine* e, bool emit) {
     TreeState a = *e->tree;
     const size_t n = e->count, groups = n / 64;
-    const size_t slots = 20 * (size_t)e->sm_count;
+    const double ratio = std::min(std::max(a.lambda, 1.0), 4.0);  // of the tree
+    const size_t want = (size_t)(10.0 * ratio * e->sm_count), most = groups > 128 ? 8 : 16;
     const int64_t asked = std::min<int64_t>(e->tune_get("bh.parts", 0), 32);
     a.parts = 1;
     if (asked > 0)
         while (2 * a.parts <= asked) a.parts *= 2;
-    else if (2 * groups <= slots)
-        while (a.parts < 16 && a.parts * groups < slots) a.parts *= 2;
+    else
+        while ((size_t)a.parts < most && a.parts * groups < want) a.parts *= 2;
     if (a.parts == 1) return a;
     const size_t sums = (size_t)a.parts * 3 * n * sizeof(double);
     const size_t counts = groups * a.parts * sizeof(unsigned);

@@ -860,10 +860,10 @@ constexpr int kSmallThreads = kSmallWarps * 32;
 constexpr int kSmallB = 2;        // bodies per lane, 32 kSmallB a block
 constexpr int kSmallFold = 16;    // quads a warp sums before the sums are folded
 constexpr long long kSmallMin = 32;  // at least so many quads per CTA
-// Up to this size the small-system kernel: fcompute 21 / 10 us at 1000 bodies
-// (symmetric / small), 25 / 14 at 3000, 25 / 21 at 5003, 35 / 35 at 8000,
-// 97 / 107 at 16000.
-constexpr int kSmallMax = 8192;
+// Up to this size the small-system kernel: fcompute 16 / 5.9 us at 1000 bodies
+// (symmetric / small), 20 / 8.7 at 3000, 20 / 15 at 5003, 30.1 / 29.6 at 8000,
+// 40 / 36 at 9000, 41 / 44 at 10000, 70 / 80 at 14000.
+constexpr int kSmallMax = 9216;
 
 struct SmallArgs {
     const float4* quads;  // 4 bodies: (x x x x) (y y y y) (z z z z) (m m m m)
@@ -1032,8 +1032,8 @@ nbg_status direct_small_launch(nbg_engine* e, const double* y, double* f) {
 
 // Which FP64 kernel: the split path from kSplitMin bodies on, where its five
 // launches and the FP64 share of its pairs cost less than the FP64 pipe's 16
-// operations a pair (1024 bodies: 46 us against 100; 1536: 91 against 84;
-// 2048: 149 against 95).
+// operations a pair (1024 bodies: 37 us against 94; 1280: 60 against 78; 1536:
+// 83 against 72; 2048: 140 against 78).
 constexpr int kSplitMin = 1536;
 
 nbg_status direct_fp64_launch(nbg_engine* e, const double* y, double* f) {
