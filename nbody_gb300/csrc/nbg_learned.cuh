@@ -27,10 +27,12 @@ constexpr int kTcwB2 = kTcwB1 + 64 * 16 / 2;
 constexpr int kTcwB3 = kTcwB2 + 64 * 16 / 2;
 constexpr int kTcwWords = kTcwB3 + 16 * 16 / 2;
 
+constexpr size_t kIoKeep = 1 << 20;  // samples: 80 MiB
+
 struct LearnState {
     // model
     float* w = nullptr;      // FP32 master parameters [kParams]
-    float* grad = nullptr;   // [kParams]
+    float* grad = nullptr;   // [kParams], behind loss in one block
     float* m1 = nullptr;     // Adam first moment
     float* m2 = nullptr;     // Adam second moment
     uint2* frag = nullptr;   // fragment-ordered BF16 weights [kFragWords]
@@ -41,6 +43,9 @@ struct LearnState {
     float* grad_part = nullptr;   // [part_blocks][kParams]
     double* loss_part = nullptr;  // [part_blocks]
     int part_blocks = 0;
+    // nbg_learn_loss_grad's samples on the device, kept up to kIoKeep of them
+    float* io = nullptr;
+    size_t io_cap = 0;
     int64_t adam_step = 0;
     bool has_weights = false;
     // training samples
