@@ -256,17 +256,28 @@ ens_force_kernel(const Body2* __restrict__ bodies, const long long* __restrict__
 //     body (l + r) mod 32, and the body's FP32 sum follows it one lane down
 //     per step -- the four warps' sums are added in warp order, and the unit
 //     writes one FP32 partial per (R, B body) to bpart.
-// Tiles before R are covered by the units of their own ranges.  The A sums
-// (two-sum per tile) go straight to the output; ens_sym_reduce_kernel then
-// adds to every body the partials of the ranges before its own, in range
-// order, in FP64 (weight -1, or -m with equal masses).  No atomics: equal
-// states give equal forces.  Per pair of bodies 14 to 16 packed FP32
+// Tiles before R are covered by the units of their own ranges.  A unit's A sums
+// (two-sum per tile) go to apart as hi and lo; ens_sym_reduce_kernel adds every
+// body's segments in order and subtracts the partials of the ranges before its
+// own, in range order.  No atomics: equal states give equal forces.  Per pair of bodies 14 to 16 packed FP32
 // operations and one reciprocal square root serve both bodies, against 11
 // to 12 operations per body and pair in the one-sided kernel.
+// A unit walks at most seg_tiles tiles of its range: 512 systems of 64 to 4096
+// bodies are 2300 ranges of 4 to 32 tiles for 608 CTAs, and one unit per range
+// left a tenth of the SM cycles without work (998 us a stage, 904 now); of few
+// systems the largest range alone set the time (two steps of 16 systems 3.34
+// ms, 0.66 now; of 100 9.1 and 3.3 ms).
 struct EnsSymUnit {
     int sys;
-    int r;  // A range
+    int r;       // A range
+    int t0, t1;  // tiles
+    int seg;     // which of the range's segments this is
 };
+
+// Segments of range r of a system of `tiles` tiles (tpr per range).
+__host__ __device__ __forceinline__ int ens_segments(int tiles, int tpr, int r, int seg_tiles) {
+    return (tiles - r * tpr + seg_tiles - 1) / seg_tiles;
+}
 
 // at least 4 CTAs per SM: a 128-register budget, which the 4-body (G = 2)
 // equal-mass build needs to run without spills
@@ -274,9 +285,9 @@ template <bool CLAMP, int G, bool UNI>
 __global__ void __launch_bounds__(kEnsThreads, 4)
 ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ off,
                const int* __restrict__ cnt, const EnsSymUnit* __restrict__ units, int nunits,
-               unsigned* __restrict__ counter, double* __restrict__ acc, size_t B, float eps2v,
-               const double* __restrict__ sys_mass, float* __restrict__ bpart,
-               const long long* __restrict__ boff, size_t bstride) {
+               unsigned* __restrict__ counter, float eps2v, float* __restrict__ bpart,
+               const long long* __restrict__ boff, size_t bstride, float2* __restrict__ apart,
+               const long long* __restrict__ aoff, size_t astride) {
     constexpr int RA = kEnsThreads * 2 * G;
     constexpr int TPR = RA / kEnsTile;
     __shared__ __align__(16) float4 txy[kEnsTile];  // (x x y y) per body
@@ -301,7 +312,6 @@ ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ o
         const long long o = off[un.sys];
         const int n = cnt[un.sys];
         const int a0 = un.r * RA;
-        const int tiles = (n + kEnsTile - 1) / kEnsTile;
         f2_t xi[G], yi[G], zi[G], mi[G], hx[G], hy[G], hz[G], lx[G], ly[G], lz[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -324,7 +334,7 @@ ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ o
             mi[g] = f2_pack(q0.z, q1.z);
             hx[g] = hy[g] = hz[g] = lx[g] = ly[g] = lz[g] = zero;
         }
-        for (int t = un.r * TPR; t < tiles; ++t) {
+        for (int t = un.t0; t < un.t1; ++t) {
             __syncthreads();  // the previous tile's readers are done
             const int j = t * kEnsTile + threadIdx.x;
             if (j < n) {
@@ -420,7 +430,7 @@ ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ o
                 f2_two_sum(hz[g], lz[g], az[g]);
             }
         }
-        const double w = UNI ? sys_mass[un.sys] : 1.0;
+        const size_t at = (size_t)aoff[un.sys] + (size_t)un.seg * n;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const int l0 = a0 + (2 * g) * kEnsThreads + threadIdx.x;
@@ -432,46 +442,62 @@ ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ o
                 float h0, h1, q0, q1;
                 f2_unpack(hh[c], h0, h1);
                 f2_unpack(ll[c], q0, q1);
-                if (l0 < n) acc[c * B + o + l0] = w * ((double)h0 + (double)q0);
-                if (l1 < n) acc[c * B + o + l1] = w * ((double)h1 + (double)q1);
+                if (l0 < n) apart[c * astride + at + l0] = make_float2(h0, q0);
+                if (l1 < n) apart[c * astride + at + l1] = make_float2(h1, q1);
             }
         }
     }
 }
 
-// Adds to every body the B partials of the ranges before its own, in range
-// order, in FP64: acc += w sum_r bpart[r], w = -1 (or -m with equal masses).
+// acc = w (sum of the body's A segments - sum of the B partials of the ranges
+// before its own), w = 1 (or m with equal masses), each in order.  The sums are
+// two-word FP32, converted once: one by one on the FP64 pipe (16 cycles a warp
+// instruction) they took 54 us for 1.06 M bodies without the segments (39 us).
 __global__ void ens_sym_reduce_kernel(const int* __restrict__ sys, const long long* __restrict__ off,
                                       const int* __restrict__ cnt,
                                       const float* __restrict__ bpart,
                                       const long long* __restrict__ boff, size_t bstride,
+                                      const float2* __restrict__ apart,
+                                      const long long* __restrict__ aoff, size_t astride,
                                       double* __restrict__ acc, size_t B,
-                                      const double* __restrict__ sys_mass, int uni, int ra) {
+                                      const double* __restrict__ sys_mass, int uni, int ra,
+                                      int seg_tiles) {
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < B;
          j += (size_t)gridDim.x * blockDim.x) {
         const int s = sys[j];
         const int l = (int)((long long)j - off[s]);
         const int rj = l / ra;
-        if (rj == 0) continue;
         const int n = cnt[s];
-        const double w = uni ? -sys_mass[s] : -1.0;
-        const size_t base = (size_t)boff[s] + (size_t)l;
+        const int segs = ens_segments((n + kEnsTile - 1) / kEnsTile, ra / kEnsTile, rj, seg_tiles);
+        const float* bp = bpart + (size_t)boff[s] + (size_t)l;
+        const float2* ap = apart + (size_t)aoff[s] + (size_t)l;
+        const double w = uni ? sys_mass[s] : 1.0;
+        float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
+        auto add = [&](int c, float p, float p_lo) {
+            const float t = hi[c] + p, b = t - hi[c];
+            lo[c] += ((hi[c] - (t - b)) + (p - b)) + p_lo;
+            hi[c] = t;
+        };
 #pragma unroll
-        for (int comp = 0; comp < 3; ++comp) {
-            double sum = 0.0;
-            for (int r = 0; r < rj; ++r) sum += (double)bpart[comp * bstride + base + (size_t)r * n];
-            acc[comp * B + j] += w * sum;
+        for (int c = 0; c < 3; ++c) {
+            const float2 p = ap[c * astride];
+            hi[c] = p.x;
+            lo[c] = p.y;
         }
+        for (int k = 1; k < segs; ++k)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float2 p = ap[c * astride + (size_t)k * n];
+                add(c, p.x, p.y);
+            }
+        for (int r = 0; r < rj; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) add(c, -bp[c * bstride + (size_t)r * n], 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c * B + j] = w * ((double)hi[c] + (double)lo[c]);
     }
 }
 
-// Candidate update y_new = y + dt sum b2_i k_i and per-system error
-// max |dt sum (b2_i - b1_i) k_i| (as ordered bits, atomicMax).
-// A warp covers 32 consecutive bodies, which belong to one system or a few
-// neighbouring ones (bodies are stored system by system): a segmented max
-// over the warp leaves each system's maximum in its first lane, and only
-// those lanes reach the system's error word (max is order-free, so the
-// result does not depend on the schedule).
 __global__ void ens_error_kernel(const double* __restrict__ y, const int* __restrict__ sys,
                                  const double* __restrict__ dt, KPtrs kp, size_t B,
                                  double* __restrict__ ynew, unsigned long long* __restrict__ err) {
@@ -601,6 +627,11 @@ struct nbg_ensemble {
     float* bpart = nullptr;
     size_t bstride = 0, bpart_cap = 0;
     long long* boff = nullptr;
+    // the A partials (3 components x astride; system s from aoff[s], segments x N_s)
+    float2* apart = nullptr;
+    size_t astride = 0, apart_cap = 0;
+    long long* aoff = nullptr;
+    int seg_tiles = 1;
 };
 
 namespace {
@@ -634,8 +665,11 @@ EnsForce ens_pick(const nbg_ensemble* s) {
 }
 
 using EnsSym = void (*)(const Body2*, const long long*, const int*, const EnsSymUnit*, int,
-                        unsigned*, double*, size_t, float, const double*, float*,
+                        unsigned*, float, float*, const long long*, size_t, float2*,
                         const long long*, size_t);
+
+constexpr size_t kEnsUnitsPerSlot = 8;  // (4 to 16 measured the same)
+constexpr size_t kEnsMaxSegBytes = size_t(1) << 30;
 
 template <bool UNI>
 EnsSym ens_pick_sym_g(bool clamp, int G) {
@@ -657,6 +691,31 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
         EnsSymUnit u;
         double cost;
     };
+    int occ = 0;
+    NBG_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_pick_sym(s), kEnsThreads, 0));
+    occ = std::max(occ, 1);
+    const int64_t bps = e->tune_get("ensemble.blocks_per_sm", 0);
+    if (bps > 0 && bps < occ) occ = (int)bps;
+    // tiles per unit: about kEnsUnitsPerSlot units for each resident CTA, and
+    // A partials of at most kEnsMaxSegBytes
+    const int tpr = ra / kEnsTile;
+    auto tiles_of = [](int n) { return (n + kEnsTile - 1) / kEnsTile; };
+    size_t tiles = 0;
+    for (int n : s->h_cnt)
+        for (int t = tiles_of(n); t > 0; t -= tpr) tiles += (size_t)t;
+    const size_t slots = (size_t)e->sm_count * occ * kEnsUnitsPerSlot;
+    s->seg_tiles = (int)std::max<size_t>(1, (tiles + slots - 1) / slots);
+    std::vector<long long> aoff(s->nsys);
+    long long atotal = 0;
+    while (true) {
+        atotal = 0;
+        for (int sI = 0; sI < s->nsys; ++sI) {
+            aoff[sI] = atotal;
+            atotal += (long long)ens_segments(tiles_of(s->h_cnt[sI]), tpr, 0, s->seg_tiles) * s->h_cnt[sI];
+        }
+        if (3 * (size_t)atotal * sizeof(float2) <= kEnsMaxSegBytes || s->seg_tiles > (1 << 24)) break;
+        s->seg_tiles *= 2;
+    }
     std::vector<Costed> units;
     std::vector<long long> boff(s->nsys);
     long long total = 0;
@@ -666,9 +725,14 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
         boff[sI] = total;
         total += (long long)ranges * n;
         for (int r = 0; r < ranges; ++r) {
-            const double own = (double)ra * std::min(ra, n - r * ra);
-            const double later = (double)ra * std::max(0, n - (r + 1) * ra);
-            units.push_back({EnsSymUnit{sI, r}, own + 0.6 * later});
+            const int segs = ens_segments(tiles_of(n), tpr, r, s->seg_tiles);
+            for (int k = 0; k < segs; ++k) {
+                const int t0 = r * tpr + k * s->seg_tiles;
+                const int t1 = std::min(t0 + s->seg_tiles, tiles_of(n));
+                // one-sided (own) and symmetric tiles
+                const int own = std::max(0, std::min(t1, (r + 1) * tpr) - t0);
+                units.push_back({EnsSymUnit{sI, r, t0, t1, k}, own + 1.2 * (t1 - t0 - own)});
+            }
         }
     }
     std::stable_sort(units.begin(), units.end(),
@@ -694,11 +758,19 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
         NBG_CUDA(e, cudaMalloc(&s->bpart, 3 * s->bstride * sizeof(float)));
         s->bpart_cap = 3 * s->bstride;
     }
-    int occ = 0;
-    NBG_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_pick_sym(s), kEnsThreads, 0));
-    occ = std::max(occ, 1);
-    const int64_t bps = e->tune_get("ensemble.blocks_per_sm", 0);
-    if (bps > 0 && bps < occ) occ = (int)bps;
+    cudaFree(s->aoff);
+    s->aoff = nullptr;
+    NBG_CUDA(e, cudaMalloc(&s->aoff, aoff.size() * sizeof(long long)));
+    NBG_CUDA(e, cudaMemcpy(s->aoff, aoff.data(), aoff.size() * sizeof(long long),
+                           cudaMemcpyHostToDevice));
+    s->astride = (size_t)std::max<long long>(atotal, 1);
+    if (s->apart_cap < 3 * s->astride) {
+        cudaFree(s->apart);
+        s->apart = nullptr;
+        s->apart_cap = 0;
+        NBG_CUDA(e, cudaMalloc(&s->apart, 3 * s->astride * sizeof(float2)));
+        s->apart_cap = 3 * s->astride;
+    }
     s->force_grid = (unsigned)std::max(1, std::min(s->nsym_units, e->sm_count * occ));
     return NBG_OK;
 }
@@ -772,13 +844,14 @@ nbg_status ens_launch_force(nbg_ensemble* s, unsigned* counter, double* acc) {
     const float eps2 = (float)(s->p.softening * s->p.softening);
     if (s->sym) {
         ens_pick_sym(s)<<<s->force_grid, kEnsThreads, 0, e->stream>>>(
-            s->bodies, s->off, s->cnt, s->sym_units, s->nsym_units, counter, acc, s->B, eps2,
-            s->sys_mass, s->bpart, s->boff, s->bstride);
+            s->bodies, s->off, s->cnt, s->sym_units, s->nsym_units, counter, eps2, s->bpart,
+            s->boff, s->bstride, s->apart, s->aoff, s->astride);
         NBG_LAUNCHED(e, "ens_sym_kernel");
         ens_sym_reduce_kernel<<<grid_for(s->B, 256, (unsigned)e->sm_count * 8u), 256, 0,
                                 e->stream>>>(s->sys, s->off, s->cnt, s->bpart, s->boff,
-                                             s->bstride, acc, s->B, s->sys_mass,
-                                             ens_uniform(s) ? 1 : 0, kEnsThreads * 2 * s->G);
+                                             s->bstride, s->apart, s->aoff, s->astride, acc,
+                                             s->B, s->sys_mass, ens_uniform(s) ? 1 : 0,
+                                             kEnsThreads * 2 * s->G, s->seg_tiles);
         NBG_LAUNCHED(e, "ens_sym_reduce_kernel");
         return NBG_OK;
     }
@@ -831,11 +904,14 @@ nbg_status ens_enqueue_step(nbg_ensemble* s) {
 void ens_free(nbg_ensemble* s) {
     void* ptrs[] = {s->off, s->cnt, s->sys, s->y, s->ynew, s->mass, s->sys_mass, s->bodies, s->dt, s->t,
                     s->err, s->accepted, s->rejected, s->decision, s->err_prev, s->units,
-                    s->counters, s->sym_units, s->bpart, s->boff};
+                    s->counters, s->sym_units, s->bpart, s->boff, s->apart, s->aoff};
     for (void* p : ptrs) cudaFree(p);
     s->sym_units = nullptr;
     s->bpart = nullptr;
     s->boff = nullptr;
+    s->apart = nullptr;
+    s->aoff = nullptr;
+    s->apart_cap = 0;
     s->bpart_cap = 0;
     for (double* k : s->k) cudaFree(k);
     if (s->graph) cudaGraphExecDestroy(s->graph);
