@@ -46,10 +46,13 @@ __constant__ double c_a[kStagesRK][kStagesRK] = {
     {19372.0 / 6561, -25360.0 / 2187, 64448.0 / 6561, -212.0 / 729, 0, 0, 0},
     {9017.0 / 3168, -355.0 / 33, 46732.0 / 5247, 49.0 / 176, -5103.0 / 18656, 0, 0},
     {35.0 / 384, 0, 500.0 / 1113, 125.0 / 192, -2187.0 / 6784, 11.0 / 84, 0}};
-__constant__ double c_b1[kStagesRK] = {35.0 / 384, 0, 500.0 / 1113, 125.0 / 192,
-                                       -2187.0 / 6784, 11.0 / 84, 0};
 __constant__ double c_b2[kStagesRK] = {5179.0 / 57600, 0, 7571.0 / 16695, 393.0 / 640,
                                        -92097.0 / 339200, 187.0 / 2100, 1.0 / 40};
+
+__constant__ double c_e[kStagesRK] = {
+    5179.0 / 57600 - 35.0 / 384,         0, 7571.0 / 16695 - 500.0 / 1113,
+    393.0 / 640 - 125.0 / 192,           -92097.0 / 339200 - -2187.0 / 6784,
+    187.0 / 2100 - 11.0 / 84,            1.0 / 40};  // c_b2 less the 5th order's weights
 
 struct Body2 {
     float4 xxyy;
@@ -71,6 +74,7 @@ __global__ void ens_stage_kernel(int stage, const double* __restrict__ y,
                                  const double* __restrict__ mass, const int* __restrict__ sys,
                                  const double* __restrict__ dt, KPtrs kp, size_t B,
                                  Body2* __restrict__ out) {
+    if (!after_previous()) return;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < B;
          i += (size_t)gridDim.x * blockDim.x) {
         const double h = dt[sys[i]];
@@ -151,6 +155,7 @@ ens_force_kernel(const Body2* __restrict__ bodies, const long long* __restrict__
                  const int* __restrict__ cnt, const EnsUnit* __restrict__ units, int nunits,
                  unsigned* __restrict__ counter, double* __restrict__ acc, size_t B, float eps2v,
                  const double* __restrict__ sys_mass) {
+    if (!after_previous()) return;
     __shared__ __align__(16) Body2 tile[kEnsTile];
     __shared__ int next_unit;
     const f2_t eps2 = f2_pack(eps2v, eps2v);
@@ -288,6 +293,7 @@ ens_sym_kernel(const Body2* __restrict__ bodies, const long long* __restrict__ o
                unsigned* __restrict__ counter, float eps2v, float* __restrict__ bpart,
                const long long* __restrict__ boff, size_t bstride, float2* __restrict__ apart,
                const long long* __restrict__ aoff, size_t astride) {
+    if (!after_previous()) return;
     constexpr int RA = kEnsThreads * 2 * G;
     constexpr int TPR = RA / kEnsTile;
     __shared__ __align__(16) float4 txy[kEnsTile];  // (x x y y) per body
@@ -462,6 +468,7 @@ __global__ void ens_sym_reduce_kernel(const int* __restrict__ sys, const long lo
                                       double* __restrict__ acc, size_t B,
                                       const double* __restrict__ sys_mass, int uni, int ra,
                                       int seg_tiles) {
+    if (!after_previous()) return;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < B;
          j += (size_t)gridDim.x * blockDim.x) {
         const int s = sys[j];
@@ -498,9 +505,17 @@ __global__ void ens_sym_reduce_kernel(const int* __restrict__ sys, const long lo
     }
 }
 
+// The larger of m and |v|'s bits, which order as the numbers do; NaN is skipped,
+// as fmax does.
+__device__ __forceinline__ long long larger(long long m, double v) {
+    const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+    return b > m && b <= 0x7ff0000000000000LL ? b : m;
+}
+
 __global__ void ens_error_kernel(const double* __restrict__ y, const int* __restrict__ sys,
                                  const double* __restrict__ dt, KPtrs kp, size_t B,
                                  double* __restrict__ ynew, unsigned long long* __restrict__ err) {
+    if (!after_previous()) return;
     const int lane = threadIdx.x & 31;
     const size_t warp0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) & ~(size_t)31;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -508,7 +523,7 @@ __global__ void ens_error_kernel(const double* __restrict__ y, const int* __rest
         const size_t i = base + lane;
         const bool live = i < B;
         const int s = live ? sys[i] : -1;
-        double emax = 0.0;
+        long long emax = 0;  // |error|'s bits
         if (live) {
             const double h = dt[s];
 #pragma unroll
@@ -516,24 +531,25 @@ __global__ void ens_error_kernel(const double* __restrict__ y, const int* __rest
                 double acc_b2 = 0.0, acc_e = 0.0;
 #pragma unroll
                 for (int j = 0; j < kStagesRK; ++j) {
+                    if (j == 1) continue;  // weight 0 in both
                     const double kv = kp.k[j][c * B + i];
                     acc_b2 = fma(c_b2[j], kv, acc_b2);
-                    acc_e = fma(c_b2[j] - c_b1[j], kv, acc_e);
+                    acc_e = fma(c_e[j], kv, acc_e);
                 }
                 ynew[c * B + i] = fma(h, acc_b2, y[c * B + i]);
-                emax = fmax(emax, fabs(h * acc_e));
+                emax = larger(emax, h * acc_e);
             }
         }
         // segmented suffix max: lanes of one system are contiguous
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const double w = __shfl_down_sync(0xffffffffu, emax, o);
+            const long long w = __shfl_down_sync(0xffffffffu, emax, o);
             const int sw = __shfl_down_sync(0xffffffffu, s, o);
-            if (lane + o < 32 && sw == s) emax = fmax(emax, w);
+            if (lane + o < 32 && sw == s && w > emax) emax = w;
         }
         const int sp = __shfl_up_sync(0xffffffffu, s, 1);
         if (live && (lane == 0 || sp != s))
-            atomicMax(&err[s], (unsigned long long)__double_as_longlong(emax));
+            atomicMax(&err[s], (unsigned long long)emax);
     }
 }
 
@@ -545,6 +561,7 @@ __global__ void ens_control_kernel(int nsys, double tol, double dt_min, double d
                                    double* __restrict__ t, unsigned* __restrict__ accepted,
                                    unsigned* __restrict__ rejected, int* __restrict__ decision,
                                    int hold, double* __restrict__ err_prev, int pi) {
+    if (!after_previous()) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nsys) return;
     const double e = __longlong_as_double((long long)err[s]);
@@ -575,12 +592,23 @@ __global__ void ens_control_kernel(int nsys, double tol, double dt_min, double d
 __global__ void ens_commit_kernel(double* __restrict__ y, const double* __restrict__ ynew,
                                   const int* __restrict__ sys, const int* __restrict__ decision,
                                   size_t B) {
+    if (!after_previous()) return;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < B;
          i += (size_t)gridDim.x * blockDim.x) {
         if (!decision[sys[i]]) continue;
 #pragma unroll
         for (int c = 0; c < 6; ++c) y[c * B + i] = ynew[c * B + i];
     }
+}
+
+// The state [6][B] as the caller's arrays [2][B][3]: taken apart by the host
+// it took 6.5 ms for 1.06 M bodies, copies of 51 MB included (1.35 ms).
+__global__ void ens_state_kernel(const double* __restrict__ y, size_t B, double* __restrict__ out) {
+    if (!after_previous()) return;
+    const size_t half = 3 * B, from = blockIdx.y * half;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < half;
+         i += (size_t)gridDim.x * blockDim.x)
+        out[from + i] = y[from + (i % 3) * B + i / 3];
 }
 
 }  // namespace
@@ -843,19 +871,19 @@ nbg_status ens_launch_force(nbg_ensemble* s, unsigned* counter, double* acc) {
     nbg_engine* e = s->eng;
     const float eps2 = (float)(s->p.softening * s->p.softening);
     if (s->sym) {
-        ens_pick_sym(s)<<<s->force_grid, kEnsThreads, 0, e->stream>>>(
+        queued(ens_pick_sym(s), s->force_grid, kEnsThreads, 0, e->stream)(
             s->bodies, s->off, s->cnt, s->sym_units, s->nsym_units, counter, eps2, s->bpart,
             s->boff, s->bstride, s->apart, s->aoff, s->astride);
         NBG_LAUNCHED(e, "ens_sym_kernel");
-        ens_sym_reduce_kernel<<<grid_for(s->B, 256, (unsigned)e->sm_count * 8u), 256, 0,
-                                e->stream>>>(s->sys, s->off, s->cnt, s->bpart, s->boff,
+        queued(ens_sym_reduce_kernel, grid_for(s->B, 256, (unsigned)e->sm_count * 8u), 256, 0,
+                                e->stream)(s->sys, s->off, s->cnt, s->bpart, s->boff,
                                              s->bstride, s->apart, s->aoff, s->astride, acc,
                                              s->B, s->sys_mass, ens_uniform(s) ? 1 : 0,
                                              kEnsThreads * 2 * s->G, s->seg_tiles);
         NBG_LAUNCHED(e, "ens_sym_reduce_kernel");
         return NBG_OK;
     }
-    ens_pick(s)<<<s->force_grid, kEnsThreads, 0, e->stream>>>(
+    queued(ens_pick(s), s->force_grid, kEnsThreads, 0, e->stream)(
         s->bodies, s->off, s->cnt, s->units, s->nunits, counter, acc, s->B, eps2, s->sys_mass);
     NBG_LAUNCHED(e, "ens_force_kernel");
     return NBG_OK;
@@ -868,7 +896,7 @@ nbg_status ens_enqueue_force(nbg_ensemble* s) {
     for (int i = 0; i < kStagesRK; ++i) kp.k[i] = s->k[i];
     const unsigned gv = grid_for(s->B, 256, (unsigned)e->sm_count * 8u);
     NBG_CUDA(e, cudaMemsetAsync(s->counters, 0, sizeof(unsigned), e->stream));
-    ens_stage_kernel<<<gv, 256, 0, e->stream>>>(0, s->y, s->mass, s->sys, s->dt, kp, s->B,
+    queued(ens_stage_kernel, gv, 256, 0, e->stream)(0, s->y, s->mass, s->sys, s->dt, kp, s->B,
                                                 s->bodies);
     NBG_LAUNCHED(e, "ens_stage_kernel");
     return ens_launch_force(s, s->counters, s->k[0] + 3 * s->B);
@@ -882,21 +910,21 @@ nbg_status ens_enqueue_step(nbg_ensemble* s) {
     NBG_CUDA(e, cudaMemsetAsync(s->counters, 0, kStagesRK * sizeof(unsigned), e->stream));
     NBG_CUDA(e, cudaMemsetAsync(s->err, 0, s->nsys * sizeof(unsigned long long), e->stream));
     for (int st = 0; st < kStagesRK; ++st) {
-        ens_stage_kernel<<<gv, 256, 0, e->stream>>>(st, s->y, s->mass, s->sys, s->dt, kp, s->B,
+        queued(ens_stage_kernel, gv, 256, 0, e->stream)(st, s->y, s->mass, s->sys, s->dt, kp, s->B,
                                                     s->bodies);
         NBG_LAUNCHED(e, "ens_stage_kernel");
         ProfScope ps(e, NBG_K_DIRECT);
         nbg_status fs = ens_launch_force(s, s->counters + st, s->k[st] + 3 * s->B);
         if (fs != NBG_OK) return fs;
     }
-    ens_error_kernel<<<gv, 256, 0, e->stream>>>(s->y, s->sys, s->dt, kp, s->B, s->ynew, s->err);
+    queued(ens_error_kernel, gv, 256, 0, e->stream)(s->y, s->sys, s->dt, kp, s->B, s->ynew, s->err);
     NBG_LAUNCHED(e, "ens_error_kernel");
-    ens_control_kernel<<<(s->nsys + 127) / 128, 128, 0, e->stream>>>(
+    queued(ens_control_kernel, (s->nsys + 127) / 128, 128, 0, e->stream)(
         s->nsys, s->p.tolerance, s->p.dt_min, s->p.dt_max, s->err, s->dt, s->t, s->accepted,
         s->rejected, s->decision, (int)e->tune_get("ensemble.hold_after_reject", 1), s->err_prev,
         (int)e->tune_get("ensemble.pi_control", 0));
     NBG_LAUNCHED(e, "ens_control_kernel");
-    ens_commit_kernel<<<gv, 256, 0, e->stream>>>(s->y, s->ynew, s->sys, s->decision, s->B);
+    queued(ens_commit_kernel, gv, 256, 0, e->stream)(s->y, s->ynew, s->sys, s->decision, s->B);
     NBG_LAUNCHED(e, "ens_commit_kernel");
     return NBG_OK;
 }
@@ -1121,14 +1149,21 @@ nbg_status nbg_ensemble_status(nbg_ensemble* s, double* t, double* dt, uint32_t*
 nbg_status nbg_ensemble_get_state(nbg_ensemble* s, double* vertices, double* velocities) {
     if (s == nullptr || vertices == nullptr || velocities == nullptr) return NBG_ERR_INVALID_ARG;
     nbg_engine* e = s->eng;
-    std::vector<double> h(6 * s->B);
+    if (s->B == 0) return NBG_OK;
+    // (ynew is free between steps)
+    const size_t half = 3 * s->B;
+    queued(ens_state_kernel, dim3(grid_for(half, 256, (unsigned)e->sm_count * 8u), 2), 256, 0,
+           e->stream)(s->y, s->B, s->ynew);
+    NBG_LAUNCHED(e, "ens_state_kernel");
+    // pages that were never written are slow to copy to (45 ms for 51 MB): the
+    // host has them mapped while the kernel runs
+    for (double* to : {vertices, velocities})
+        for (size_t i = 0; i < half; i += 4096 / sizeof(double)) static_cast<volatile double*>(to)[i] = 0.0;
+    NBG_CUDA(e, cudaMemcpyAsync(vertices, s->ynew, half * sizeof(double), cudaMemcpyDeviceToHost,
+                                e->stream));
+    NBG_CUDA(e, cudaMemcpyAsync(velocities, s->ynew + half, half * sizeof(double),
+                                cudaMemcpyDeviceToHost, e->stream));
     NBG_CUDA(e, cudaStreamSynchronize(e->stream));
-    NBG_CUDA(e, cudaMemcpy(h.data(), s->y, 6 * s->B * sizeof(double), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < s->B; ++i)
-        for (int d = 0; d < 3; ++d) {
-            vertices[3 * i + d] = h[d * s->B + i];
-            velocities[3 * i + d] = h[(3 + d) * s->B + i];
-        }
     return NBG_OK;
 }
 
