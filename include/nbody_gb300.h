@@ -280,7 +280,7 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  * Keys: "direct.symmetric" (1: each unordered pair evaluated once and
  *       applied to both bodies, the default; 0: one-sided kernel),
  *       "direct.small" (with "direct.symmetric" 1: 1 the kernel for small
- *       systems, which evaluates ordered pairs, the default up to 9216 bodies
+ *       systems, which evaluates ordered pairs, the default up to 5120 bodies
  *       unless "direct.sym_g" is set; 0 the symmetric kernel),
  *       "direct.sym_g" (4 or 3: packed A-body pairs per lane of the
  *       symmetric kernel; 3 runs 5 CTAs per SM),

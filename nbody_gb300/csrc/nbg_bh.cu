@@ -641,6 +641,7 @@ __device__ __forceinline__ void group_pair_lo(f2_t xj, f2_t yj, f2_t zj, f2_t mj
 // samples; with some of them unknown an upper bound of it, ~0 while half are.
 // All lanes of a warp call it and get it.
 __device__ __forceinline__ unsigned long long walk_cap(const TreeState& t) {
+    if (t.cap_samples == 0) return t.test_cap;
     const WalkCtl* ctl = reinterpret_cast<const WalkCtl*>(t.fb_count);
     const int lane = threadIdx.x & 31;
     const unsigned f = lane < t.cap_samples ? *(volatile const unsigned*)&ctl->finished[lane] : 0u;
@@ -653,6 +654,24 @@ __device__ __forceinline__ unsigned long long walk_cap(const TreeState& t) {
     const unsigned at = __ballot_sync(0xffffffffu, rank == t.cap_samples / 2);
     const unsigned m = __shfl_sync(0xffffffffu, v, __ffs(at) - 1);
     return m == ~0u ? ~0ull : max((unsigned long long)t.cap_ratio * m, 4096ull);
+}
+
+// A part of a sampled group is done.  The last one knows the group's total;
+// once more than half of the samples have one, the cap has an upper bound.
+__device__ __noinline__ void walk_sample_done(const TreeState& t, int gw) {
+    WalkCtl* ctl = reinterpret_cast<WalkCtl*>(t.fb_count);
+    const int s = gw / t.cap_stride, lane = threadIdx.x & 31;
+    unsigned d = 0;
+    __threadfence();
+    if (lane == 0) d = atomicAdd(&ctl->done[s], 1u);
+    d = __shfl_sync(0xffffffffu, d, 0);
+    if (d != (unsigned)t.parts - 1u) return;
+    __threadfence();
+    if (lane == 0) atomicExch(&ctl->finished[s], atomicAdd(&ctl->group[gw], 0u) + 1u);
+    __threadfence();
+    __syncwarp();
+    const unsigned long long u = walk_cap(t);
+    if (lane == 0 && u != ~0ull) atomicMax(&ctl->bound, ~u);
 }
 
 // a group's counts: 64 bits, 32 where a group's fit (nodes of one tree)
@@ -766,8 +785,9 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
     __syncwarp();
     int sp = 1, lc = 0, peak = 1, ec = 0;
     bool overflow = false, abandoned = false;
-    const unsigned long long test_cap = t.test_cap != 0 ? t.test_cap : t.cap_state[0];
+    const unsigned long long test_cap = SPLIT || t.test_cap != 0 ? t.test_cap : t.cap_state[0];
     WalkCtl* ctl = reinterpret_cast<WalkCtl*>(t.fb_count);
+    const bool capped = SPLIT && test_cap != ~0ull;
     unsigned sent = 0;  // SPLIT: tests already added to the group's
 
     auto evaluate = [&]() {
@@ -921,19 +941,22 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
             }
         }
         const bool full = lc > kGWList - 32 * NPL, qfull = ORDER == 2 && qc > kGWQList - 32 * NPL;
-        // SPLIT: at each evaluation (which hides the atomic) the group's node
-        // tests so far, over all its parts, are compared with the cap
+        // SPLIT: at each evaluation (which hides the loads) the group's node
+        // tests so far, over all its parts, are compared with the cap, or its
+        // upper bound while the samples are walked
+        unsigned long long bound = ~0ull;
         unsigned seen = 0;
-        if (SPLIT && (full || qfull)) {
+        if (SPLIT && capped && (full || qfull)) {
+            bound = test_cap != 0 ? test_cap : ~*(volatile unsigned long long*)&ctl->bound;
             if (lane == 0) seen = atomicAdd(&ctl->group[gw], (unsigned)tests - sent);
             __syncwarp();  // else lane 0 evaluates the list by itself: 505 -> 832 us at 2^18 bodies
         }
         if (full) evaluate();  // room for this step's entries
         if (qfull) evaluate_quad();
-        if (SPLIT && (full || qfull)) {
+        if (SPLIT && capped && (full || qfull)) {
             seen = __shfl_sync(0xffffffffu, seen, 0) + (unsigned)tests - sent;
             sent = (unsigned)tests;
-            if ((unsigned long long)seen + 1 > test_cap) {
+            if ((unsigned long long)seen + 1 > bound) {
                 abandoned = true;
                 break;
             }
@@ -981,9 +1004,21 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
                 nb += __popc(bm[w]);
             }
             if (ec + nb > t.cand_cap) {  // walked body by body instead
-                abandoned = true;
-                if (SPLIT && lane == 0) t.cand_part_n[gw * t.parts + part] = (unsigned)t.cand_cap + 1u;
-                break;
+                // (a sample goes on without its cells: its tests set the cap)
+                if (SPLIT && t.cap_samples > 0 && gw % t.cap_stride == 0) {
+                    ec = t.cand_cap + 1;
+                    nb = 0;
+#pragma unroll
+                    for (int w = 0; w < NPL; ++w) {
+                        bm[w] = 0;
+                        band[w] = false;
+                    }
+                } else {
+                    abandoned = true;
+                    if (SPLIT && lane == 0)
+                        t.cand_part_n[gw * t.parts + part] = (unsigned)t.cand_cap + 1u;
+                    break;
+                }
             }
             int* cells = SPLIT ? t.cand_part + ((size_t)gw * t.parts + part) * t.cand_cap
                                : t.cand + (size_t)gw * t.cand_cap;
@@ -1062,8 +1097,8 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
     }
     if (!SPLIT) tests -= 1;  // child 0 of the first step
     if (lane == 0) {
-        if (SPLIT) atomicAdd(&ctl->group[gw], (unsigned)tests - sent);
-        else atomicAdd(&t.counters[0], (unsigned long long)tests);
+        if (!SPLIT) atomicAdd(&t.counters[0], (unsigned long long)tests);
+        else atomicAdd(&ctl->group[gw], (unsigned)tests - sent);
         atomicMax(&t.counters[2], (unsigned long long)peak);
         if (EMIT && !SPLIT) t.cand_n[gw] = abandoned ? 0u : (unsigned)ec;
     }
@@ -1081,6 +1116,8 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
             atomicAdd(&ctl->group[n / (32 * BPL) + gw], (unsigned)inter);
             if (EMIT) t.cand_part_n[gw * t.parts + part] = (unsigned)ec;
         }
+        if (t.cap_samples > 0 && gw % t.cap_stride == 0)
+            walk_sample_done(t, gw);
         double* out = t.part + (size_t)part * 3 * n + gw * 32 * BPL + lane;
 #pragma unroll
         for (int bb = 0; bb < BPL; ++bb)
@@ -1110,7 +1147,7 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         f2_unpack(slot(6 * bb + 5), l0, l1);
         f[5 * n + b] = ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
     }
-    if (!SPLIT && lane == 0) atomicAdd(&t.counters[1], inter * 32ull * BPL);
+    if (lane == 0) atomicAdd(&t.counters[1], inter * 32ull * BPL);
 }
 
 // Persistent over the groups (n is a power of two >= 32 BPL, so groups are
@@ -1142,10 +1179,13 @@ bh_group_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n
 // nodes above level t.top are tested by every part and summed by one, the
 // subtrees under that level are dealt out (node mod parts).  A system of few
 // groups then fills the GPU: 16384 bodies are 256 groups, and one warp each
-// took 152 us (59 us with 16, and 5 us in bh_walk_finish_kernel).  A part stops once its group's tests exceed the cap;
-// whether the group goes to the per-body walk is decided by
-// bh_walk_finish_kernel from the totals alone, and the parts are added in
-// order, so equal trees give equal forces.
+// took 152 us (59 us with 16, and 5 us in bh_walk_finish_kernel).
+// The groups whose tests set the cap are walked first instead of in a pass
+// before the walk (18 us at 16384 bodies): a group counts its tests in
+// ctl.group and stops when they exceed the cap or its upper bound, and
+// bh_walk_finish_kernel decides from the totals alone which groups go to the
+// per-body walk, so equal trees give equal forces.  (A walk with one warp per
+// group keeps the pass: 2^20 bodies 2060 us a step with it, 2120 without.)
 template <bool CLAMP, int MINB, int ORDER, bool SMACC, int NPL, bool EMIT = false>
 __global__ void __launch_bounds__(kGWThreads, MINB)
 bh_split_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n, float eps2v,
@@ -1156,8 +1196,14 @@ bh_split_walk_kernel(const double* __restrict__ y, double* __restrict__ f, int n
     const int tasks = n / 64 * t.parts;
     int task = blockIdx.x * kGWWarps + (threadIdx.x >> 5);
     while (task < tasks) {
+        const int q = task / t.parts;
+        // the samples (every cap_stride-th group), then the others
+        int gw = q;
+        if (t.cap_samples > 0 && t.cap_stride > 1)
+            gw = q < t.cap_samples ? q * t.cap_stride
+                                   : q - t.cap_samples + (q - t.cap_samples) / (t.cap_stride - 1) + 1;
         group_walk_one<CLAMP, 2, ORDER, 2, SMACC, false, EMIT, NPL, true>(
-            y, f, n, eps2v, t, stack_cap, err, smem_raw, task / t.parts, task % t.parts);
+            y, f, n, eps2v, t, stack_cap, err, smem_raw, gw, task % t.parts);
         int next = 0;
         if (lane == 0) next = (int)atomicAdd(&t.fb_count[1], 1u);
         task = gridDim.x * kGWWarps + __shfl_sync(0xffffffffu, next, 0);
@@ -1171,19 +1217,24 @@ template <bool EMIT>
 __global__ void __launch_bounds__(192)
 bh_walk_finish_kernel(const double* __restrict__ y, double* __restrict__ f, int n, TreeState t) {
     if (!after_previous()) return;
+    __shared__ unsigned long long s_cap;
     const WalkCtl* ctl = reinterpret_cast<const WalkCtl*>(t.fb_count);
     const int gw = blockIdx.x, tid = threadIdx.x;
-    const unsigned long long cap = t.test_cap != 0 ? t.test_cap : t.cap_state[0];
+    if (tid < 32) {
+        const unsigned long long cap = walk_cap(t);
+        if (tid == 0) s_cap = cap;
+    }
+    __syncthreads();
     const unsigned long long tests = ctl->group[gw];
     unsigned cells = 0;
     if (EMIT)
         for (int q = 0; q < t.parts; ++q)
             cells = min(cells + t.cand_part_n[gw * t.parts + q], (unsigned)t.cand_cap + 1u);
-    const bool hand = tests + 1 > cap || (EMIT && cells > (unsigned)t.cand_cap);
+    const bool hand = tests + 1 > s_cap || (EMIT && cells > (unsigned)t.cand_cap);
     if (tid == 0) {
         if (hand) t.fb_list[atomicAdd(t.fb_count, 1u)] = gw;
         if (EMIT) t.cand_n[gw] = hand ? 0u : cells;
-        atomicAdd(&t.counters[0], min(tests, cap));
+        atomicAdd(&t.counters[0], min(tests, s_cap));
         atomicAdd(&t.counters[hand ? 3 : 1], hand ? 1ull : 64ull * ctl->group[gridDim.x + gw]);
     }
     if (hand) return;
@@ -1208,7 +1259,8 @@ bh_walk_finish_kernel(const double* __restrict__ y, double* __restrict__ f, int 
 // groups spread over the leaves (every stride-th), a function of the tree
 // alone, so that equal trees give equal forces.  A CTA per sample runs the
 // group walk's traversal without its force evaluation, its warps sharing the
-// tree as in bh_split_walk_kernel.  Samples that exceed the upper bound of
+// tree as in bh_split_walk_kernel (which finds its cap by itself; this is for
+// a walk with one warp per group).  Samples that exceed the upper bound of
 // the cap which the finished ones give (known once more than half are) are
 // above the median and stop.  It is bound by the longest chain of dependent
 // node loads; all samples as the warps of one CTA took 43 us at 16384 bodies
@@ -1313,7 +1365,7 @@ bh_test_cap_kernel(int n, TreeState t, int stack_cap) {
     if (lane == 0 && u != ~0ull) atomicMax(&ctl->bound, ~u);
     unsigned d = 0;
     __threadfence();
-    if (lane == 0) d = atomicAdd(&ctl->done, 1u);
+    if (lane == 0) d = atomicAdd(&ctl->done[0], 1u);
     if (__shfl_sync(0xffffffffu, d, 0) != gridDim.x - 1) return;
     __threadfence();
     u = walk_cap(t);  // every sample is in: the cap
@@ -1620,24 +1672,24 @@ using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, 
 
 // Warps per group of the default walk, and the state of such a walk with its
 // scratch (the parts' sums and, with emit, their band cells).  By default
-// enough warps for ratio / 2 times the resident ones (20 per SM): a larger
-// ratio means more work per group to set against the second kernel and the top
-// of the tree, which every part walks.  fcompute with 1, 2, 4, 8 and 16 parts,
-// us: 2^10 bodies 98, 81, 77, 72, 69; 2^14 243, 191, 160, 155, 158; 2^16 at
-// ratio 1.3 242, 238, 253, at ratio 2 353, 328, 307, 311, at ratio 4 with
-// quadrupoles 1202, 923, 860, 820, 852; 2^17 at ratio 1.3 289, 307, at ratio 2
-// 440, 403, 411, at ratio 4 with quadrupoles 1767, 1666, 1562, 1550.
+// enough warps for a third of the resident ones (20 per SM).  More shorten a
+// lone walk's tail, but every part walks the top of the tree, which the GPU has
+// no time for when other engines' kernels share it.  An Euler step alone / of
+// three engines side by side, us, with 1, 2, 4, 8 and 16 parts: 2^10 bodies
+// 105/36, 84/30, 79/26, 75/27, 73/26; 2^14 242/84, 180/67, 154/58, 144/56,
+// 148/72; 2^15 300/118, 227/89, 203/82, 191/94, with the learned correction
+// 951/542, 915/525, 898/540; 2^16 361/148, 307/150, 284/165, with quadrupoles
+// at ratio 4 1078/555, 946/605, 848/617.
 TreeState split_state(nbg_engine* e, bool emit) {
     TreeState a = *e->tree;
     const size_t n = e->count, groups = n / 64;
-    const double ratio = std::min(std::max(a.lambda, 1.0), 4.0);  // of the tree
-    const size_t want = (size_t)(10.0 * ratio * e->sm_count), most = groups > 128 ? 8 : 16;
+    const size_t want = 13 * (size_t)e->sm_count / 2;
     const int64_t asked = std::min<int64_t>(e->tune_get("bh.parts", 0), 32);
     a.parts = 1;
     if (asked > 0)
         while (2 * a.parts <= asked) a.parts *= 2;
     else
-        while ((size_t)a.parts < most && a.parts * groups < want) a.parts *= 2;
+        while (a.parts < 16 && a.parts * groups < want) a.parts *= 2;
     if (a.parts == 1) return a;
     const size_t sums = (size_t)a.parts * 3 * n * sizeof(double);
     const size_t counts = groups * a.parts * sizeof(unsigned);
@@ -1802,15 +1854,16 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
         t->test_cap = (unsigned long long)std::max<int64_t>(e->tune_get("bh.test_cap", 0), 0);
         if (t->test_cap == 0 && t->curve == 0) t->test_cap = ~0ull;
         a.test_cap = t->test_cap;
+        const int samples = std::min(warps, kCapSamples);  // both powers of two
+        a.cap_ratio = (unsigned)std::max<int64_t>(e->tune_get("bh.test_cap_ratio", 2), 1);
+        a.cap_samples = t->test_cap == 0 ? samples : 0;
+        a.cap_stride = warps / samples;
         // the walk's counters (and, of a shared walk, its groups')
         NBG_CUDA(e, cudaMemsetAsync(t->fb_count, 0,
                                     sizeof(WalkCtl) + (a.parts > 1 ? 2 * sizeof(unsigned) * (size_t)warps : 0),
                                     e->stream));
-        if (t->test_cap == 0) {
-            TreeState tc = *t;
-            tc.cap_ratio = (unsigned)std::max<int64_t>(e->tune_get("bh.test_cap_ratio", 2), 1);
-            tc.cap_samples = std::min(warps, kCapSamples);  // both powers of two
-            tc.cap_stride = warps / tc.cap_samples;
+        if (t->test_cap == 0 && a.parts == 1) {
+            TreeState tc = a;
             const size_t csmem = (size_t)kCapWarps * stack_cap * sizeof(int);
             auto capk = bpl == 4 ? bh_test_cap_kernel<4>
                         : bpl == 2 ? bh_test_cap_kernel<2> : bh_test_cap_kernel<1>;
@@ -1819,7 +1872,7 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
             // the cap counts acceptance tests: against the step build's
             // records when those decide acceptance
             if (frozen) tc.node4 = t->node4_acc;
-            queued(capk, (unsigned)tc.cap_samples, kCapWarps * 32, csmem, e->stream)(n, tc, stack_cap);
+            queued(capk, (unsigned)samples, kCapWarps * 32, csmem, e->stream)(n, tc, stack_cap);
             NBG_LAUNCHED(e, "bh_test_cap_kernel");
         }
         // "bh.persistent" (default 1): as many CTAs as fit at once; 0: one

@@ -861,9 +861,11 @@ constexpr int kSmallB = 2;        // bodies per lane, 32 kSmallB a block
 constexpr int kSmallFold = 16;    // quads a warp sums before the sums are folded
 constexpr long long kSmallMin = 32;  // at least so many quads per CTA
 // Up to this size the small-system kernel: fcompute 16 / 5.9 us at 1000 bodies
-// (symmetric / small), 20 / 8.7 at 3000, 20 / 15 at 5003, 30.1 / 29.6 at 8000,
-// 40 / 36 at 9000, 41 / 44 at 10000, 70 / 80 at 14000.
-constexpr int kSmallMax = 9216;
+// (symmetric / small), 20 / 8.7 at 3000, 20 / 15 at 5003.  Alone it is the
+// faster one up to 9000 bodies (30.1 / 29.6 us at 8000), but it does twice the
+// symmetric kernel's pairs, and three engines side by side take 54 / 55 us an
+// RK4 step of 5003 bodies and 79 / 113 at 8000.
+constexpr int kSmallMax = 5120;
 
 struct SmallArgs {
     const float4* quads;  // 4 bodies: (x x x x) (y y y y) (z z z z) (m m m m)

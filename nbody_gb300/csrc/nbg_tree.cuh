@@ -88,7 +88,8 @@ struct TreeState {
     // group walks that exceed a node-test cap give up; their group ids go
     // to fb_list and a per-body walk computes those bodies (nbg_bh.cu).
     // The cap is test_cap when that is set, else cap_state[0], set from the
-    // test counts of sampled groups by bh_test_cap_kernel.
+    // test counts of sampled groups by bh_test_cap_kernel; a shared walk finds
+    // it from the samples' counts in WalkCtl.
     int* fb_list = nullptr;                  // [n / 32]
     unsigned* fb_count = nullptr;            // [2]: queued groups, the walk's next group; then WalkCtl's rest
     unsigned long long* cap_state = nullptr; // [1]
@@ -111,7 +112,7 @@ struct WalkCtl {
     unsigned next;               // next group (or share of one) to take
     unsigned long long bound;    // ~(an upper bound of the cap), 0 = none yet
     unsigned finished[kCapSamples];  // sampled groups: node tests + 1, 0 = not known
-    unsigned done;               // sampled groups finished or given up
+    unsigned done[kCapSamples];  // parts of each sampled group done
     unsigned group[1];           // of a shared walk: [groups] node tests, then [groups] interactions
 };
 inline size_t walk_ctl_words(size_t n) { return sizeof(WalkCtl) / 4 + 2 * (n / 32 + 1); }
