@@ -1672,8 +1672,9 @@ using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, 
 
 // Warps per group of the default walk, and the state of such a walk with its
 // scratch (the parts' sums and, with emit, their band cells).  By default
-// enough warps for a third of the resident ones (20 per SM).  More shorten a
-// lone walk's tail, but every part walks the top of the tree, which the GPU has
+// 16 up to 2^13 bodies, 8 at 2^14, 2 at 2^15: the idle share of the GPU falls
+// with the number of groups, and so does what another part gains.  Parts shorten
+// a lone walk's tail, but every part walks the top of the tree, which the GPU has
 // no time for when other engines' kernels share it.  An Euler step alone / of
 // three engines side by side, us, with 1, 2, 4, 8 and 16 parts: 2^10 bodies
 // 105/36, 84/30, 79/26, 75/27, 73/26; 2^14 242/84, 180/67, 154/58, 144/56,
@@ -1683,13 +1684,13 @@ using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, 
 TreeState split_state(nbg_engine* e, bool emit) {
     TreeState a = *e->tree;
     const size_t n = e->count, groups = n / 64;
-    const size_t want = 13 * (size_t)e->sm_count / 2;
+    const size_t want = 20 * (size_t)e->sm_count * e->sm_count;
     const int64_t asked = std::min<int64_t>(e->tune_get("bh.parts", 0), 32);
     a.parts = 1;
     if (asked > 0)
         while (2 * a.parts <= asked) a.parts *= 2;
     else
-        while (a.parts < 16 && a.parts * groups < want) a.parts *= 2;
+        while (a.parts < 16 && a.parts * groups * groups < want) a.parts *= 2;
     if (a.parts == 1) return a;
     const size_t sums = (size_t)a.parts * 3 * n * sizeof(double);
     const size_t counts = groups * a.parts * sizeof(unsigned);
