@@ -877,6 +877,16 @@ nbg_status radix_sort(nbg_engine* e, TreeState* t, int n, int first_pass = 0) {
     return NBG_OK;
 }
 
+// Whether cluster_sort_kernel sorts n keys.  Its 8 CTAs need 8 SMs to
+// themselves, which another engine's network kernel (resident on every SM for
+// most of a learned step) holds back: with three learned engines side by side
+// 2^15 bodies take 540 us a step with it and 480 with the passes, 2^14 bodies
+// 293 and 299; alone 923 and 950.  Without the correction it is the faster one
+// up to its capacity (2^15 bodies side by side 96 against 105 us).
+bool sorts_in_cluster(const nbg_engine* e, int n) {
+    return n <= (e->params.learned ? kCSMax / 2 : kCSMax);
+}
+
 // cluster_sort_kernel for n <= kCSMax keys; axes: 3 for the coordinate lists
 template <int ITEMS>
 nbg_status cluster_sort_launch(nbg_engine* e, const ClusterSortArgs& a, int axes) {
@@ -1006,7 +1016,7 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         // the key bits from 16 up (47 of 63: the curve down to cells of
         // about 2^-16 of the box per axis), bodies sharing one in index order
         nbg_status s;
-        if (n <= kCSMax)
+        if (sorts_in_cluster(e, n))
             s = cluster_sort(e, ClusterSortArgs{t->keys[0], nullptr, {t->vals[0], nullptr, nullptr}, n, 2}, 1);
         else
             s = radix_sort(e, t, n, 2);
@@ -1024,12 +1034,13 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
     }
     t->curve = 0;
     // 1. three sorted lists
-    if (n <= kCSMax) {
+    const bool cluster = sorts_in_cluster(e, n);
+    if (cluster) {
         nbg_status s = cluster_sort(
             e, ClusterSortArgs{nullptr, y, {t->lists[0], t->lists[1], t->lists[2]}, n, 0}, 3);
         if (s != NBG_OK) return s;
     }
-    for (int d = 0; d < 3 && n > kCSMax; ++d) {
+    for (int d = 0; d < 3 && !cluster; ++d) {
         queued(init_keys_kernel, g, 256, 0, e->stream)(y + (size_t)d * n, n, t->keys[0], t->vals[0]);
         NBG_LAUNCHED(e, "init_keys_kernel");
         nbg_status s = radix_sort(e, t, n);
