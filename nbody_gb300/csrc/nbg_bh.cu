@@ -10,9 +10,12 @@
 // (nbody/nbody_space_heap.cpp:64-97) visits the same nodes in the same order,
 // so both layouts use the stackless form here.
 //
-//  * FP64 walk (precision fp64): one thread per body, the reference's
-//    arithmetic in its order (nbody_data::force, then / m_i) -- the parity
-//    path, equal to the reference's simple_bh results.
+//  * FP64 walk (precision fp64), the parity path: the reference's accepted
+//    nodes per body (exact FP64 acceptance), summed to FP64 rounding in
+//    two-word FP32 arithmetic with the large terms in FP64
+//    (bh_walk_split_kernel, 64 bodies per warp with per-body masks); without
+//    memory for its records one thread per body in the reference's order
+//    (bh_walk_fp64_kernel).
 //  * mixed walk (precision mixed): FP32 node records, one warp walks one
 //    node sequence for its 32 bodies (leaf order, so a warp holds 32
 //    neighbouring bodies): a node is opened when any lane needs it opened,
@@ -26,7 +29,8 @@
 //    with packed FP32x2 pair math (details at bh_group_walk_kernel).  Warps
 //    are persistent; a group that exceeds a node-test cap (bh_test_cap_kernel,
 //    from sampled groups' tests) is queued, and bh_body_walk_kernel walks its
-//    bodies one warp per body.
+//    bodies one warp per body.  In small systems several warps share a group
+//    (bh_split_walk_kernel, bh_walk_finish_kernel).
 //  * the quadrupole term (bh.order = 2) uses per-node second moments
 //    (quad_levels_kernel) in both the group walk and the per-body walk.
 #include <algorithm>

@@ -1,6 +1,6 @@
 // nbg_direct.cu -- direct O(N^2) gravity: f = [v ; a(y)].
 //
-// Three paths share the engine entry point:
+// Four paths share the engine entry point:
 //
 //  * FP64 (parity) -- the reference 'simple' engine's sum
 //    (nbody/nbody_engine_simple.cpp:143-172 with nbody_data::force,
@@ -28,6 +28,9 @@
 //  * mixed, symmetric (the default, tuning key direct.symmetric = 1) -- the
 //    same arithmetic with every unordered pair evaluated once and applied to
 //    both bodies (details at direct_sym_kernel).
+//
+//  * mixed, small systems (tuning key direct.small) -- ordered pairs again, a
+//    block of bodies' sums leaving its CTA once (direct_small_kernel).
 #include <algorithm>
 #include <cmath>
 #include <mutex>
