@@ -678,16 +678,6 @@ __device__ __noinline__ void walk_sample_done(const TreeState& t, int gw) {
     if (lane == 0 && u != ~0ull) atomicMax(&ctl->bound, ~u);
 }
 
-// a group's counts: 64 bits, 32 where a group's fit (nodes of one tree)
-template <bool SMALL>
-struct CountOf {
-    using T = unsigned long long;
-};
-template <>
-struct CountOf<true> {
-    using T = unsigned;
-};
-
 // BPL bodies per lane: a group of 32 BPL consecutive leaves per warp (lane l
 // holds leaves l, l + 32, ...); every list entry is evaluated for all of them.
 // SMACC: the per-body two-sum accumulators (6 BPL packed values per lane)
@@ -783,15 +773,16 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         for (int q = 0; q < 6; ++q) slot(6 * b + q) = zero;
     }
     const unsigned lt = (1u << lane) - 1u;
-    using Count = typename CountOf<SPLIT>::T;
+    using Count = unsigned;  // (a group's tests and interactions: below the tree's 2^32 nodes)
     Count tests = 0, inter = 0;
     if (lane == 0) stack[0] = 0;
     __syncwarp();
-    int sp = 1, lc = 0, peak = 1, ec = 0;
+    int sp = 1, lc = 0, peak = 1, ec = 0, first = 1;
     bool overflow = false, abandoned = false;
     const unsigned long long test_cap = SPLIT || t.test_cap != 0 ? t.test_cap : t.cap_state[0];
     WalkCtl* ctl = reinterpret_cast<WalkCtl*>(t.fb_count);
     const bool capped = SPLIT && test_cap != ~0ull;
+    const unsigned cap32 = (unsigned)min(test_cap, 0xffffffffull);
     unsigned sent = 0;  // SPLIT: tests already added to the group's
 
     auto evaluate = [&]() {
@@ -993,8 +984,8 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
                 band[w] = band[w] && mine[w];
             }
         } else {
-            tests += (unsigned long long)(2 * k);
-            if (tests > test_cap) {  // a group spread over much of the system:
+            tests += (Count)(2 * k);
+            if (tests > cap32) {  // a group spread over much of the system:
                 abandoned = true;      // its bodies are walked one by one instead
                 break;
             }
@@ -1034,13 +1025,16 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         }
         // cells with moments go to the quadrupole list (ORDER 2), the rest
         // (leaves, or every node for ORDER 1) to the monopole list
+        int before[NPL], taken[NPL];  // accepted by lower lanes, by all
 #pragma unroll
         for (int w = 0; w < NPL; ++w) {
             const bool to_quad = ORDER == 2 && accept[w] && c[w] < n;
             const bool to_mono = accept[w] && !to_quad;
             const unsigned am = __ballot_sync(0xffffffffu, to_mono);
+            before[w] = __popc(am & lt);
+            taken[w] = __popc(am);
             if (to_mono) {
-                const int q = lc + __popc(am & lt);
+                const int q = lc + before[w];
                 lx[q] = nd[w].x;
                 ly[q] = nd[w].y;
                 lz[q] = nd[w].z;
@@ -1053,12 +1047,13 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
                     llz[q] = lo.z;
                 }
             }
-            lc += __popc(am);
+            lc += taken[w];
             if (ORDER == 2) {
                 const unsigned aq = __ballot_sync(0xffffffffu, to_quad);
+                const int quads_before = __popc(aq & lt), quads = __popc(aq);
                 if (to_quad) {
                     float(*v)[kGWQList] = Q.v[warp];
-                    const int q = qc + __popc(aq & lt);
+                    const int q = qc + quads_before;
                     const float4 q0 = nq0[w], q1 = nq1[w];
                     v[0][q] = nd[w].x;
                     v[1][q] = nd[w].y;
@@ -1072,26 +1067,40 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
                     v[9][q] = q1.y;
                     v[10][q] = q1.z;
                 }
-                qc += __popc(aq);
+                qc += quads;
+                before[w] += quads_before;
+                taken[w] += quads;
             }
         }
-        unsigned om[NPL];
-        int npush = 0;
+        // the opened nodes' places on the stack.  A tested node is accepted or
+        // opened and the tested lanes are the first ones (but child 0 of the
+        // first step), so they follow from the accepted ones' counts; POPC, a
+        // quarter-rate instruction, bound the step otherwise.  A part of a
+        // shared group drops nodes and counts the opened ones.
+        int place[NPL], npush = 0;
+        if constexpr (SPLIT) {
+            unsigned om[NPL];
 #pragma unroll
-        for (int w = 0; w < NPL; ++w) {
-            om[w] = __ballot_sync(0xffffffffu, open[w]);
-            npush += __popc(om[w]);
+            for (int w = 0; w < NPL; ++w) {
+                om[w] = __ballot_sync(0xffffffffu, open[w]);
+                place[w] = sp + npush + __popc(om[w] & lt);
+                npush += __popc(om[w]);
+            }
+        } else {
+#pragma unroll
+            for (int w = 0; w < NPL; ++w) {
+                place[w] = sp + npush + lane - before[w] - (w == 0 ? first : 0);
+                npush += min(max(2 * k - 32 * w, 0), 32) - taken[w] - (w == 0 ? first : 0);
+            }
+            first = 0;
         }
         if (sp + npush > stack_cap) {  // beyond 48 entries per level: reported, never written
             overflow = true;
             break;
         }
-        int base = sp;
 #pragma unroll
-        for (int w = 0; w < NPL; ++w) {
-            if (open[w]) stack[base + __popc(om[w] & lt)] = c[w];
-            base += __popc(om[w]);
-        }
+        for (int w = 0; w < NPL; ++w)
+            if (open[w]) stack[place[w]] = c[w];
         sp += npush;
         peak = max(peak, sp);
         __syncwarp();
@@ -1151,7 +1160,7 @@ __device__ __forceinline__ void group_walk_one(const double* __restrict__ y, dou
         f2_unpack(slot(6 * bb + 5), l0, l1);
         f[5 * n + b] = ((double)h0 + (double)h1) + ((double)l0 + (double)l1);
     }
-    if (lane == 0) atomicAdd(&t.counters[1], inter * 32ull * BPL);
+    if (lane == 0) atomicAdd(&t.counters[1], (unsigned long long)inter * 32ull * BPL);
 }
 
 // Persistent over the groups (n is a power of two >= 32 BPL, so groups are
