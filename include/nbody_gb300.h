@@ -286,7 +286,8 @@ uint64_t nbg_launch_count(const nbg_engine* e);
  *       symmetric kernel; 3 runs 5 CTAs per SM),
  *       "direct.sym_blocks" (4 or 5: CTAs per SM the symmetric kernel's
  *       register budget is set for), "direct.sym_unroll" (1, 2, 4 or 8:
- *       unroll of its 32-step rotation loop, default 4),
+ *       unroll of its 32-step rotation loop, default 4, 8 from 16384
+ *       bodies on),
  *       "direct.pairs_per_lane" (2 or 4 packed i-pairs per lane, one-sided),
  *       "direct.unroll" (2, 4 or 8: j-loop unroll),
  *       "direct.blocks_per_sm" (CTAs per SM of the persistent direct grid),
