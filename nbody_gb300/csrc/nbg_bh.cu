@@ -1873,9 +1873,9 @@ nbg_status mixed_walk_impl(nbg_engine* e, const double* y, double* f, bool emit)
         a.cap_samples = t->test_cap == 0 ? samples : 0;
         a.cap_stride = warps / samples;
         // the walk's counters (and, of a shared walk, its groups')
-        NBG_CUDA(e, cudaMemsetAsync(t->fb_count, 0,
-                                    sizeof(WalkCtl) + (a.parts > 1 ? 2 * sizeof(unsigned) * (size_t)warps : 0),
-                                    e->stream));
+        nbg_status zs = set_words(
+            e, t->fb_count, sizeof(WalkCtl) / sizeof(unsigned) + (a.parts > 1 ? 2 * (size_t)warps : 0), 0);
+        if (zs != NBG_OK) return zs;
         if (t->test_cap == 0 && a.parts == 1) {
             TreeState tc = a;
             const size_t csmem = (size_t)kCapWarps * stack_cap * sizeof(int);

@@ -190,6 +190,8 @@ inline unsigned grid_for(size_t n, unsigned block, unsigned cap) {
 // ---- kernels implemented in other translation units -------------------------
 // nbg_vecops.cu
 nbg_status launch_fill(nbg_engine* e, double* a, double v, size_t n);
+// p[0 .. ones) = all ones, p[ones .. n) = 0, for a few words between kernels
+nbg_status set_words(nbg_engine* e, unsigned* p, size_t n, unsigned ones);
 struct Terms {
     static constexpr int kMax = 16;
     const double* p[kMax];

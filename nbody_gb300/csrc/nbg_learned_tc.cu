@@ -712,7 +712,8 @@ nbg_status learned_tc_walk(nbg_engine* e, const double* y, double* f) {
     // band rows on the tensor cores
     nbg_status as = tc_kernel_attrs(e, (const void*)learned_tc_kernel);
     if (as != NBG_OK) return as;
-    NBG_CUDA(e, cudaMemsetAsync(L->tc_next, 0, sizeof(unsigned), e->stream));
+    s = set_words(e, L->tc_next, 1, 0);
+    if (s != NBG_OK) return s;
     TreeState tt = *t;
     tt.cand = L->cand;
     tt.cand_n = L->cand_n;

@@ -1006,8 +1006,8 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
         // (a different tree from the reference's; the FP64 path always
         // builds the reference's)
         // box = {min keys: all ones, max keys: zero}
-        NBG_CUDA(e, cudaMemsetAsync(t->box, 0xFF, 3 * sizeof(unsigned long long), e->stream));
-        NBG_CUDA(e, cudaMemsetAsync(t->box + 3, 0, 3 * sizeof(unsigned long long), e->stream));
+        nbg_status bs = set_words(e, reinterpret_cast<unsigned*>(t->box), 12, 6);
+        if (bs != NBG_OK) return bs;
         queued(bbox_kernel, std::min(g, (unsigned)e->sm_count * 2u), 256, 0, e->stream)(y, n, t->box);
         NBG_LAUNCHED(e, "bbox_kernel");
         queued(morton_keys_kernel, g, 256, 0, e->stream)(y, n, t->box, t->keys[0], t->vals[0],
