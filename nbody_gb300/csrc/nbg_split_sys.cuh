@@ -1,6 +1,7 @@
 // nbg_split_sys.cuh -- a body system prepared for two-word arithmetic
 // (nbg_split.cuh): scaled bodies and, per body, the scale of its sum.  Used by
-// the FP64 direct sum (nbg_direct.cu) and the potential energy (nbg_stats.cu).
+// the FP64 direct sum (nbg_direct.cu), the FP64 Barnes-Hut walk (nbg_bh.cu) and
+// the potential energy (nbg_stats.cu).
 #pragma once
 
 #include <cmath>

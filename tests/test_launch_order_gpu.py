@@ -35,15 +35,14 @@ def test_dependent_vector_operations(make_engine, n):
     assert np.array_equal(got, np.stack([x, y]))
 
 
-@pytest.mark.parametrize("param", [
-    dict(algo="bh", precision="mixed", softening=1e-3, distance_to_node_radius_ratio=2.0),
-    dict(algo="bh", precision="fp64", distance_to_node_radius_ratio=2.0),
-    dict(precision="fp64"),
-])
-@pytest.mark.parametrize("n", [64, 4096, 65536])
+BH = dict(algo="bh", distance_to_node_radius_ratio=2.0)
+
+
+@pytest.mark.parametrize("n,param", [
+    (n, dict(BH, **p)) for n in (64, 4096, 65536)
+    for p in (dict(precision="mixed", softening=1e-3), dict(precision="fp64"))
+] + [(64, dict(precision="fp64")), (4096, dict(precision="fp64"))])
 def test_repeated_steps_are_equal(make_engine, param, n):
-    if n == 65536 and "algo" not in param:
-        pytest.skip("the direct sum has one chain of kernels at all sizes")
     d = NBodyData.plummer(n, seed=5)
     out = []
     for sync in (False, True):  # every kernel alone, then queued one after the other
