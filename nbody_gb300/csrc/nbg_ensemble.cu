@@ -620,7 +620,8 @@ struct nbg_ensemble {
     nbg_engine* eng = nullptr;  // stream, error text, launch count
     nbg_ensemble_params p{};
     int nsys = 0;
-    size_t B = 0;
+    size_t B = 0;               // bodies, 0 without (a whole) batch
+    bool init_failed = false;   // the last nbg_ensemble_init
     std::vector<long long> h_off;
     std::vector<int> h_cnt;
     long long* off = nullptr;
@@ -929,95 +930,29 @@ nbg_status ens_enqueue_step(nbg_ensemble* s) {
     return NBG_OK;
 }
 
+// Back to an ensemble without systems: no pointer, size or graph stays behind
+// for a later call to launch on.
 void ens_free(nbg_ensemble* s) {
-    void* ptrs[] = {s->off, s->cnt, s->sys, s->y, s->ynew, s->mass, s->sys_mass, s->bodies, s->dt, s->t,
-                    s->err, s->accepted, s->rejected, s->decision, s->err_prev, s->units,
-                    s->counters, s->sym_units, s->bpart, s->boff, s->apart, s->aoff};
-    for (void* p : ptrs) cudaFree(p);
-    s->sym_units = nullptr;
-    s->bpart = nullptr;
-    s->boff = nullptr;
-    s->apart = nullptr;
-    s->aoff = nullptr;
+    auto release = [](auto*&... p) { ((cudaFree(p), p = nullptr), ...); };
+    release(s->off, s->cnt, s->sys, s->y, s->ynew, s->mass, s->sys_mass, s->bodies, s->dt, s->t,
+            s->err, s->accepted, s->rejected, s->decision, s->err_prev, s->units, s->counters,
+            s->sym_units, s->bpart, s->boff, s->apart, s->aoff);
+    for (double*& k : s->k) release(k);
     s->apart_cap = 0;
     s->bpart_cap = 0;
-    for (double* k : s->k) cudaFree(k);
     if (s->graph) cudaGraphExecDestroy(s->graph);
     if (s->graph_def) cudaGraphDestroy(s->graph_def);
     s->graph = nullptr;
     s->graph_def = nullptr;
+    s->nsys = 0;
+    s->B = 0;
 }
 
-}  // namespace
-
-extern "C" {
-
-void nbg_ensemble_params_default(nbg_ensemble_params* p) {
-    if (p == nullptr) return;
-    memset(p, 0, sizeof(*p));
-    p->struct_size = sizeof(nbg_ensemble_params);
-    p->device = 0;
-    p->softening = 1e-3;
-    p->tolerance = 1e-8;
-    p->dt_initial = 1e-3;
-    p->dt_min = 1e-9;
-    p->dt_max = 1e-1;
-    p->use_graph = 1;
-}
-
-nbg_status nbg_ensemble_create(const nbg_ensemble_params* p, nbg_ensemble** out) {
-    if (out == nullptr) return NBG_ERR_INVALID_ARG;
-    *out = nullptr;
-    nbg_ensemble_params prm;
-    nbg_ensemble_params_default(&prm);
-    if (p != nullptr) {
-        if (p->struct_size != sizeof(nbg_ensemble_params)) return NBG_ERR_INVALID_ARG;
-        prm = *p;
-    }
-    if (!(prm.softening >= 0.0) || !(prm.tolerance > 0.0) || !(prm.dt_initial > 0.0) ||
-        !(prm.dt_min > 0.0) || !(prm.dt_max >= prm.dt_min))
-        return NBG_ERR_INVALID_ARG;
-    nbg_params ep;
-    nbg_params_default(&ep);
-    ep.device = prm.device;
-    ep.precision = NBG_PREC_MIXED;
-    ep.softening = prm.softening;
-    nbg_engine* eng = nullptr;
-    nbg_status st = nbg_engine_create(&ep, &eng);
-    if (st != NBG_OK) return st;
-    nbg_ensemble* s = new (std::nothrow) nbg_ensemble();
-    if (s == nullptr) {
-        nbg_engine_destroy(eng);
-        return NBG_ERR_OUT_OF_MEMORY;
-    }
-    s->eng = eng;
-    s->p = prm;
-    *out = s;
-    return NBG_OK;
-}
-
-void nbg_ensemble_destroy(nbg_ensemble* s) {
-    if (s == nullptr) return;
-    cudaSetDevice(s->eng->device);
-    cudaStreamSynchronize(s->eng->stream);
-    ens_free(s);
-    nbg_engine_destroy(s->eng);
-    delete s;
-}
-
-const char* nbg_ensemble_last_error(const nbg_ensemble* s) {
-    return s == nullptr ? "" : s->eng->last_error.c_str();
-}
-
-nbg_status nbg_ensemble_init(nbg_ensemble* s, size_t nsys, const uint32_t* counts,
-                             const double* vertices, const double* velocities, const double* mass) {
-    if (s == nullptr || nsys == 0 || counts == nullptr || vertices == nullptr ||
-        velocities == nullptr || mass == nullptr)
-        return NBG_ERR_INVALID_ARG;
+// The batch of nbg_ensemble_init onto the device; after an error the caller
+// frees what there is of it.
+nbg_status ens_load(nbg_ensemble* s, size_t nsys, const uint32_t* counts, const double* vertices,
+                    const double* velocities, const double* mass) {
     nbg_engine* e = s->eng;
-    NBG_CUDA(e, cudaSetDevice(e->device));
-    NBG_CUDA(e, cudaStreamSynchronize(e->stream));
-    ens_free(s);
     s->nsys = (int)nsys;
     s->h_off.assign(nsys, 0);
     s->h_cnt.assign(nsys, 0);
@@ -1086,6 +1021,84 @@ nbg_status nbg_ensemble_init(nbg_ensemble* s, size_t nsys, const uint32_t* count
     return ens_configure(s);
 }
 
+}  // namespace
+
+extern "C" {
+
+void nbg_ensemble_params_default(nbg_ensemble_params* p) {
+    if (p == nullptr) return;
+    memset(p, 0, sizeof(*p));
+    p->struct_size = sizeof(nbg_ensemble_params);
+    p->device = 0;
+    p->softening = 1e-3;
+    p->tolerance = 1e-8;
+    p->dt_initial = 1e-3;
+    p->dt_min = 1e-9;
+    p->dt_max = 1e-1;
+    p->use_graph = 1;
+}
+
+nbg_status nbg_ensemble_create(const nbg_ensemble_params* p, nbg_ensemble** out) {
+    if (out == nullptr) return NBG_ERR_INVALID_ARG;
+    *out = nullptr;
+    nbg_ensemble_params prm;
+    nbg_ensemble_params_default(&prm);
+    if (p != nullptr) {
+        if (p->struct_size != sizeof(nbg_ensemble_params)) return NBG_ERR_INVALID_ARG;
+        prm = *p;
+    }
+    if (!(prm.softening >= 0.0) || !(prm.tolerance > 0.0) || !(prm.dt_initial > 0.0) ||
+        !(prm.dt_min > 0.0) || !(prm.dt_max >= prm.dt_min))
+        return NBG_ERR_INVALID_ARG;
+    nbg_params ep;
+    nbg_params_default(&ep);
+    ep.device = prm.device;
+    ep.precision = NBG_PREC_MIXED;
+    ep.softening = prm.softening;
+    nbg_engine* eng = nullptr;
+    nbg_status st = nbg_engine_create(&ep, &eng);
+    if (st != NBG_OK) return st;
+    nbg_ensemble* s = new (std::nothrow) nbg_ensemble();
+    if (s == nullptr) {
+        nbg_engine_destroy(eng);
+        return NBG_ERR_OUT_OF_MEMORY;
+    }
+    s->eng = eng;
+    s->p = prm;
+    *out = s;
+    return NBG_OK;
+}
+
+void nbg_ensemble_destroy(nbg_ensemble* s) {
+    if (s == nullptr) return;
+    cudaSetDevice(s->eng->device);
+    cudaStreamSynchronize(s->eng->stream);
+    ens_free(s);
+    nbg_engine_destroy(s->eng);
+    delete s;
+}
+
+const char* nbg_ensemble_last_error(const nbg_ensemble* s) {
+    return s == nullptr ? "" : s->eng->last_error.c_str();
+}
+
+nbg_status nbg_ensemble_init(nbg_ensemble* s, size_t nsys, const uint32_t* counts,
+                             const double* vertices, const double* velocities, const double* mass) {
+    if (s == nullptr || nsys == 0 || counts == nullptr || vertices == nullptr ||
+        velocities == nullptr || mass == nullptr)
+        return NBG_ERR_INVALID_ARG;
+    NBG_CUDA(s->eng, cudaSetDevice(s->eng->device));
+    NBG_CUDA(s->eng, cudaStreamSynchronize(s->eng->stream));
+    ens_free(s);
+    const nbg_status st = ens_load(s, nsys, counts, vertices, velocities, mass);
+    s->init_failed = st != NBG_OK;
+    if (st != NBG_OK) {  // no half-loaded batch, and no error left for a later launch's check
+        ens_free(s);
+        cudaGetLastError();
+    }
+    return st;
+}
+
 nbg_status nbg_ensemble_step(nbg_ensemble* s, int steps) {
     if (s == nullptr || steps < 0) return NBG_ERR_INVALID_ARG;
     if (s->B == 0) return set_error(s->eng, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
@@ -1136,6 +1149,7 @@ nbg_status nbg_ensemble_status(nbg_ensemble* s, double* t, double* dt, uint32_t*
                                uint32_t* rejected) {
     if (s == nullptr) return NBG_ERR_INVALID_ARG;
     nbg_engine* e = s->eng;
+    if (s->init_failed) return set_error(e, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
     NBG_CUDA(e, cudaStreamSynchronize(e->stream));
     if (t) NBG_CUDA(e, cudaMemcpy(t, s->t, s->nsys * sizeof(double), cudaMemcpyDeviceToHost));
     if (dt) NBG_CUDA(e, cudaMemcpy(dt, s->dt, s->nsys * sizeof(double), cudaMemcpyDeviceToHost));
@@ -1149,7 +1163,9 @@ nbg_status nbg_ensemble_status(nbg_ensemble* s, double* t, double* dt, uint32_t*
 nbg_status nbg_ensemble_get_state(nbg_ensemble* s, double* vertices, double* velocities) {
     if (s == nullptr || vertices == nullptr || velocities == nullptr) return NBG_ERR_INVALID_ARG;
     nbg_engine* e = s->eng;
-    if (s->B == 0) return NBG_OK;
+    if (s->B == 0)
+        return s->init_failed ? set_error(e, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised")
+                              : NBG_OK;
     // (ynew is free between steps)
     const size_t half = 3 * s->B;
     queued(ens_state_kernel, dim3(grid_for(half, 256, (unsigned)e->sm_count * 8u), 2), 256, 0,
@@ -1182,6 +1198,7 @@ nbg_status nbg_ensemble_fcompute(nbg_ensemble* s, double* f) {
 nbg_status nbg_ensemble_statistics(nbg_ensemble* s, double* out) {
     if (s == nullptr || out == nullptr) return NBG_ERR_INVALID_ARG;
     nbg_engine* e = s->eng;
+    if (s->B == 0) return set_error(e, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
     DevScratch res;
     NBG_CUDA(e, cudaMalloc(&res.p, 12 * (size_t)s->nsys * sizeof(double)));
     nbg_status st = stats_segments(e, s->y, s->mass, s->B, s->nsys, s->off, s->cnt,
