@@ -1,0 +1,78 @@
+"""The library's host code when a CUDA call fails, in a process whose CUDA
+runtime is tests/fakes/fake_cudart.c: no GPU, no kernel runs."""
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from conftest import ROOT
+
+PRELUDE = """
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from nbody_gb300 import _lib
+from nbody_gb300._lib import NbgError
+from nbody_gb300.data import NBodyData
+from nbody_gb300.engine import create_engine
+from nbody_gb300.ensemble import Ensemble
+lib, fake = _lib.load(), C.CDLL(None)
+fake.fake_launches.restype = C.c_char_p
+fake.fake_used.restype = fake.fake_block.restype = C.c_size_t
+fake.fake_block.argtypes = [C.c_void_p]
+
+def put(name, value, kind=C.c_int):
+    kind.in_dll(fake, "fake_" + name).value = value
+
+def memory(value):
+    put("memory", value, C.c_size_t)
+
+def launched():
+    return fake.fake_launches().decode().split()
+
+def error_of(call):
+    try:
+        call()
+    except NbgError as e:
+        return str(e)
+    return None
+"""
+
+
+@pytest.fixture(scope="module")
+def run(gpulib, tmp_path_factory):
+    cc = shutil.which("gcc")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = str((ROOT / nvcc).resolve().parent.parent / "include")
+    if cc is None:
+        pytest.skip("no host compiler")
+    so = tmp_path_factory.mktemp("fake") / "fake_cudart.so"
+    r = subprocess.run([cc, "-shared", "-fPIC", "-O1", "-Wall", "-Wextra", "-Werror", "-I", include,
+                        str(ROOT / "tests" / "fakes" / "fake_cudart.c"), "-o", str(so)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def _run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code), str(ROOT)],
+                           capture_output=True, text=True, timeout=300,
+                           env={"LD_PRELOAD": str(so), "PATH": "/usr/bin:/bin"})
+        assert r.returncode == 0, r.stdout + r.stderr[-3000:]
+
+    return _run
+
+
+@pytest.mark.parametrize("fails", ["sync", "copy"])
+def test_state_arrays_keep_their_contents(run, fails):
+    """A get_state that reports an error has written nothing to the caller's
+    arrays."""
+    run(f"""
+    ens = Ensemble()
+    ens.init([NBodyData.plummer(700, seed=1)])
+    v, u = (np.random.default_rng(k).normal(size=(700, 3)) for k in (1, 2))
+    want = v.copy(), u.copy()
+    put("{fails}_error", 719)
+    assert lib.nbg_ensemble_get_state(ens._h, v.ctypes.data, u.ctypes.data) != 0
+    assert np.array_equal(v, want[0]) and np.array_equal(u, want[1])
+    """)
