@@ -626,6 +626,7 @@ struct nbg_ensemble {
     int nsys = 0;
     size_t B = 0;               // bodies, 0 without (a whole) batch
     bool init_failed = false;   // the last nbg_ensemble_init
+    bool ready = false;         // units, partials and launch shape are those of the batch
     std::vector<long long> h_off;
     std::vector<int> h_cnt;
     long long* off = nullptr;
@@ -704,6 +705,21 @@ using EnsSym = void (*)(const Body2*, const long long*, const int*, const EnsSym
 constexpr size_t kEnsUnitsPerSlot = 8;  // (4 to 16 measured the same)
 constexpr size_t kEnsMaxSegBytes = size_t(1) << 30;
 
+// At least `count` entries at *p; false (and no buffer) when they cannot be had.
+template <class T>
+bool ens_reserve(T** p, size_t* cap, size_t count) {
+    if (*cap >= count) return true;
+    cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    if (cudaMalloc(p, count * sizeof(T)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    *cap = count;
+    return true;
+}
+
 template <bool UNI>
 EnsSym ens_pick_sym_g(bool clamp, int G) {
     return clamp ? (G == 1 ? ens_sym_kernel<true, 1, UNI> : ens_sym_kernel<true, 2, UNI>)
@@ -716,8 +732,9 @@ EnsSym ens_pick_sym(const nbg_ensemble* s) {
 }
 
 // The symmetric kernel's units, cost-ordered (largest first, so the tail of
-// the persistent launch is made of small units), and its partial buffer.
-nbg_status ens_configure_sym(nbg_ensemble* s) {
+// the persistent launch is made of small units), and its partial buffers;
+// *done false when there is no memory for those.
+nbg_status ens_configure_sym(nbg_ensemble* s, bool* done) {
     nbg_engine* e = s->eng;
     const int ra = kEnsThreads * 2 * s->G;
     struct Costed {
@@ -729,8 +746,9 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
     occ = std::max(occ, 1);
     const int64_t bps = e->tune_get("ensemble.blocks_per_sm", 0);
     if (bps > 0 && bps < occ) occ = (int)bps;
-    // tiles per unit: about kEnsUnitsPerSlot units for each resident CTA, and
-    // A partials of at most kEnsMaxSegBytes
+    // tiles per unit: about kEnsUnitsPerSlot units for each resident CTA, and A
+    // partials of at most kEnsMaxSegBytes, or of one segment a range (24 bytes a
+    // body) when the device has no memory for more
     const int tpr = ra / kEnsTile;
     auto tiles_of = [](int n) { return (n + kEnsTile - 1) / kEnsTile; };
     size_t tiles = 0;
@@ -738,25 +756,42 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
         for (int t = tiles_of(n); t > 0; t -= tpr) tiles += (size_t)t;
     const size_t slots = (size_t)e->sm_count * occ * kEnsUnitsPerSlot;
     s->seg_tiles = (int)std::max<size_t>(1, (tiles + slots - 1) / slots);
-    std::vector<long long> aoff(s->nsys);
-    long long atotal = 0;
-    while (true) {
-        atotal = 0;
+    std::vector<long long> aoff(s->nsys), boff(s->nsys);
+    long long btotal = 0;
+    for (int sI = 0; sI < s->nsys; ++sI) {
+        boff[sI] = btotal;
+        btotal += (long long)((s->h_cnt[sI] + ra - 1) / ra) * s->h_cnt[sI];
+    }
+    s->bstride = (size_t)btotal;
+    bool fits = ens_reserve(&s->bpart, &s->bpart_cap, 3 * s->bstride);
+    const int one_segment = tiles_of(*std::max_element(s->h_cnt.begin(), s->h_cnt.end()));
+    for (bool again = fits; again;) {
+        long long atotal = 0;
         for (int sI = 0; sI < s->nsys; ++sI) {
             aoff[sI] = atotal;
             atotal += (long long)ens_segments(tiles_of(s->h_cnt[sI]), tpr, 0, s->seg_tiles) * s->h_cnt[sI];
         }
-        if (3 * (size_t)atotal * sizeof(float2) <= kEnsMaxSegBytes || s->seg_tiles > (1 << 24)) break;
-        s->seg_tiles *= 2;
+        s->astride = (size_t)atotal;
+        const bool more = s->seg_tiles < one_segment;
+        if (more && 3 * s->astride * sizeof(float2) > kEnsMaxSegBytes) {
+            s->seg_tiles *= 2;
+            continue;
+        }
+        fits = ens_reserve(&s->apart, &s->apart_cap, 3 * s->astride);
+        again = !fits && more;
+        s->seg_tiles = again ? one_segment : s->seg_tiles;
+    }
+    *done = fits;
+    if (!fits) {
+        cudaFree(s->bpart);
+        s->bpart = nullptr;
+        s->bpart_cap = 0;
+        return NBG_OK;
     }
     std::vector<Costed> units;
-    std::vector<long long> boff(s->nsys);
-    long long total = 0;
     for (int sI = 0; sI < s->nsys; ++sI) {
         const int n = s->h_cnt[sI];
         const int ranges = (n + ra - 1) / ra;
-        boff[sI] = total;
-        total += (long long)ranges * n;
         for (int r = 0; r < ranges; ++r) {
             const int segs = ens_segments(tiles_of(n), tpr, r, s->seg_tiles);
             for (int k = 0; k < segs; ++k) {
@@ -783,29 +818,20 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
     NBG_CUDA(e, cudaMalloc(&s->boff, boff.size() * sizeof(long long)));
     NBG_CUDA(e, cudaMemcpy(s->boff, boff.data(), boff.size() * sizeof(long long),
                            cudaMemcpyHostToDevice));
-    s->bstride = (size_t)std::max<long long>(total, 1);
-    if (s->bpart_cap < 3 * s->bstride) {
-        cudaFree(s->bpart);
-        s->bpart = nullptr;
-        s->bpart_cap = 0;
-        NBG_CUDA(e, cudaMalloc(&s->bpart, 3 * s->bstride * sizeof(float)));
-        s->bpart_cap = 3 * s->bstride;
-    }
     cudaFree(s->aoff);
     s->aoff = nullptr;
     NBG_CUDA(e, cudaMalloc(&s->aoff, aoff.size() * sizeof(long long)));
     NBG_CUDA(e, cudaMemcpy(s->aoff, aoff.data(), aoff.size() * sizeof(long long),
                            cudaMemcpyHostToDevice));
-    s->astride = (size_t)std::max<long long>(atotal, 1);
-    if (s->apart_cap < 3 * s->astride) {
-        cudaFree(s->apart);
-        s->apart = nullptr;
-        s->apart_cap = 0;
-        NBG_CUDA(e, cudaMalloc(&s->apart, 3 * s->astride * sizeof(float2)));
-        s->apart_cap = 3 * s->astride;
-    }
     s->force_grid = (unsigned)std::max(1, std::min(s->nsym_units, e->sm_count * occ));
     return NBG_OK;
+}
+
+void ens_drop_graph(nbg_ensemble* s) {
+    if (s->graph) cudaGraphExecDestroy(s->graph);
+    if (s->graph_def) cudaGraphDestroy(s->graph_def);
+    s->graph = nullptr;
+    s->graph_def = nullptr;
 }
 
 // Work units and launch shape from the tuning keys (the i-block tile of
@@ -816,10 +842,14 @@ nbg_status ens_configure_sym(nbg_ensemble* s) {
 // component: small for many small systems (300 MB for 2048 systems of up to
 // 4096 bodies), but growing as N^2 / RA for one large system; above this
 // size the ensemble uses the one-sided kernel, which needs no such buffer.
+// It also uses that kernel when the device has no memory for the partials.
 constexpr size_t kEnsSymMaxPartialBytes = size_t(8) << 30;
 
 nbg_status ens_configure(nbg_ensemble* s) {
     nbg_engine* e = s->eng;
+    s->ready = false;
+    NBG_CUDA(e, cudaStreamSynchronize(e->stream));
+    ens_drop_graph(s);
     s->G = (int)std::max<int64_t>(1, std::min<int64_t>(2, e->tune_get("ensemble.pairs_per_lane", 2)));
     s->sym = e->tune_get("ensemble.symmetric", 1) != 0;
     if (s->sym) {
@@ -832,14 +862,10 @@ nbg_status ens_configure(nbg_ensemble* s) {
         if (3 * floats * sizeof(float) > kEnsSymMaxPartialBytes) s->sym = false;
     }
     if (s->sym) {
-        NBG_CUDA(e, cudaStreamSynchronize(e->stream));
-        nbg_status st = ens_configure_sym(s);
+        nbg_status st = ens_configure_sym(s, &s->sym);
         if (st != NBG_OK) return st;
-        if (s->graph) cudaGraphExecDestroy(s->graph);
-        if (s->graph_def) cudaGraphDestroy(s->graph_def);
-        s->graph = nullptr;
-        s->graph_def = nullptr;
-        return NBG_OK;
+        s->ready = s->sym;
+        if (s->ready) return NBG_OK;
     }
     const int blk = kEnsThreads * 2 * s->G;
     std::vector<EnsUnit> units;
@@ -857,16 +883,12 @@ nbg_status ens_configure(nbg_ensemble* s) {
     const int64_t bps = e->tune_get("ensemble.blocks_per_sm", 0);
     if (bps > 0 && bps < occ) occ = (int)bps;
     s->force_grid = (unsigned)std::max(1, std::min(s->nunits, e->sm_count * occ));
-    NBG_CUDA(e, cudaStreamSynchronize(e->stream));
     cudaFree(s->units);
     s->units = nullptr;
     NBG_CUDA(e, cudaMalloc(&s->units, units.size() * sizeof(EnsUnit)));
     NBG_CUDA(e, cudaMemcpy(s->units, units.data(), units.size() * sizeof(EnsUnit),
                            cudaMemcpyHostToDevice));
-    if (s->graph) cudaGraphExecDestroy(s->graph);
-    if (s->graph_def) cudaGraphDestroy(s->graph_def);
-    s->graph = nullptr;
-    s->graph_def = nullptr;
+    s->ready = true;
     return NBG_OK;
 }
 
@@ -958,12 +980,10 @@ void ens_free(nbg_ensemble* s) {
     for (double*& k : s->k) release(k);
     s->apart_cap = 0;
     s->bpart_cap = 0;
-    if (s->graph) cudaGraphExecDestroy(s->graph);
-    if (s->graph_def) cudaGraphDestroy(s->graph_def);
-    s->graph = nullptr;
-    s->graph_def = nullptr;
+    ens_drop_graph(s);
     s->nsys = 0;
     s->B = 0;
+    s->ready = false;
 }
 
 // The batch of nbg_ensemble_init onto the device; after an error the caller
@@ -1119,7 +1139,7 @@ nbg_status nbg_ensemble_init(nbg_ensemble* s, size_t nsys, const uint32_t* count
 
 nbg_status nbg_ensemble_step(nbg_ensemble* s, int steps) {
     if (s == nullptr || steps < 0) return NBG_ERR_INVALID_ARG;
-    if (s->B == 0) return set_error(s->eng, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
+    if (!s->ready) return set_error(s->eng, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
     nbg_engine* e = s->eng;
     NBG_CUDA(e, cudaSetDevice(e->device));
     if (!s->p.use_graph) {
@@ -1205,7 +1225,7 @@ nbg_status nbg_ensemble_get_state(nbg_ensemble* s, double* vertices, double* vel
 nbg_status nbg_ensemble_fcompute(nbg_ensemble* s, double* f) {
     if (s == nullptr || f == nullptr) return NBG_ERR_INVALID_ARG;
     nbg_engine* e = s->eng;
-    if (s->B == 0) return set_error(e, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
+    if (!s->ready) return set_error(e, NBG_ERR_NOT_INITIALIZED, "ensemble not initialised");
     // stage 0 of a step: k_0 = [v ; a(y)] of the current state
     nbg_status st = ens_enqueue_force(s);
     if (st != NBG_OK) return st;

@@ -76,3 +76,53 @@ def test_state_arrays_keep_their_contents(run, fails):
     assert lib.nbg_ensemble_get_state(ens._h, v.ctypes.data, u.ctypes.data) != 0
     assert np.array_equal(v, want[0]) and np.array_equal(u, want[1])
     """)
+
+
+@pytest.mark.parametrize("spare,kernel", [
+    (2 ** 40, "ens_sym_kernel"),    # segments of two tiles
+    (10 << 20, "ens_sym_kernel"),   # 24 bytes a body: one segment a range
+    (1 << 20, "ens_force_kernel"),  # the other partials fit, these do not
+    (-20 << 20, "ens_force_kernel"),  # none do
+])
+def test_ensemble_with_little_memory(run, spare, kernel):
+    """A batch whose state fits is accepted, whatever is left for the symmetric
+    kernel's partials; `spare` bytes beyond the state and the B partials."""
+    run(f"""
+    systems = [NBodyData.uniform_cube(16384, seed=k) for k in range(4)]
+    ens = Ensemble(use_graph=False)
+    ens.tune_set("ensemble.symmetric", 0)
+    ens.init(systems)
+    state = fake.fake_used()
+    partials = 4 * 16384 * (16384 // 512) * 12
+    ens.tune_set("ensemble.symmetric", 1)   # with all the memory there is
+    launched()
+    ens.step(1)
+    assert any("ens_sym_kernel" in k for k in launched())
+    memory(state + partials + {spare})
+    ens.init(systems)
+    for call in (lambda: ens.step(1), lambda: ens.fcompute(), lambda: ens.autotune(1)):
+        launched()
+        call()
+        assert any("{kernel}" in k for k in launched())
+    assert fake.fake_used() <= state + partials + {spare}
+    """)
+
+
+def test_ensemble_without_a_configuration(run):
+    """A tuning key whose shape cannot be had leaves a batch that says so and
+    that another key makes whole again."""
+    run("""
+    ens = Ensemble()
+    ens.init([NBodyData.uniform_cube(16384, seed=k) for k in range(4)])
+    ens.step(1)
+    memory(0)
+    assert error_of(lambda: ens.tune_set("ensemble.symmetric", 0)) is not None
+    launched()
+    assert "not initialised" in error_of(lambda: ens.step(1))
+    assert "not initialised" in error_of(lambda: ens.fcompute())
+    assert launched() == []
+    memory(2 ** 40)
+    fake.cudaGetLastError()
+    ens.tune_set("ensemble.symmetric", 0)
+    ens.step(1)
+    """)
