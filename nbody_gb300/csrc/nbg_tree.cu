@@ -882,42 +882,77 @@ nbg_status radix_sort(nbg_engine* e, TreeState* t, int n, int first_pass = 0) {
 // most of a learned step) holds back: with three learned engines side by side
 // 2^15 bodies take 540 us a step with it and 480 with the passes, 2^14 bodies
 // 293 and 299; alone 923 and 950.  Without the correction it is the faster one
-// up to its capacity (2^15 bodies side by side 96 against 105 us).
+// up to its capacity (2^15 bodies side by side 96 against 105 us).  A process
+// that has only part of the GPU's SMs may have no room for the cluster at all
+// (TreeState::clusters).
 bool sorts_in_cluster(const nbg_engine* e, int n) {
-    return n <= (e->params.learned ? kCSMax / 2 : kCSMax);
+    return e->tree->clusters && n <= (e->params.learned ? kCSMax / 2 : kCSMax);
+}
+
+struct ClusterLaunch {
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = {};
+    ClusterLaunch(int axes, size_t smem, cudaStream_t stream) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kCSCtas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = dim3(kCSCtas, (unsigned)axes);
+        cfg.blockDim = dim3(kCSThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 2;  // (as queued() launches, which take no cluster)
+    }
+};
+
+template <int ITEMS>
+cudaError_t cluster_sort_attrs() {
+    return cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(ClusterSortSmem<ITEMS>));
+}
+
+// Whether its cluster fits the SMs that this process has.
+template <int ITEMS>
+bool cluster_fits(nbg_engine* e) {
+    const ClusterLaunch l(1, sizeof(ClusterSortSmem<ITEMS>), e->stream);
+    int clusters = 0;
+    if (cluster_sort_attrs<ITEMS>() == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel<ITEMS>, &l.cfg) == cudaSuccess)
+        return clusters > 0;
+    cudaGetLastError();
+    return false;
 }
 
 // cluster_sort_kernel for n <= kCSMax keys; axes: 3 for the coordinate lists
 template <int ITEMS>
 nbg_status cluster_sort_launch(nbg_engine* e, const ClusterSortArgs& a, int axes) {
-    const size_t smem = sizeof(ClusterSortSmem<ITEMS>);
-    NBG_CUDA(e, cudaFuncSetAttribute(cluster_sort_kernel<ITEMS>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kCSCtas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kCSCtas, (unsigned)axes);
-    cfg.blockDim = dim3(kCSThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = e->stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;  // (as queued() launches, which take no cluster)
-    NBG_CUDA(e, cudaLaunchKernelEx(&cfg, cluster_sort_kernel<ITEMS>, a));
+    NBG_CUDA(e, cluster_sort_attrs<ITEMS>());
+    const ClusterLaunch l(axes, sizeof(ClusterSortSmem<ITEMS>), e->stream);
+    NBG_CUDA(e, cudaLaunchKernelEx(&l.cfg, cluster_sort_kernel<ITEMS>, a));
     NBG_LAUNCHED(e, "cluster_sort_kernel");
     return NBG_OK;
 }
 
+// keys per thread of a sort of n keys
+constexpr int cluster_items(int n) { return (n + kCSCtas * kCSThreads - 1) / (kCSCtas * kCSThreads); }
+
 nbg_status cluster_sort(nbg_engine* e, const ClusterSortArgs& a, int axes) {
-    const int per = (a.n + kCSCtas * kCSThreads - 1) / (kCSCtas * kCSThreads);
+    const int per = cluster_items(a.n);
     if (per <= 1) return cluster_sort_launch<1>(e, a, axes);
     if (per <= 2) return cluster_sort_launch<2>(e, a, axes);
     if (per <= 4) return cluster_sort_launch<4>(e, a, axes);
     return cluster_sort_launch<kCSItems>(e, a, axes);
+}
+
+bool cluster_fits(nbg_engine* e, int n) {
+    const int per = cluster_items(n);
+    return per <= 1   ? cluster_fits<1>(e)
+           : per <= 2 ? cluster_fits<2>(e)
+           : per <= 4 ? cluster_fits<4>(e)
+                      : per <= kCSItems && cluster_fits<kCSItems>(e);
 }
 
 // Levels [lv_lo, lv_hi) of the heap, bottom-up, in one launch: block b owns
@@ -987,6 +1022,7 @@ nbg_status tree_build(nbg_engine* e, const double* y, bool fp64_nodes, double la
             tree_destroy(e);
             return s;
         }
+        e->tree->clusters = cluster_fits(e, n);
     }
     TreeState* t = e->tree;
     t->lambda = lambda;

@@ -22,6 +22,7 @@ struct TreeState {
     // build scratch
     uint64_t* keys[2] = {nullptr, nullptr};  // radix keys (ping-pong)
     int* vals[2] = {nullptr, nullptr};       // radix values (ping-pong)
+    bool clusters = false;  // cluster_sort_kernel takes n and has room
     int* lists[3] = {nullptr, nullptr, nullptr};  // bodies sorted by x / y / z per segment
     int* spare[2] = {nullptr, nullptr};      // partition outputs
     unsigned char* flag = nullptr;           // [n] 1 = goes to the left child

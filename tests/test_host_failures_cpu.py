@@ -126,3 +126,21 @@ def test_ensemble_without_a_configuration(run):
     ens.tune_set("ensemble.symmetric", 0)
     ens.step(1)
     """)
+
+
+@pytest.mark.parametrize("param", [dict(precision="fp64"), dict(precision="mixed")])
+@pytest.mark.parametrize("clusters", [0, 1])
+def test_tree_without_clusters(run, param, clusters):
+    """A process whose SMs have no room for a cluster sorts in passes."""
+    run(f"""
+    put("clusters", {clusters})
+    e = create_engine(dict({param}, engine="gb300", algo="bh"))
+    assert e.init(NBodyData.uniform_cube(1024, seed=1))
+    f = e.create_buffer(8 * 6 * 1024)
+    for _ in range(2):
+        e.fcompute(0.0, e.get_y(), f)
+        names = launched()
+        assert any("cluster_sort_kernel" in k for k in names) == bool({clusters})
+        assert any("radix_scatter_kernel" in k for k in names) != bool({clusters})
+        e.advise_time(0.0)
+    """)
