@@ -127,8 +127,8 @@ __global__ void bh_walk_fp64_kernel(const double* __restrict__ y, const double* 
 // lane, against the bounding box of the 64 bodies: most are accepted or
 // opened by every body whatever its place in the box; the others (a quarter
 // in a Plummer sphere) are tested body by body, in FP32 outside a margin of
-// 2^-20 around the critical radius and by the reference's FP64 expression
-// inside it.  Accepted nodes are listed and summed as in the direct sum
+// 2^-20 around the critical radius (kSWSure) and by the reference's FP64
+// expression inside it.  Accepted nodes are listed and summed as in the direct sum
 // (split_force_kernel): two-word terms; large ones (t > kSplitNear of the
 // body's scale) and close ones are queued per body and taken in FP64.
 // Nodes above level `top` are tested by every part and summed by one, the
@@ -146,6 +146,11 @@ __global__ void bh_walk_fp64_kernel(const double* __restrict__ y, const double* 
 constexpr int kSWStack = 320;   // see the pop rule
 constexpr int kSWList = 64;     // accepted nodes: fewer than 32 before a step adds at most 32
 constexpr int kSWQ = 16;        // queued nodes per body
+// A body's test leaves out the coordinates' last words, up to 2^-46 each: r^2 is
+// off by 2 sqrt(3) 2^-45 / r of itself, and by 6 2^-24 from the roundings of the
+// differences, the squares' sum and the critical radius.  Above this r^2 (in
+// units of the extent's square) both together stay below 2^-20.
+constexpr float kSWSure = 4e-14f;
 constexpr int kSWWarps = 16384;  // warps wanted: parts = kSWWarps / groups, 2 to 16
 
 struct SplitWalkArgs {
@@ -386,8 +391,8 @@ __global__ void __launch_bounds__(32, 16) bh_walk_split_kernel(SplitWalkArgs a) 
             float r0, r1;
             f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), r0, r1);
             bool a0 = r0 > cr.x, a1 = r1 > cr.x;
-            const bool sure0 = a0 ? r0 > 1e-24f : r0 < cr.y && cr.y > 1e-24f;
-            const bool sure1 = a1 ? r1 > 1e-24f : r1 < cr.y && cr.y > 1e-24f;
+            const bool sure0 = a0 ? r0 > kSWSure : r0 < cr.y && cr.y > kSWSure;
+            const bool sure1 = a1 ? r1 > kSWSure : r1 < cr.y && cr.y > kSWSure;
             if (!sure0) a0 = accept_fp64(t, nr, n + k0);
             if (!sure1) a1 = accept_fp64(t, nr, n + k1);
             const unsigned A0 = __ballot_sync(0xffffffffu, a0) & m0;
