@@ -183,14 +183,13 @@ __global__ void __launch_bounds__(256) split_nodes_kernel(SplitSystem s, TreeSta
             split3(ex == 2048 ? nan("") : fabs(x) < 1.0 ? x : 0.0, h[c], m[c], l[c]);
         }
         const double ms = t.mass[i] * s.mass_scale;
-        const bool tiny = ms != 0.0 && fabs(ms) < 9.313225746154785e-10;  // as in split_pack_kernel
         const float mh = (float)ms, ml = (float)(ms - (double)mh);
         const double cr = scalbn(t.crit2[i], -2 * min(ex, 1000));
         SplitNode& o = reinterpret_cast<SplitNode*>(t.split)[i];
         o.b.a = make_float4(h[0], m[0], l[0], h[1]);
         o.b.b = make_float4(m[1], l[1], h[2], m[2]);
         const float none = __int_as_float(0x7fffffff);
-        o.b.c = make_float4(l[2], mh, ml, tiny || !inside ? none : fabsf(mh));
+        o.b.c = make_float4(l[2], mh, ml, inside ? split_mass_size(ms) : none);
         o.crit = make_float4(inside ? (float)(cr * (1.0 + 9.5367431640625e-07)) : none,
                              inside ? (float)(cr * (1.0 - 9.5367431640625e-07)) : none, 0.f, 0.f);
     }

@@ -85,6 +85,15 @@ __device__ __forceinline__ int split_exponent(const SplitSystem& a) {
     return ex == 0x7ff ? 2048 : ex - 1022;
 }
 
+// |m| of a scaled mass as the near test reads it: NaN, so that FP64 takes all of
+// its terms, for a mass far below the largest and for one that is not finite
+// (whose two words would be inf - inf).
+__device__ __forceinline__ float split_mass_size(double ms) {
+    const double a = fabs(ms);
+    const bool words = ms == 0.0 || (a >= 9.313225746154785e-10 && a <= 1.7976931348623157e308);  // 2^-30
+    return words ? (float)a : __int_as_float(0x7fffffff);
+}
+
 __global__ void __launch_bounds__(256) split_pack_kernel(SplitSystem a) {
     if (!after_previous()) return;
     const int ex = split_exponent(a);
@@ -96,12 +105,10 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitSystem a) {
             for (int c = 0; c < 3; ++c)
                 split3(ex == 2048 ? nan("") : scalbn(a.y[(size_t)c * a.n + i], -ex), h[c], m[c], l[c]);
             const double ms = a.mass[i] * a.mass_scale;
-            // a mass far below the largest is taken in FP64 throughout
-            const bool tiny = ms != 0.0 && fabs(ms) < 9.313225746154785e-10;  // 2^-30
             const float mh = (float)ms, ml = (float)(ms - (double)mh);
             b.a = make_float4(h[0], m[0], l[0], h[1]);
             b.b = make_float4(m[1], l[1], h[2], m[2]);
-            b.c = make_float4(l[2], mh, ml, tiny ? __int_as_float(0x7fffffff) : fabsf(mh));
+            b.c = make_float4(l[2], mh, ml, split_mass_size(ms));
         } else {
             // padding: massless, and so far away that r^-3 underflows to 0
             b.a = make_float4(1e18f, 0.f, 0.f, 1e18f);
@@ -135,7 +142,8 @@ __global__ void __launch_bounds__(kSplitT) split_estimate_kernel(SplitSystem a) 
         __syncthreads();
         SplitBody b = a.bodies[min(run, runs - 1) * 32 + (tid & 31)];
         if (run >= runs) b.c.y = 0.f;
-        const float m = fabsf(b.c.y);
+        // (a mass that is not finite does not count: the scale stays finite)
+        const float m = fabsf(b.c.y) <= 1.f ? fabsf(b.c.y) : 0.f;
         tile[tid][0] = make_float4(b.a.x, b.a.x, b.a.w, b.a.w);
         tile[tid][1] = make_float4(b.b.z, b.b.z, m, m);
         __syncthreads();
