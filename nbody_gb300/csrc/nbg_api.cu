@@ -358,7 +358,8 @@ nbg_status nbg_init(nbg_engine* e, size_t count, const double* vertices,
     double largest = 0.0;
     for (size_t i = 0; i < count; ++i)
         if (std::isfinite(mass[i])) largest = std::max(largest, std::fabs(mass[i]));
-    std::frexp(largest, &e->mass_exp);  // 0 for 0
+    std::frexp(largest, &e->mass_exp);          // 0 for 0
+    e->mass_exp = std::max(e->mass_exp, -1022);  // 2^-mass_exp is finite
     NBG_CUDA(e, cudaMemcpy(y->dptr, h.data(), 6 * count * sizeof(double),
                            cudaMemcpyHostToDevice));
     NBG_CUDA(e, cudaMemcpy(e->d_mass, mass, count * sizeof(double), cudaMemcpyHostToDevice));
