@@ -144,3 +144,29 @@ def test_tree_without_clusters(run, param, clusters):
         assert any("radix_scatter_kernel" in k for k in names) != bool({clusters})
         e.advise_time(0.0)
     """)
+
+
+def test_scratch_of_captured_launches_is_kept(run):
+    """A scratch block that captured launches read outlives its growth and is
+    given back with the engine; one that none read is given back at once."""
+    run("""
+    def growth(captured):
+        free = fake.fake_used()
+        e = create_engine(dict(engine="gb300", precision="mixed", softening=1e-2))
+        assert e.init(NBodyData.uniform_cube(20000, seed=1))
+        f = e.create_buffer(8 * 6 * 20000)
+        before = fake.fake_used()
+        e.fcompute(0.0, e.get_y(), f)
+        block = fake.fake_used() - before
+        put("capturing", captured)
+        e.fcompute(0.0, e.get_y(), f)
+        put("capturing", 0)
+        e.statistics()   # needs a larger block
+        grown = fake.fake_used() - before
+        e.close()
+        assert fake.fake_used() == free
+        return block, grown
+    (b0, g0), (b1, g1) = growth(0), growth(1)
+    assert b0 == b1 and b0 >= 20000 * 32 and g0 > b0
+    assert g1 == g0 + b0
+    """)
