@@ -49,3 +49,14 @@ def test_state_of_an_ensemble_without_a_batch(gpulib):
     v, u = ens.get_state()
     assert v.shape == u.shape == (0, 3)
     ens.close()
+
+
+@pytest.mark.parametrize("sizes", [(1,), (8192,), (8193,), (4096, 4096), (4096, 4096, 1)])
+def test_state_laid_out_by_host_and_kernel(gpulib, sizes):
+    systems = _systems(*sizes)
+    ens = Ensemble()
+    ens.init(systems)
+    v, u = ens.get_state()
+    assert np.array_equal(v, np.concatenate([d.vertices for d in systems]))
+    assert np.array_equal(u, np.concatenate([d.velocities for d in systems]))
+    ens.close()

@@ -63,18 +63,30 @@ def run(gpulib, tmp_path_factory):
     return _run
 
 
+@pytest.mark.parametrize("n", [700, 9000])
 @pytest.mark.parametrize("fails", ["sync", "copy"])
-def test_state_arrays_keep_their_contents(run, fails):
+def test_state_arrays_keep_their_contents(run, fails, n):
     """A get_state that reports an error has written nothing to the caller's
     arrays."""
     run(f"""
     ens = Ensemble()
-    ens.init([NBodyData.plummer(700, seed=1)])
-    v, u = (np.random.default_rng(k).normal(size=(700, 3)) for k in (1, 2))
+    ens.init([NBodyData.plummer({n}, seed=1)])
+    v, u = (np.random.default_rng(k).normal(size=({n}, 3)) for k in (1, 2))
     want = v.copy(), u.copy()
     put("{fails}_error", 719)
     assert lib.nbg_ensemble_get_state(ens._h, v.ctypes.data, u.ctypes.data) != 0
     assert np.array_equal(v, want[0]) and np.array_equal(u, want[1])
+    """)
+
+
+@pytest.mark.parametrize("n,kernels", [(1, 0), (8192, 0), (8193, 1)])
+def test_state_of_a_small_batch_needs_no_kernel(run, n, kernels):
+    run(f"""
+    ens = Ensemble()
+    ens.init([NBodyData.uniform_cube({n}, seed=1)])
+    launched()
+    ens.get_state()
+    assert len(launched()) == {kernels}
     """)
 
 
