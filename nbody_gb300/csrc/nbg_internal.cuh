@@ -52,7 +52,7 @@ struct nbg_engine {
     float* d_massf = nullptr;    // [N] (mixed paths)
     bool uniform_mass = false;   // every body has the mass mass_value
     double mass_value = 0.0;
-    int mass_exp = 0;            // largest finite |mass| < 2^mass_exp
+    int mass_exp = 0;            // largest finite |mass| < 2^mass_exp, at least -1022
 
     // scratch of one call (packed bodies, partial sums), kept and grown
     float4* d_xyzm = nullptr;
