@@ -138,8 +138,8 @@ __global__ void bh_walk_fp64_kernel(const double* __restrict__ y, const double* 
 // Bound by instruction issue and latency (16 warps of 128 registers per SM):
 // 2^15 bodies of a Plummer sphere at ratio 2 (2448 interactions a body) in
 // 1.4 ms, 2^18 in 26 ms and 2^20 in 0.21 s with the kd build; one thread per
-// body on the FP64 pipe 18.4 ms, 0.49 s and 4.66 s, testing every node body
-// by body 2.0 ms, 43 ms and - (59 % of the time).  Fewer, larger parts leave
+// body on the FP64 pipe 18.4 ms, 0.49 s and 4.66 s.  Testing every node body by
+// body took 59 % of the walk, 2.0 ms at 2^15 and 43 at 2^18.  Fewer, larger parts leave
 // SMs idle at the end (2^18 bodies: 32 ms with 1 part, 27 with 4), more repeat
 // the top of the tree (2^15 bodies of a uniform cube: 1.70 ms with 16, 1.79
 // with 32).
@@ -1689,15 +1689,19 @@ using WalkKernel = void (*)(const double*, double*, int, float, TreeState, int, 
 
 // Warps per group of the default walk, and the state of such a walk with its
 // scratch (the parts' sums and, with emit, their band cells).  By default
-// 16 up to 2^13 bodies, 8 at 2^14, 2 at 2^15: the idle share of the GPU falls
-// with the number of groups, and so does what another part gains.  Parts shorten
-// a lone walk's tail, but every part walks the top of the tree, which the GPU has
-// no time for when other engines' kernels share it.  An Euler step alone / of
-// three engines side by side, us, with 1, 2, 4, 8 and 16 parts: 2^10 bodies
+// 16 up to 2^13 bodies, 8 at 2^14, 2 at 2^15, else 1: the idle share of the GPU
+// falls with the number of groups, and so does what another part gains.  Parts
+// shorten a lone walk's tail, but every part walks the top of the tree, which the
+// GPU has no time for when other engines' kernels share it.  An Euler step alone /
+// of three engines side by side, us, with 1, 2, 4, 8 and 16 parts: 2^10 bodies
 // 105/36, 84/30, 79/26, 75/27, 73/26; 2^14 242/84, 180/67, 154/58, 144/56,
 // 148/72; 2^15 300/118, 227/89, 203/82, 191/94, with the learned correction
 // 951/542, 915/525, 898/540; 2^16 361/148, 307/150, 284/165, with quadrupoles
-// at ratio 4 1078/555, 946/605, 848/617.
+// at ratio 4 1078/555, 946/605, 848/617.  One rule serves every walk and is set by
+// the engines side by side, a lone one could do with more: at 2^15 two parts are
+// the learned walk's best side by side, without the correction four are 8 to 11 %
+// faster; at 2^16 one part gives up a fifth of a lone engine's step for 10 % of
+// three engines' ("bh.parts" sets the number by hand).
 TreeState split_state(nbg_engine* e, bool emit) {
     TreeState a = *e->tree;
     const size_t n = e->count, groups = n / 64;

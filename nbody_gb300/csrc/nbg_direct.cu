@@ -866,10 +866,15 @@ constexpr int kSmallB = 2;        // bodies per lane, 32 kSmallB a block
 constexpr int kSmallFold = 16;    // quads a warp sums before the sums are folded
 constexpr long long kSmallMin = 32;  // at least so many quads per CTA
 // Up to this size the small-system kernel: fcompute 16 / 5.9 us at 1000 bodies
-// (symmetric / small), 20 / 8.7 at 3000, 20 / 15 at 5003.  Alone it is the
-// faster one up to 9000 bodies (30.1 / 29.6 us at 8000), but it does twice the
-// symmetric kernel's pairs, and three engines side by side take 54 / 55 us an
-// RK4 step of 5003 bodies and 79 / 113 at 8000.
+// (symmetric / small), 20 / 8.7 at 3000, 20 / 15 at 5003.  It does twice the
+// symmetric kernel's pairs, which an engine that has the GPU to itself does not
+// notice and several side by side do.  An RK4 step of a Plummer sphere alone, and
+// of three engines side by side, us: 4096 bodies 111 / 75 and 42 / 42, 5003
+// 114 / 87 and 47 / 54, 5120 114 / 89 and 47 / 56, 5500 146 / 98 and 55 / 62, 6000
+// 146 / 99 and 55 / 71, 7000 150 / 126 and 64 / 90, 8000 152 / 148 and 75 / 113.  So
+// no limit serves both: side by side it would be 4096, alone 8000; at this one
+// (five of the symmetric kernel's ranges of 1024 bodies) the small kernel gains
+// 22 % alone and costs 19 % side by side.
 constexpr int kSmallMax = 5120;
 
 struct SmallArgs {

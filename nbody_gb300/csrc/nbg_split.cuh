@@ -27,8 +27,10 @@ __device__ __forceinline__ f2_t f2_mul_rn(f2_t a, f2_t b) {
 }
 
 // -a, 2 a and a / 2 in integer registers: the FP32 pipe is what bounds the
-// kernels that use them (2 a and a / 2 of a zero come out as 2^-126, which
-// the sums below do not see).
+// kernels that use them.  They add to the exponent field: 2 a of a zero comes out
+// as 2^-126, which the sums below do not see, and a / 2 wants a normal number (a
+// zero gives an infinity; split_rsqrt meets one only for an infinite r^2, whose
+// NaN the callers' near test sends to FP64).
 __device__ __forceinline__ f2_t f2_neg(f2_t a) { return a ^ 0x8000000080000000ull; }
 __device__ __forceinline__ f2_t f2_scale_exp(f2_t a, int exp_bits) {
     float l, h;
