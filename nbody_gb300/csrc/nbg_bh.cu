@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) split_nodes_kernel(SplitSystem s, TreeSta
             split3(ex == 2048 ? nan("") : fabs(x) < 1.0 ? x : 0.0, h[c], m[c], l[c]);
         }
         const double ms = t.mass[i] * s.mass_scale;
-        const float mh = (float)ms, ml = (float)(ms - (double)mh);
+        const float mh = (float)ms, ml = split_word(ms - (double)mh, (unsigned)i);
         const double cr = scalbn(t.crit2[i], -2 * min(ex, 1000));
         SplitNode& o = reinterpret_cast<SplitNode*>(t.split)[i];
         o.b.a = make_float4(h[0], m[0], l[0], h[1]);

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) split_pack_kernel(SplitSystem a) {
             for (int c = 0; c < 3; ++c)
                 split3(ex == 2048 ? nan("") : scalbn(a.y[(size_t)c * a.n + i], -ex), h[c], m[c], l[c]);
             const double ms = a.mass[i] * a.mass_scale;
-            const float mh = (float)ms, ml = (float)(ms - (double)mh);
+            const float mh = (float)ms, ml = split_word(ms - (double)mh, (unsigned)i);
             b.a = make_float4(h[0], m[0], l[0], h[1]);
             b.b = make_float4(m[1], l[1], h[2], m[2]);
             b.c = make_float4(l[2], mh, ml, split_mass_size(ms));

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kSplitT, 4) split_potential_kernel(PotArgs a) 
     // unsoftened: pairs at or below the minimum distance are taken in FP64
     const float far_p = SOFT ? kSplitFarP : fminf(kSplitFarP, (float)scalbn(0.999 / kMinDistance, 2 * exc));
     const double e2 = SOFT ? scalbn(s.eps2, -2 * exc) : 0.0;
-    const float e2h = (float)e2, e2l = (float)(e2 - (double)e2h);
+    const float e2h = (float)e2, e2l = split_word(e2 - (double)e2h, blockIdx.y * gridDim.x + blockIdx.x);
     const f2_t zero = f2_pack(0.f, 0.f);
     f2_t hi = zero, lo = zero;
     double far0 = 0.0, far1 = 0.0, near0 = 0.0, near1 = 0.0;
