@@ -505,7 +505,7 @@ __global__ void ens_sym_reduce_kernel(const int* __restrict__ sys, const long lo
 #pragma unroll
             for (int c = 0; c < 3; ++c) add(c, -bp[c * bstride + (size_t)r * n], 0.f);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[c * B + j] = w * ((double)hi[c] + (double)lo[c]);
+        for (int c = 0; c < 3; ++c) acc[c * B + j] = w * two_word_value(hi[c], lo[c]);
     }
 }
 

@@ -156,6 +156,12 @@ __device__ __forceinline__ float rcp_mufu(float x) {
     return r;
 }
 
+// The value of a two-word sum.  One that is not finite is in its high word (the
+// low word's error terms are then inf - inf).
+__device__ __forceinline__ double two_word_value(float hi, float lo) {
+    return fabsf(hi) <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi;
+}
+
 // Knuth two-sum in packed form: (hi, lo) += p with the rounding error of the
 // high-part addition carried into lo.
 __device__ __forceinline__ void f2_two_sum(f2_t& hi, f2_t& lo, f2_t p) {

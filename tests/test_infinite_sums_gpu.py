@@ -1,0 +1,35 @@
+"""A body of infinite mass in the mixed-precision sums that end in two FP32 words:
+every other body's acceleration is infinite, towards it."""
+import numpy as np
+import pytest
+
+from nbody_gb300.data import NBodyData
+from nbody_gb300.ensemble import Ensemble
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(n, heavy, sign):
+    d = NBodyData.uniform_cube(n, side=2.0, seed=n)
+    d.mass[heavy] = sign * np.inf
+    return d
+
+
+def _check(a, d, heavy, sign):
+    want = np.copysign(np.inf, sign * (d.vertices[heavy] - d.vertices))
+    rows = np.arange(d.get_count()) != heavy
+    assert np.array_equal(a[rows], want[rows])
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("heavy", [0, 700, 1499])
+@pytest.mark.parametrize("g", [1, 2])
+def test_ensemble(gpulib, g, heavy, sign):
+    systems = [_data(1500, heavy, sign), NBodyData.plummer(300, seed=1)]
+    ens = Ensemble(softening=1e-2)
+    ens.tune_set("ensemble.pairs_per_lane", g)
+    ens.init(systems)
+    a = ens.fcompute().reshape(6, -1)[3:].T
+    _check(a[:1500], systems[0], heavy, sign)
+    assert np.all(np.isfinite(a[1500:]))
+    ens.close()
