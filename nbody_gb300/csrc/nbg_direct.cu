@@ -1001,7 +1001,7 @@ direct_small_kernel(SmallArgs a) {
                 const float s1 = s.x + p.x, b1 = s1 - s.x;
                 s = make_float2(s1, s.y + (((s.x - (s1 - b1)) + (p.x - b1)) + p.y));
             }
-            const double v = (double)s.x + (double)s.y;
+            const double v = two_word_value(s.x, s.y);
             if (i < a.n) atomicAdd(a.acc + (size_t)(k % 3) * a.n + i, UNI ? a.m_uni * v : v);
         }
         __syncthreads();

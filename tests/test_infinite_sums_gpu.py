@@ -33,3 +33,16 @@ def test_ensemble(gpulib, g, heavy, sign):
     _check(a[:1500], systems[0], heavy, sign)
     assert np.all(np.isfinite(a[1500:]))
     ens.close()
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("soft", [0.0, 1e-2])
+@pytest.mark.parametrize("n,heavy", [(2, 0), (65, 64), (1500, 700), (5120, 5119)])
+def test_small_direct_sum(make_engine, n, heavy, soft, sign):
+    d = _data(n, heavy, sign)
+    e = make_engine(precision="mixed", softening=soft)
+    assert e.init(d)
+    f, a = e.create_buffer(8 * 6 * n), np.zeros(6 * n)
+    e.fcompute(0.0, e.get_y(), f)
+    e.read_buffer(a, f)
+    _check(a[3 * n:].reshape(3, n).T, d, heavy, sign)
