@@ -448,7 +448,7 @@ split_walk_sum_kernel(SplitWalkArgs a, const double* __restrict__ y, double* __r
     for (int p = 0; p < a.parts; ++p) s += __ldg(a.part + (size_t)p * 3 * n + at);
     const size_t row = at / n * n + b;
     f[row] = y[3 * n + row];
-    f[3 * n + row] = fp64_result(s, a.s.mass[b]);
+    f[3 * n + row] = fp64_result(s, a.s.mass[b], a.s.n);
 }
 
 // Warp-coherent FP32 walk; acceleration a_i = sum m (c - x_i) (d^2 + eps^2)^-3/2.

@@ -99,7 +99,7 @@ direct_fp64_kernel(const double* __restrict__ y, const double* __restrict__ mass
     }
     if (lane < 3) {
         f[lane * sn + i] = y[(3 + lane) * sn + i];
-        f[(3 + lane) * sn + i] = fp64_result(lane == 0 ? ax : lane == 1 ? ay : az, mass[i]);
+        f[(3 + lane) * sn + i] = fp64_result(lane == 0 ? ax : lane == 1 ? ay : az, mass[i], n);
     }
 }
 
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(128) split_reduce_kernel(SplitArgs a) {
 #pragma unroll 16
     for (int r = 0; r < a.ranges; ++r) s += __ldg(a.part + (size_t)r * 3 * sn + at);
     a.f[at] = a.s.y[3 * sn + at];
-    a.f[3 * sn + at] = fp64_result(s, a.s.mass[at % sn]);
+    a.f[3 * sn + at] = fp64_result(s, a.s.mass[at % sn], a.s.n);
 }
 
 // ---------------------------------------------------------------------------

@@ -35,9 +35,10 @@ __device__ __forceinline__ void pair_fp64(double dx, double dy, double dz, doubl
 }
 
 // The reference forms the force with m_i and divides by m_i again: for a
-// massless or non-finite m_i that is NaN.
-__device__ __forceinline__ double fp64_result(double a, double m) {
-    return m != 0.0 && fabs(m) <= 1.7976931348623157e308 ? a : a * m / m;
+// massless or non-finite m_i that is NaN, but for a lone body, whose force is 0.
+__device__ __forceinline__ double fp64_result(double a, double m, int n) {
+    if (m != 0.0 && fabs(m) <= 1.7976931348623157e308) return a;
+    return (n == 1 ? 0.0 : a * m) / m;
 }
 
 struct SplitBody {  // 48 bytes

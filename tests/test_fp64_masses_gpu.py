@@ -88,3 +88,13 @@ def test_largest_mass_at_the_ends_of_the_range(make_engine, algo, exp):
     else:
         error = [np.sqrt(((x - acc) ** 2).sum() / (acc ** 2).sum()) for x in (one, a)]
         assert 0 < error[0] < 0.1 and abs(error[1] / error[0] - 1) < 1e-2
+
+
+@pytest.mark.parametrize("split", [0, 1])
+@pytest.mark.parametrize("algo", ["direct", "bh"])
+@pytest.mark.parametrize("mass,want", [(np.inf, 0.0), (-np.inf, 0.0), (2.0, 0.0), (0.0, np.nan), (np.nan, np.nan)])
+def test_lone_body(make_engine, algo, split, mass, want):
+    """Its force is 0, which the reference divides by its mass."""
+    d = NBodyData.uniform_cube(1, side=2.0, seed=1)
+    d.mass[0] = mass
+    assert np.array_equal(_forces(make_engine, d, algo, split), np.full((1, 3), want), equal_nan=True)
