@@ -64,12 +64,15 @@ __device__ __forceinline__ void split3(double x, float& h, float& m, float& l) {
 // word.  Two words are off by up to 2^-49 of the value; rounded alike, equal
 // masses (or the softening) would be off by the same in every term, up to 1.8e-15
 // that no sum averages out (1.2e-15 of the potential of 20011 bodies of mass
-// 1 / 20011).  So the k-th of them is rounded up or down with the two neighbours'
-// distances as the shares, by the multiples of the golden ratio.
+// 1 / 20011).  So the k-th of them is rounded down after a share of FP32's last
+// place has been added, the shares being the multiples of the golden ratio.
+// (Three FP64 operations, the last place's exponent and the share put together in
+// integers.)
 __device__ __forceinline__ float split_word(double r, unsigned k) {
-    const float lo = __double2float_rd(r), hi = __double2float_ru(r);
-    const double share = (double)(k * 2654435769u) * 0x1p-32;
-    return share * ((double)hi - (double)lo) < r - (double)lo ? hi : lo;
+    const unsigned h = k * 2654435769u;
+    const double share = __hiloint2double((int)(0x3ff00000u | h >> 12), (int)(h << 20));  // + 1
+    const double last = __hiloint2double(max((__double2hiint(r) & 0x7ff00000) - (23 << 20), 0), 0);
+    return __double2float_rd(fma(share, last, r) - last);
 }
 
 // Packed difference of one coordinate, d = d1 + d2 with |d2| <= ulp(d1) / 2
