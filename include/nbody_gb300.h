@@ -404,7 +404,9 @@ void nbg_ensemble_params_default(nbg_ensemble_params* p);
 nbg_status nbg_ensemble_create(const nbg_ensemble_params* p, nbg_ensemble** out);
 void nbg_ensemble_destroy(nbg_ensemble* s);
 const char* nbg_ensemble_last_error(const nbg_ensemble* s);
-/* counts[nsys]; vertices / velocities AoS [sum counts][3], systems concatenated. */
+/* counts[nsys]; vertices / velocities AoS [sum counts][3], systems concatenated.
+ * A batch that is refused (an empty system, no memory) leaves no batch: the calls
+ * below then report NBG_ERR_NOT_INITIALIZED until one is accepted. */
 nbg_status nbg_ensemble_init(nbg_ensemble* s, size_t nsys, const uint32_t* counts,
                              const double* vertices, const double* velocities,
                              const double* mass);
@@ -414,6 +416,7 @@ nbg_status nbg_ensemble_synchronize(nbg_ensemble* s);
 /* Per system (any pointer may be NULL): time, next dt, accepted, rejected. */
 nbg_status nbg_ensemble_status(nbg_ensemble* s, double* t, double* dt, uint32_t* accepted,
                                uint32_t* rejected);
+/* The state as nbg_ensemble_init takes it. */
 nbg_status nbg_ensemble_get_state(nbg_ensemble* s, double* vertices, double* velocities);
 /* f = [v ; a] of the current state, SoA [6][sum counts] (parity checks). */
 nbg_status nbg_ensemble_fcompute(nbg_ensemble* s, double* f);
@@ -424,7 +427,8 @@ nbg_status nbg_ensemble_statistics(nbg_ensemble* s, double* out);
  * a system evaluated once for both bodies, the reaction sums kept as
  * per-range partials and added in a fixed order, so results stay
  * bit-reproducible; the partials take sum_s ceil(N_s / (256 G)) N_s floats
- * per component, and above 8 GiB the one-sided kernel runs instead; 0: the
+ * per component, and above 8 GiB, or where the device has no memory for
+ * them, the one-sided kernel runs instead; 0: the
  * one-sided kernel), "ensemble.pairs_per_lane" (1
  * or 2: i-tile of 256 or 512 bodies per work unit), "ensemble.blocks_per_sm"
  * (0 = as many as fit),
